@@ -298,6 +298,82 @@ struct DivisorF32 {
 __device__ __forceinline__ DivisorF32 divisor(float b) { return {b}; }
 __device__ __forceinline__ float div_rn(float a, const DivisorF32& d) { return a / d.b; }
 
+// FP64 adds and multiplies issued as fused multiply-adds of three registers.
+//
+// GB300's FP64 unit takes a warp's DADD or DMUL every 19 SM cycles, and a
+// DFMA with a constant operand too, but a DFMA with three register operands
+// every 16 (measured: 4 to 64 warps per SM, 1 to 8 independent chains).  The
+// plain path is bound by that unit, so it writes a + b as fma(a, one, b) and
+// a * b as fma(a, b, nz) with one = 1.0 and nz = -0.0 held in registers: the
+// products a * 1 and a * b are exact inside the fused operation, so the
+// single rounding is the one of the sum or the product, and adding -0.0
+// leaves every product as it is, signed zeros included.  Same bits, 17.0
+// instead of 19.7 SM cycles per operation in a barrier-free WENO5 loop
+// (two blocks of 256 threads per SM).
+struct Fma64 {
+  double v, one, nz;
+};
+// The two constants, opaque to the compiler (eps is a run-time parameter,
+// finite and positive), so that they stay in registers.
+__device__ __forceinline__ Fma64 fma64_unit(double eps) {
+  return {0.0, __fma_rn(eps, 0.0, 1.0), __dmul_rn(eps, -0.0)};
+}
+__device__ __forceinline__ Fma64 operator+(const Fma64& a, const Fma64& b) {
+  return {__fma_rn(a.v, a.one, b.v), a.one, a.nz};
+}
+__device__ __forceinline__ Fma64 operator-(const Fma64& a, const Fma64& b) {
+  return {__fma_rn(-b.v, a.one, a.v), a.one, a.nz};
+}
+__device__ __forceinline__ Fma64 operator*(const Fma64& a, const Fma64& b) {
+  return {__fma_rn(a.v, b.v, a.nz), a.one, a.nz};
+}
+__device__ __forceinline__ Fma64 operator-(const Fma64& a) { return {-a.v, a.one, a.nz}; }
+// constants of the generic formulas (exact in every number type they meet)
+__device__ __forceinline__ Fma64 operator*(double a, const Fma64& b) { return Fma64{a, b.one, b.nz} * b; }
+__device__ __forceinline__ Fma64 operator+(double a, const Fma64& b) { return Fma64{a, b.one, b.nz} + b; }
+__device__ __forceinline__ Fma64 operator-(const Fma64& a, double b) { return a - Fma64{b, a.one, a.nz}; }
+__device__ __forceinline__ Fma64 operator-(double a, const Fma64& b) { return Fma64{a, b.one, b.nz} - b; }
+__device__ __forceinline__ DivisorF64 divisor(const Fma64& b) { return divisor(b.v); }
+__device__ __forceinline__ Fma64 div_rn(const Fma64& a, const DivisorF64& d) { return {div_rn(a.v, d), a.one, a.nz}; }
+
+// Number types of the generic formulas: float and double themselves, and
+// Fma64.  lift: a constant or loaded value as a number; low: back to storage.
+__device__ __forceinline__ float lift(double x, float) { return float(x); }
+__device__ __forceinline__ float lift(float x, float) { return x; }
+__device__ __forceinline__ double lift(double x, double) { return x; }
+__device__ __forceinline__ Fma64 lift(double x, const Fma64& u) { return {x, u.one, u.nz}; }
+__device__ __forceinline__ float low(float x) { return x; }
+__device__ __forceinline__ double low(double x) { return x; }
+__device__ __forceinline__ double low(const Fma64& x) { return x.v; }
+__device__ __forceinline__ float num_min(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ double num_min(double a, double b) { return fmin(a, b); }
+__device__ __forceinline__ Fma64 num_min(const Fma64& a, const Fma64& b) { return {fmin(a.v, b.v), a.one, a.nz}; }
+__device__ __forceinline__ float num_max(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double num_max(double a, double b) { return fmax(a, b); }
+__device__ __forceinline__ Fma64 num_max(const Fma64& a, const Fma64& b) { return {fmax(a.v, b.v), a.one, a.nz}; }
+__device__ __forceinline__ float num_sqrt(float a) { return sqrtf(a); }
+__device__ __forceinline__ double num_sqrt(double a) { return sqrt(a); }
+__device__ __forceinline__ Fma64 num_sqrt(const Fma64& a) { return {sqrt(a.v), a.one, a.nz}; }
+
+// The number type of the plain FP64 kernels.  The unit that contracts
+// multiplies and adds (MFC_PREC_FP64_FMA) computes on doubles, which the
+// compiler fuses.
+#ifdef MFC_FP64_CONTRACT
+using Num64 = double;
+__device__ __forceinline__ Num64 num64_unit(double) { return 0.0; }
+#else
+using Num64 = Fma64;
+__device__ __forceinline__ Num64 num64_unit(double eps) { return fma64_unit(eps); }
+#endif
+
+// A coefficient record read as numbers.
+template <class N>
+struct NumCoef {
+  const double* c;
+  N u;
+  __device__ __forceinline__ N operator[](int k) const { return lift(c[k], u); }
+};
+
 // True for an infinity or NaN: the exponent field of the high word is all
 // ones.  The mask is applied in inline PTX so that the test stays an integer
 // operation (an equivalent floating-point comparison would occupy GB300's
@@ -313,26 +389,34 @@ __device__ __forceinline__ bool not_finite(double x) {
 // the primitive ones on exit (partial densities and volume fractions are the
 // same in both sets).  Always FP64: the pressure recovery from total energy
 // cancels digits in the stiffened-gas EOS.
-template <int ND, int NF>
-__device__ __forceinline__ void cons_to_prim(double (&q)[Eqs<ND, NF>::S], const DevParams& P) {
+//
+// The sums start from their first term instead of zero where that changes
+// nothing: the density goes through the maximum, and the kinetic energy's
+// terms are never -0 (the momentum and its velocity have one sign).
+template <int ND, int NF, class N>
+__device__ __forceinline__ void cons_to_prim(double (&q)[Eqs<ND, NF>::S], const DevParams& P, const N& u) {
   using Q = Eqs<ND, NF>;
-  double rho = 0.0, gam = 0.0, pinf = 0.0, dyn = 0.0;
+  N rho = lift(q[0], u), gam = lift(0.0, u), pinf = lift(0.0, u), dyn = lift(0.0, u);
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
-    rho = rho + q[f];
-    gam = gam + q[Q::ADV + f] * P.gammas[f];
-    pinf = pinf + q[Q::ADV + f] * P.pi_infs[f];
+    if (f > 0) rho = rho + lift(q[f], u);
+    gam = gam + lift(q[Q::ADV + f], u) * lift(P.gammas[f], u);
+    pinf = pinf + lift(q[Q::ADV + f], u) * lift(P.pi_infs[f], u);
   }
-  rho = fmax(rho, 1e-16);
-  const DivisorF64 R = divisor(rho);
+  const DivisorF64 R = divisor(fmax(low(rho), 1e-16));
 #pragma unroll
   for (int d = 0; d < ND; ++d) {
-    const double mom = q[Q::MOM + d];
-    const double vel = div_rn(mom, R);
-    q[Q::MOM + d] = vel;
-    dyn = dyn + 0.5 * mom * vel;
+    const N mom = lift(q[Q::MOM + d], u);
+    const N vel = div_rn(mom, R);
+    q[Q::MOM + d] = low(vel);
+    const N t = 0.5 * mom * vel;
+    dyn = d == 0 ? t : dyn + t;
   }
-  q[Q::E] = div_rn(q[Q::E] - dyn - pinf, divisor(gam));
+  q[Q::E] = low(div_rn(lift(q[Q::E], u) - dyn - pinf, divisor(gam)));
+}
+template <int ND, int NF>
+__device__ __forceinline__ void cons_to_prim(double (&q)[Eqs<ND, NF>::S], const DevParams& P) {
+  cons_to_prim<ND, NF, double>(q, P, 0.0);
 }
 
 // The reference's run-time stability criterion of one cell
@@ -488,8 +572,8 @@ __device__ __forceinline__ void weno5_pair_fast(const Coef& C, const f32x2 (&v)[
 // WENO reconstruction of one cell from its stencil, m_weno.fpp:391-536.
 // c: the cell's kNumCoef coefficients; v[k] = value at offset k - 2.
 // Returns the left-face (x_{j-1/2}) and right-face (x_{j+1/2}) values.
-template <int WO, class RT>
-__device__ __forceinline__ void weno_cell(const RT* __restrict__ c, const RT (&v)[5], RT eps, RT& vL, RT& vR) {
+template <int WO, class RT, class Coef>
+__device__ __forceinline__ void weno_cell(const Coef& c, const RT (&v)[5], RT eps, RT& vL, RT& vR) {
   if constexpr (WO == 1) {
     vL = v[2];
     vR = v[2];
@@ -543,8 +627,8 @@ __device__ __forceinline__ void weno_cell(const RT* __restrict__ c, const RT (&v
 // x_{j+1/2}), for a cell whose other face value nobody reads: the smoothness
 // indicators, divisors and the chosen side are the same operations as in
 // weno_cell, so the value has the same bits.
-template <int WO, int SIDE, class RT>
-__device__ __forceinline__ RT weno_cell_side(const RT* __restrict__ c, const RT (&v)[5], RT eps) {
+template <int WO, int SIDE, class RT, class Coef>
+__device__ __forceinline__ RT weno_cell_side(const Coef& c, const RT (&v)[5], RT eps) {
   constexpr int kP = SIDE ? kPR : kPL, kD = SIDE ? kDR : kDL;
   if constexpr (WO == 1) {
     return v[2];
@@ -595,14 +679,15 @@ __device__ __forceinline__ void hllc_face(const RT (&qL)[Eqs<ND, NF>::S], const 
                                           const RT (&gam_i)[NF], const RT (&pi_i)[NF], RT (&F)[Eqs<ND, NF>::S],
                                           RT& ustar, RT* vsrc = nullptr) {
   using Q = Eqs<ND, NF>;
-  RT rmsL = RT(0), rmsR = RT(0);
+  const RT u0 = qL[0];  // carries the number type's constants
+  RT rmsL = qL[Q::MOM] * qL[Q::MOM], rmsR = qR[Q::MOM] * qR[Q::MOM];
 #pragma unroll
-  for (int d = 0; d < ND; ++d) {
+  for (int d = 1; d < ND; ++d) {
     rmsL = rmsL + qL[Q::MOM + d] * qL[Q::MOM + d];
     rmsR = rmsR + qR[Q::MOM + d] * qR[Q::MOM + d];
   }
   const RT pL = qL[Q::E], pR = qR[Q::E];
-  RT rhoL = RT(0), gamL = RT(0), piL = RT(0), rhoR = RT(0), gamR = RT(0), piR = RT(0);
+  RT rhoL = lift(0.0, u0), gamL = rhoL, piL = rhoL, rhoR = rhoL, gamR = rhoL, piR = rhoL;
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
     rhoL = rhoL + qL[f];
@@ -612,33 +697,34 @@ __device__ __forceinline__ void hllc_face(const RT (&qL)[Eqs<ND, NF>::S], const 
     gamR = gamR + qR[Q::ADV + f] * gam_i[f];
     piR = piR + qR[Q::ADV + f] * pi_i[f];
   }
-  const RT EL = gamL * pL + piL + RT(0.5) * rhoL * rmsL;
-  const RT ER = gamR * pR + piR + RT(0.5) * rhoR * rmsR;
+  const RT half = lift(0.5, u0), none = lift(1.0, u0), zero = lift(0.0, u0);
+  const RT EL = gamL * pL + piL + half * rhoL * rmsL;
+  const RT ER = gamR * pR + piR + half * rhoR * rmsR;
   const RT HL = div_rn(EL + pL, divisor(rhoL));
   const RT HR = div_rn(ER + pR, divisor(rhoR));
-  const RT cL = sqrt(div_rn(HL - RT(0.5) * rmsL, divisor(gamL)));
-  const RT cR = sqrt(div_rn(HR - RT(0.5) * rmsR, divisor(gamR)));
+  const RT cL = num_sqrt(div_rn(HL - half * rmsL, divisor(gamL)));
+  const RT cR = num_sqrt(div_rn(HR - half * rmsR, divisor(gamR)));
   const RT uL = qL[Q::MOM + DIR], uR = qR[Q::MOM + DIR];
-  const RT sL = fmin(uL - cL, uR - cR);
-  const RT sR = fmax(uR + cR, uL + cL);
+  const RT sL = num_min(uL - cL, uR - cR);
+  const RT sR = num_max(uR + cR, uL + cL);
   const RT sS = div_rn(pR - pL + rhoL * uL * (sL - uL) - rhoR * uR * (sR - uR),
                       divisor(rhoL * (sL - uL) - rhoR * (sR - uR)));
   if constexpr (VS) {
-    const RT sM = fmin(RT(0), sL), sP = fmax(RT(0), sR);
+    const RT sM = num_min(zero, sL), sP = num_max(zero, sR);
     const RT xiL = div_rn(sL - uL, divisor(sL - sS));
     const RT xiR = div_rn(sR - uR, divisor(sR - sS));
-    const RT xiM = RT(0.5) + copysign(RT(0.5), sS);
-    const RT xiP = RT(0.5) - copysign(RT(0.5), sS);
+    const RT xiM = lift(0.5 + copysign(0.5, double(low(sS))), u0);
+    const RT xiP = lift(0.5 - copysign(0.5, double(low(sS))), u0);
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
-      const RT flg = d == DIR ? RT(1) : RT(0);
-      vsrc[d] = xiM * (qL[Q::MOM + d] + flg * sM * (xiL - RT(1))) + xiP * (qR[Q::MOM + d] + flg * sP * (xiR - RT(1)));
+      const RT flg = d == DIR ? none : zero;
+      vsrc[d] = xiM * (qL[Q::MOM + d] + flg * sM * (xiL - none)) + xiP * (qR[Q::MOM + d] + flg * sP * (xiR - none));
     }
   }
-  if (!signbit(sS)) {  // xi_M = 1, xi_P = 0
-    const RT sM = fmin(RT(0), sL);
+  if (!signbit(low(sS))) {  // xi_M = 1, xi_P = 0
+    const RT sM = num_min(zero, sL);
     const RT xi = div_rn(sL - uL, divisor(sL - sS));
-    const RT w = uL + sM * (xi - RT(1));
+    const RT w = uL + sM * (xi - none);
 #pragma unroll
     for (int f = 0; f < NF; ++f) F[f] = qL[f] * w;
 #pragma unroll
@@ -652,9 +738,9 @@ __device__ __forceinline__ void hllc_face(const RT (&qL)[Eqs<ND, NF>::S], const 
     for (int f = 0; f < NF; ++f) F[Q::ADV + f] = qL[Q::ADV + f] * w;
     ustar = w;
   } else {  // xi_M = 0, xi_P = 1
-    const RT sP = fmax(RT(0), sR);
+    const RT sP = num_max(zero, sR);
     const RT xi = div_rn(sR - uR, divisor(sR - sS));
-    const RT w = uR + sP * (xi - RT(1));
+    const RT w = uR + sP * (xi - none);
 #pragma unroll
     for (int f = 0; f < NF; ++f) F[f] = qR[f] * w;
 #pragma unroll
@@ -674,6 +760,7 @@ __device__ __forceinline__ void hllc_face(const RT (&qL)[Eqs<ND, NF>::S], const 
 // reference's rounded product followed by the rounded sum.
 __device__ __forceinline__ float mul_add(float a, float b, float r) { return fmaf(a, b, r); }
 __device__ __forceinline__ double mul_add(double a, double b, double r) { return r + a * b; }
+__device__ __forceinline__ Fma64 mul_add(const Fma64& a, const Fma64& b, const Fma64& r) { return r + a * b; }
 
 // HLLC for the split-precision path: the same wave speeds, star state and
 // upwind flux as hllc_face (same cases, same sign test on s_S), in FP32 with
@@ -747,26 +834,28 @@ __device__ __forceinline__ void viscous_face_flux(const RT (&qL)[Eqs<ND, NF>::S]
                                                   const ViscParams& V, const RT (&vs)[ND], const RT (&dx)[2],
                                                   const RT (&dy)[2], RT (&out)[3]) {
   using Q = Eqs<ND, NF>;
+  const RT u0 = qL[0];  // carries the number type's constants
+  const RT none = lift(1.0, u0), zero = lift(0.0, u0), tiny = lift(1e-16, u0);
   RT re_avg[2];
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    RT reL = RT(-1e6), reR = RT(-1e6);
-    if (V.re_size[r] > 0) reL = reR = RT(0);
+    RT reL = lift(-1e6, u0), reR = reL;
+    if (V.re_size[r] > 0) reL = reR = zero;
     for (int q = 0; q < V.re_size[r]; ++q) {
       const int f = V.re_idx[r][q];
-      const auto D = divisor(RT(V.res[r][f]));
+      const auto D = divisor(lift(V.res[r][f], u0));
       reL = div_rn(qL[Q::ADV + f], D) + reL;
       reR = div_rn(qR[Q::ADV + f], D) + reR;
     }
-    reL = div_rn(RT(1), divisor(reL < RT(1e-16) ? RT(1e-16) : reL));
-    reR = div_rn(RT(1), divisor(reR < RT(1e-16) ? RT(1e-16) : reR));
-    re_avg[r] = div_rn(RT(2), divisor(div_rn(RT(1), divisor(reL)) + div_rn(RT(1), divisor(reR))));
+    reL = div_rn(none, divisor(low(reL) < low(tiny) ? tiny : reL));
+    reR = div_rn(none, divisor(low(reR) < low(tiny) ? tiny : reR));
+    re_avg[r] = div_rn(lift(2.0, u0), divisor(div_rn(none, divisor(reL)) + div_rn(none, divisor(reR))));
   }
   const bool shear = V.re_size[0] > 0, bulk = V.re_size[1] > 0;
-  RT fm[2] = {RT(0), RT(0)}, fe = RT(0);
+  RT fm[2] = {zero, zero}, fe = zero;
   if (DIR == 0) {
     if (shear) {
-      const RT tau = div_rn(RT(4.0 / 3.0) * dx[0], divisor(re_avg[0]));
+      const RT tau = div_rn(lift(4.0 / 3.0, u0) * dx[0], divisor(re_avg[0]));
       fm[0] = fm[0] - tau;
       fe = fe - vs[0] * tau;
     }
@@ -777,7 +866,7 @@ __device__ __forceinline__ void viscous_face_flux(const RT (&qL)[Eqs<ND, NF>::S]
     }
     if constexpr (ND > 1) {
       if (shear) {
-        const RT t0 = -div_rn(RT(2.0 / 3.0) * dy[1], divisor(re_avg[0]));
+        const RT t0 = -div_rn(lift(2.0 / 3.0, u0) * dy[1], divisor(re_avg[0]));
         const RT t1 = div_rn(dy[0] + dx[1], divisor(re_avg[0]));
         fm[0] = fm[0] - t0;
         fe = fe - vs[0] * t0;
@@ -793,7 +882,7 @@ __device__ __forceinline__ void viscous_face_flux(const RT (&qL)[Eqs<ND, NF>::S]
   } else if constexpr (ND > 1) {
     if (shear) {
       const RT t0 = div_rn(dy[0] + dx[1], divisor(re_avg[0]));
-      const RT t1 = div_rn(RT(4) * dy[1] - RT(2) * dx[0], divisor(RT(3) * re_avg[0]));
+      const RT t1 = div_rn(lift(4.0, u0) * dy[1] - lift(2.0, u0) * dx[0], divisor(lift(3.0, u0) * re_avg[0]));
       fm[0] = fm[0] - t0;
       fe = fe - vs[0] * t0;
       fm[1] = fm[1] - t1;
@@ -834,17 +923,18 @@ struct FlagC {
   static constexpr bool value = B;
 };
 
-__device__ __forceinline__ double rk_combine(int kind, double base, double in, double dt, double r) {
+template <class N>
+__device__ __forceinline__ double rk_combine(int kind, const N& base, const N& in, const N& dt, const N& r) {
   switch (kind) {
-    case kRkEuler: return base + dt * r;
-    case kRk2Final: return (base + in + dt * r) / 2.0;
-    case kRk3Mid: return (3.0 * base + in + dt * r) / 4.0;
+    case kRkEuler: return low(base + dt * r);
+    case kRk2Final: return low(base + in + dt * r) / 2.0;
+    case kRk3Mid: return low(3.0 * base + in + dt * r) / 4.0;
     case kRk3Final: {
       // divisor(3.0), spelled out: significand 1.5, 2^64 / 1.5 rounded down, exponent 1024
       constexpr DivisorF64 kThree{3.0, 0x18000000000000ULL, 0xaaaaaaaaaaaaaaaaULL, 0x400u, true};
-      return div_rn(base + 2.0 * in + 2.0 * dt * r, kThree);
+      return low(div_rn(base + 2.0 * in + 2.0 * dt * r, kThree));
     }
-    default: return r;
+    default: return low(r);
   }
 }
 

@@ -17,6 +17,8 @@
 // RK base register, and one write of the stage output.
 #pragma once
 
+#include <type_traits>
+
 #include "mfc_device.cuh"
 #include "mfc_gate.cuh"
 #include "mfc_tma.cuh"
@@ -187,7 +189,7 @@ constexpr size_t stage_smem_total(bool shared_coef) {
 // in the same order.
 template <int ND, int NF, int WO, int DIR, class At, class OutL, class OutR>
 __device__ __forceinline__ void char_weno_position(const double (&c)[kCoefRec], const At& at, const double eps,
-                                                   const DevParams& P, const OutL& L, const OutR& R) {
+                                                   const DevParams& P, const Num64& u0, const OutL& L, const OutR& R) {
   using Q = Eqs<ND, NF>;
   constexpr int S = Q::S, UN = Q::MOM + DIR;
   double rho = 0.0, gam = 0.0, pinf = 0.0;
@@ -225,10 +227,12 @@ __device__ __forceinline__ void char_weno_position(const double (&c)[kCoefRec], 
         st[k] = at(v, o);
       }
     }
-    double vl, vr;
-    weno_cell<WO, double>(c, st, eps, vl, vr);
-    L(v) = vl;
-    R(v) = vr;
+    Num64 ns[5], vl, vr;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) ns[k] = lift(st[k], u0);
+    weno_cell<WO, Num64>(NumCoef<Num64>{c, u0}, ns, lift(eps, u0), vl, vr);
+    L(v) = low(vl);
+    R(v) = low(vr);
   }
   const DivisorF64 D2 = divisor(2.0 * rc);
   auto back = [&](const auto& O) {
@@ -265,7 +269,13 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
   // split precision: FP32 reconstruction, Riemann solve and flux divergence;
   // the plain path keeps everything in FP64 in the reference's order
   constexpr bool kSplit = sizeof(RT) == 4;
-  using AT = RT;  // type of the flux-divergence accumulation
+  using AT = RT;  // storage of the flux-divergence accumulation
+  // what the arithmetic runs on (Fma64 for the plain path)
+  using N = std::conditional_t<kSplit, float, Num64>;
+  N u0;
+  if constexpr (kSplit) u0 = 0.f;
+  else u0 = num64_unit(P.weno_eps);
+  auto num = [&](RT x) { return lift(x, u0); };
 
   RT* sq = reinterpret_cast<RT*>(smem_raw);  // [S][LY][LX] primitive ([S/2][LY][LX][2] in pairs)
   RT* wl = sq + Sh::OW;                       // left-face values
@@ -288,24 +298,28 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
     return kPair ? (((v >> 1) * NCY_ + cy) * TX + tx) * 2 + (v & 1) : (v * NCY_ + cy) * TX + tx;
   };
   (void)wyi;
+  // row r of the flux of x face f (left of cell f) of row ty, and of y face f
+  auto fxv = [&](int r, int ty, int f) -> RT& { return fl[(r * TYE + ty) * (TX + 1) + f]; };
+  auto fyv = [&](int r, int f, int tx) -> RT& { return fl[(r * (TY + 1) + f) * TX + tx]; };
+  (void)fyv;
 
   const int tid = threadIdx.x;
   const int nx = P.n[0], ny = P.n[1];
 
-  RT gam_i[NF], pi_i[NF];
+  N gam_i[NF], pi_i[NF];
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
     if constexpr (kSplit) {
       gam_i[f] = P.gammas_f[f];
       pi_i[f] = P.pi_infs_f[f];
     } else {
-      gam_i[f] = P.gammas[f];
-      pi_i[f] = P.pi_infs[f];
+      gam_i[f] = num(P.gammas[f]);
+      pi_i[f] = num(P.pi_infs[f]);
     }
   }
-  RT eps;
+  N eps;
   if constexpr (kSplit) eps = P.weno_eps_f;
-  else eps = P.weno_eps;
+  else eps = num(P.weno_eps);
   // split WENO5 on a uniform grid: every cell of a direction shares one
   // coefficient record, read from the kernel parameters
   const bool ux = Sh::NCOEF > 0 && U != nullptr && U->on[0];
@@ -356,7 +370,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
       for (int v = 0; v < S; ++v) sq[qi(v, ly, lx)] = pr[v];
       if constexpr (Sh::SP > S) sq[qi(S, ly, lx)] = 0.f;  // the padding lane
     } else {
-      cons_to_prim<ND, NF>(q, P);
+      cons_to_prim<ND, NF>(q, P, u0);
 #pragma unroll
       for (int v = 0; v < S; ++v) sq[qi(v, ly, lx)] = RT(q[v]);
     }
@@ -577,16 +591,17 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
     constexpr int NCX = TX + 2;
     // variable v of the cell at (cx, ty); c: the cell's coefficient record
     auto x_recon = [&](const RT* __restrict__ c, const int cx, const int ty, const int v) {
-      RT st[5];
+      N st[5];
 #pragma unroll
       for (int k = 0; k < 5; ++k) {
         const int o = k - 2;
-        st[k] = (o >= -(WO / 2) && o <= WO / 2) ? sq[qi(v, (ND > 1) ? ty + H : 0, cx + H - 1 + o)] : RT(0);
+        st[k] = num(o >= -(WO / 2) && o <= WO / 2 ? sq[qi(v, (ND > 1) ? ty + H : 0, cx + H - 1 + o)] : RT(0));
       }
-      RT vl, vr;
-      weno_cell<WO, RT>(c, st, eps, vl, vr);
-      wl[wxi(v, ty, cx)] = vl;
-      wr[wxi(v, ty, cx)] = vr;
+      N vl, vr;
+      if constexpr (kSplit) weno_cell<WO, N>(c, st, eps, vl, vr);
+      else weno_cell<WO, N>(NumCoef<N>{c, u0}, st, eps, vl, vr);
+      wl[wxi(v, ty, cx)] = low(vl);
+      wr[wxi(v, ty, cx)] = low(vr);
     };
     if constexpr (kPair) {
       constexpr int NPR = Sh::SP / 2;  // variable pairs
@@ -648,7 +663,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
         for (int k = 0; k < kNumCoef; ++k) c[k] = RT(__ldg(cf + k * cs + gi));
         const int ly = (ND > 1) ? ty + H : 0, lx = cx + H - 1;
         char_weno_position<ND, NF, WO, 0>(
-            c, [&](int v, int o) { return sq[qi(v, ly, lx + o)]; }, eps, P,
+            c, [&](int v, int o) { return sq[qi(v, ly, lx + o)]; }, low(eps), P, u0,
             [&](int v) -> RT& { return wl[wxi(v, ty, cx)]; }, [&](int v) -> RT& { return wr[wxi(v, ty, cx)]; });
       }
     } else if constexpr (sizeof(RT) == 8 && WO > 1) {
@@ -683,14 +698,14 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
         const int ty = r % TYE, v = r / TYE, cx = side ? NCX - 1 : 0;
         RT c[kCoefRec];
         coef(cx, c);
-        RT st[5];
+        N st[5];
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
           const int o = k - 2;
-          st[k] = (o >= -(WO / 2) && o <= WO / 2) ? sq[qi(v, (ND > 1) ? ty + H : 0, cx + H - 1 + o)] : RT(0);
+          st[k] = num(o >= -(WO / 2) && o <= WO / 2 ? sq[qi(v, (ND > 1) ? ty + H : 0, cx + H - 1 + o)] : RT(0));
         }
-        if (side) wl[wxi(v, ty, cx)] = weno_cell_side<WO, 0, RT>(c, st, eps);
-        else wr[wxi(v, ty, cx)] = weno_cell_side<WO, 1, RT>(c, st, eps);
+        if (side) wl[wxi(v, ty, cx)] = low(weno_cell_side<WO, 0, N>(NumCoef<N>{c, u0}, st, eps));
+        else wr[wxi(v, ty, cx)] = low(weno_cell_side<WO, 1, N>(NumCoef<N>{c, u0}, st, eps));
       }
     } else {
       // split WENO1/3 (and FP64 WENO1): coefficients per reconstruction from global memory
@@ -718,19 +733,19 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
     for (int it = tid; it < TYE * NFXr; it += NT) {
       const int f = it % NFXr, ty = it / NFXr;
       const int gface = x0 - 1 + f;  // face gface+1/2
-      RT qL[S], qR[S], F[S], us;
+      N qL[S], qR[S], F[S], us;
       const bool lfr = (gface == -1 && P.bc_beg[0] == -4);      // qL(-1) = qR(0)
       const bool rfl = (gface == nx - 1 && P.bc_end[0] == -4);  // qR(m+1) = qL(m)
 #pragma unroll
       for (int v = 0; v < S; ++v) {
-        const RT a = wr[wxi(v, ty, f)];
-        const RT b = wl[wxi(v, ty, f + 1)];
+        const N a = num(wr[wxi(v, ty, f)]);
+        const N b = num(wl[wxi(v, ty, f + 1)]);
         qL[v] = lfr ? b : a;
         qR[v] = rfl ? a : b;
       }
       if constexpr (VISC) {
-        RT vs[ND], dxv[2] = {RT(0), RT(0)}, dyv[2] = {RT(0), RT(0)}, vf[3];
-        hllc_face<ND, NF, 0, RT, true>(qL, qR, gam_i, pi_i, F, us, vs);
+        N vs[ND], dxv[2] = {num(RT(0)), num(RT(0))}, dyv[2] = {num(RT(0)), num(RT(0))}, vf[3];
+        hllc_face<ND, NF, 0, N, true>(qL, qR, gam_i, pi_i, F, us, vs);
         const ViscParams& V = *P.visc;
         if (V.fg[0] != nullptr) {
           // weno_Re_flux = T: the prepared face gradients (clamped indices
@@ -740,17 +755,17 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
           const double* g = V.fg[0] + (int64_t)gy * (nx + 1) + (min(max(gface, -1), nx - 1) + 1);
 #pragma unroll
           for (int c = 0; c < ND; ++c) {
-            dxv[c] = narrow<RT>(__ldg(g + (c * ND) * plane));
-            if constexpr (ND > 1) dyv[c] = narrow<RT>(__ldg(g + (c * ND + 1) * plane));
+            dxv[c] = num(narrow<RT>(__ldg(g + (c * ND) * plane)));
+            if constexpr (ND > 1) dyv[c] = num(narrow<RT>(__ldg(g + (c * ND + 1) * plane)));
           }
         } else {
           const int ly = (ND > 1) ? ty + H : 0, lx = f + H - 1;  // the face's left cell
-          auto U = [&](int c, int x, int y) { return sq[qi(Q::MOM + c, y, x)]; };
+          auto U = [&](int c, int x, int y) { return num(sq[qi(Q::MOM + c, y, x)]); };
           const auto Dx = divisor(narrow<RT>(__ldg(V.dcc[0] + min(x0 + f, nx))));  // x_cc(j+1) - x_cc(j)
 #pragma unroll
           for (int c = 0; c < ND; ++c) {
-            const RT g = div_rn(U(c, lx + 1, ly) - U(c, lx, ly), Dx);
-            dxv[c] = RT(0.5) * (g + g);
+            const N g = div_rn(U(c, lx + 1, ly) - U(c, lx, ly), Dx);
+            dxv[c] = num(RT(0.5)) * (g + g);
           }
           if constexpr (ND > 1) {
             const int gy = min(y0 + ty, ny - 1);
@@ -760,22 +775,22 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
             for (int c = 0; c < ND; ++c) {
               auto Ly = [&](int x) { return div_rn(U(c, x, ly) - U(c, x, ly - 1), D0); };
               auto Ry = [&](int x) { return div_rn(U(c, x, ly + 1) - U(c, x, ly), D1); };
-              const RT A = RT(0.25) * (Ly(lx + 1) + Ry(lx + 1) + Ly(lx) + Ry(lx));
-              dyv[c] = RT(0.5) * (A + A);
+              const N A = num(RT(0.25)) * (Ly(lx + 1) + Ry(lx + 1) + Ly(lx) + Ry(lx));
+              dyv[c] = num(RT(0.5)) * (A + A);
             }
           }
         }
-        viscous_face_flux<ND, NF, 0, RT>(qL, qR, V, vs, dxv, dyv, vf);
+        viscous_face_flux<ND, NF, 0, N>(qL, qR, V, vs, dxv, dyv, vf);
 #pragma unroll
-        for (int t = 0; t < 3; ++t) fl[((S + 1 + t) * TYE + ty) * NFXr + f] = vf[t];
+        for (int t = 0; t < 3; ++t) fxv(S + 1 + t, ty, f) = low(vf[t]);
       } else if constexpr (kSplit) {
         hllc_face_fast<ND, NF, 0>(qL, qR, gam_i, pi_i, F, us);
       } else {
-        hllc_face<ND, NF, 0, RT>(qL, qR, gam_i, pi_i, F, us);
+        hllc_face<ND, NF, 0, N>(qL, qR, gam_i, pi_i, F, us);
       }
 #pragma unroll
-      for (int v = 0; v < S; ++v) fl[(v * TYE + ty) * NFXr + f] = F[v];
-      fl[(S * TYE + ty) * NFXr + f] = us;
+      for (int v = 0; v < S; ++v) fxv(v, ty, f) = low(F[v]);
+      fxv(S, ty, f) = low(us);
     }
   }
   __syncthreads();
@@ -788,22 +803,20 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
     if (e >= TX * TYE) break;
     const int tx = e % TX, ty = e / TX;
     const int gx = x0 + tx;
-    constexpr int NFXr = TX + 1;
-    const AT inv = narrow<AT>(__ldg(P.inv_d[0] + (gx < nx ? gx : nx - 1)));
+    const N inv = num(narrow<AT>(__ldg(P.inv_d[0] + (gx < nx ? gx : nx - 1))));
 #pragma unroll
-    for (int v = 0; v < S; ++v)
-      rhs[k][v] = inv * (AT(fl[(v * TYE + ty) * NFXr + tx]) - AT(fl[(v * TYE + ty) * NFXr + tx + 1]));
-    const AT du = AT(fl[(S * TYE + ty) * NFXr + tx + 1]) - AT(fl[(S * TYE + ty) * NFXr + tx]);
+    for (int v = 0; v < S; ++v) rhs[k][v] = low(inv * (num(fxv(v, ty, tx)) - num(fxv(v, ty, tx + 1))));
+    const N du = num(fxv(S, ty, tx + 1)) - num(fxv(S, ty, tx));
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
-      const AT a = AT(sq[qi(Q::ADV + f, ND > 1 ? ty + H : 0, tx + H)]);
-      rhs[k][Q::ADV + f] = mul_add(inv * a, du, rhs[k][Q::ADV + f]);
+      const N a = num(sq[qi(Q::ADV + f, ND > 1 ? ty + H : 0, tx + H)]);
+      rhs[k][Q::ADV + f] = low(mul_add(inv * a, du, num(rhs[k][Q::ADV + f])));
     }
     if constexpr (VISC) {  // m_rhs.fpp:591-603: momentum .. energy
 #pragma unroll
       for (int t = 0; t <= ND; ++t) {
         const int v = t < ND ? Q::MOM + t : Q::E, r = S + 1 + (t < ND ? t : 2);
-        rhs[k][v] = mul_add(inv, AT(fl[(r * TYE + ty) * NFXr + tx]) - AT(fl[(r * TYE + ty) * NFXr + tx + 1]), rhs[k][v]);
+        rhs[k][v] = low(mul_add(inv, num(fxv(r, ty, tx)) - num(fxv(r, ty, tx + 1)), num(rhs[k][v])));
       }
     }
   }
@@ -811,16 +824,17 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
     constexpr int NCY = TY + 2;
     // variable v of the cell at (tx, cy)
     auto y_recon = [&](const RT* __restrict__ c, const int tx, const int cy, const int v) {
-      RT st[5];
+      N st[5];
 #pragma unroll
       for (int k = 0; k < 5; ++k) {
         const int o = k - 2;
-        st[k] = (o >= -(WO / 2) && o <= WO / 2) ? sq[qi(v, cy + H - 1 + o, tx + H)] : RT(0);
+        st[k] = num(o >= -(WO / 2) && o <= WO / 2 ? sq[qi(v, cy + H - 1 + o, tx + H)] : RT(0));
       }
-      RT vl, vr;
-      weno_cell<WO, RT>(c, st, eps, vl, vr);
-      wl[wyi(v, cy, tx)] = vl;
-      wr[wyi(v, cy, tx)] = vr;
+      N vl, vr;
+      if constexpr (kSplit) weno_cell<WO, N>(c, st, eps, vl, vr);
+      else weno_cell<WO, N>(NumCoef<N>{c, u0}, st, eps, vl, vr);
+      wl[wyi(v, cy, tx)] = low(vl);
+      wr[wyi(v, cy, tx)] = low(vr);
     };
     if constexpr (kPair) {
       constexpr int NPR = Sh::SP / 2;
@@ -877,7 +891,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
         for (int k = 0; k < kNumCoef; ++k) c[k] = RT(__ldg(cf + k * cs + gi));
         const int ly = cy + H - 1, lx = tx + H;
         char_weno_position<ND, NF, WO, 1>(
-            c, [&](int v, int o) { return sq[qi(v, ly + o, lx)]; }, eps, P,
+            c, [&](int v, int o) { return sq[qi(v, ly + o, lx)]; }, low(eps), P, u0,
             [&](int v) -> RT& { return wl[wyi(v, cy, tx)]; }, [&](int v) -> RT& { return wr[wyi(v, cy, tx)]; });
       }
     } else if constexpr (sizeof(RT) == 8 && WO > 1) {
@@ -908,14 +922,14 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
         const int tx = r % TX, v = r / TX, cy = side ? NCY - 1 : 0;
         RT c[kCoefRec];
         coef(cy, c);
-        RT st[5];
+        N st[5];
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
           const int o = k - 2;
-          st[k] = (o >= -(WO / 2) && o <= WO / 2) ? sq[qi(v, cy + H - 1 + o, tx + H)] : RT(0);
+          st[k] = num(o >= -(WO / 2) && o <= WO / 2 ? sq[qi(v, cy + H - 1 + o, tx + H)] : RT(0));
         }
-        if (side) wl[wyi(v, cy, tx)] = weno_cell_side<WO, 0, RT>(c, st, eps);
-        else wr[wyi(v, cy, tx)] = weno_cell_side<WO, 1, RT>(c, st, eps);
+        if (side) wl[wyi(v, cy, tx)] = low(weno_cell_side<WO, 0, N>(NumCoef<N>{c, u0}, st, eps));
+        else wr[wyi(v, cy, tx)] = low(weno_cell_side<WO, 1, N>(NumCoef<N>{c, u0}, st, eps));
       }
     } else {
       const double* cf = P.coef[1];
@@ -940,19 +954,19 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
     for (int it = tid; it < NFYr * TX; it += NT) {
       const int tx = it % TX, f = it / TX;
       const int gface = y0 - 1 + f;
-      RT qL[S], qR[S], F[S], us;
+      N qL[S], qR[S], F[S], us;
       const bool lfr = (gface == -1 && P.bc_beg[1] == -4);
       const bool rfl = (gface == ny - 1 && P.bc_end[1] == -4);
 #pragma unroll
       for (int v = 0; v < S; ++v) {
-        const RT a = wr[wyi(v, f, tx)];
-        const RT b = wl[wyi(v, f + 1, tx)];
+        const N a = num(wr[wyi(v, f, tx)]);
+        const N b = num(wl[wyi(v, f + 1, tx)]);
         qL[v] = lfr ? b : a;
         qR[v] = rfl ? a : b;
       }
       if constexpr (VISC) {
-        RT vs[ND], dxv[2], dyv[2], vf[3];
-        hllc_face<ND, NF, 1, RT, true>(qL, qR, gam_i, pi_i, F, us, vs);
+        N vs[ND], dxv[2], dyv[2], vf[3];
+        hllc_face<ND, NF, 1, N, true>(qL, qR, gam_i, pi_i, F, us, vs);
         const ViscParams& V = *P.visc;
         const int gx = min(x0 + tx, nx - 1);
         if (V.fg[1] != nullptr) {
@@ -961,12 +975,12 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
           const double* g = V.fg[1] + (int64_t)(min(max(gface, -1), ny - 1) + 1) * nx + gx;
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
-            dxv[c] = narrow<RT>(__ldg(g + (c * 2) * plane));
-            dyv[c] = narrow<RT>(__ldg(g + (c * 2 + 1) * plane));
+            dxv[c] = num(narrow<RT>(__ldg(g + (c * 2) * plane)));
+            dyv[c] = num(narrow<RT>(__ldg(g + (c * 2 + 1) * plane)));
           }
         } else {
           const int ly = f + H - 1, lx = tx + H;  // the face's lower cell
-          auto U = [&](int c, int x, int y) { return sq[qi(Q::MOM + c, y, x)]; };
+          auto U = [&](int c, int x, int y) { return num(sq[qi(Q::MOM + c, y, x)]); };
           const auto Dy = divisor(narrow<RT>(__ldg(V.dcc[1] + min(y0 + f, ny))));  // y_cc(k+1) - y_cc(k)
           const auto D0 = divisor(narrow<RT>(__ldg(V.dcc[0] + gx))),
                      D1 = divisor(narrow<RT>(__ldg(V.dcc[0] + gx + 1)));
@@ -974,23 +988,23 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
           for (int c = 0; c < 2; ++c) {
             auto Lx = [&](int y) { return div_rn(U(c, lx, y) - U(c, lx - 1, y), D0); };
             auto Rx = [&](int y) { return div_rn(U(c, lx + 1, y) - U(c, lx, y), D1); };
-            const RT A = RT(0.25) * (Lx(ly + 1) + Rx(ly + 1) + Lx(ly) + Rx(ly));
-            dxv[c] = RT(0.5) * (A + A);
-            const RT g = div_rn(U(c, lx, ly + 1) - U(c, lx, ly), Dy);
-            dyv[c] = RT(0.5) * (g + g);
+            const N A = num(RT(0.25)) * (Lx(ly + 1) + Rx(ly + 1) + Lx(ly) + Rx(ly));
+            dxv[c] = num(RT(0.5)) * (A + A);
+            const N g = div_rn(U(c, lx, ly + 1) - U(c, lx, ly), Dy);
+            dyv[c] = num(RT(0.5)) * (g + g);
           }
         }
-        viscous_face_flux<ND, NF, 1, RT>(qL, qR, V, vs, dxv, dyv, vf);
+        viscous_face_flux<ND, NF, 1, N>(qL, qR, V, vs, dxv, dyv, vf);
 #pragma unroll
-        for (int t = 0; t < 3; ++t) fl[((S + 1 + t) * NFYr + f) * TX + tx] = vf[t];
+        for (int t = 0; t < 3; ++t) fyv(S + 1 + t, f, tx) = low(vf[t]);
       } else if constexpr (kSplit) {
         hllc_face_fast<ND, NF, 1>(qL, qR, gam_i, pi_i, F, us);
       } else {
-        hllc_face<ND, NF, 1, RT>(qL, qR, gam_i, pi_i, F, us);
+        hllc_face<ND, NF, 1, N>(qL, qR, gam_i, pi_i, F, us);
       }
 #pragma unroll
-      for (int v = 0; v < S; ++v) fl[(v * NFYr + f) * TX + tx] = F[v];
-      fl[(S * NFYr + f) * TX + tx] = us;
+      for (int v = 0; v < S; ++v) fyv(v, f, tx) = low(F[v]);
+      fyv(S, f, tx) = low(us);
     }
     __syncthreads();
 
@@ -1001,21 +1015,21 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
       if (e >= TX * TY) break;
       const int tx = e % TX, ty = e / TX;
       const int gy = y0 + ty;
-      const AT inv = narrow<AT>(__ldg(P.inv_d[1] + (gy < ny ? gy : ny - 1)));
+      const N inv = num(narrow<AT>(__ldg(P.inv_d[1] + (gy < ny ? gy : ny - 1))));
 #pragma unroll
       for (int v = 0; v < S; ++v)
-        rhs[k][v] = mul_add(inv, AT(fl[(v * NFYr + ty) * TX + tx]) - AT(fl[(v * NFYr + ty + 1) * TX + tx]), rhs[k][v]);
-      const AT du = AT(fl[(S * NFYr + ty + 1) * TX + tx]) - AT(fl[(S * NFYr + ty) * TX + tx]);
+        rhs[k][v] = low(mul_add(inv, num(fyv(v, ty, tx)) - num(fyv(v, ty + 1, tx)), num(rhs[k][v])));
+      const N du = num(fyv(S, ty + 1, tx)) - num(fyv(S, ty, tx));
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
-        const AT a = AT(sq[qi(Q::ADV + f, ty + H, tx + H)]);
-        rhs[k][Q::ADV + f] = mul_add(inv * a, du, rhs[k][Q::ADV + f]);
+        const N a = num(sq[qi(Q::ADV + f, ty + H, tx + H)]);
+        rhs[k][Q::ADV + f] = low(mul_add(inv * a, du, num(rhs[k][Q::ADV + f])));
       }
       if constexpr (VISC) {  // m_rhs.fpp:639-651
 #pragma unroll
         for (int t = 0; t <= ND; ++t) {
           const int v = t < ND ? Q::MOM + t : Q::E, r = S + 1 + (t < ND ? t : 2);
-          rhs[k][v] = mul_add(inv, AT(fl[(r * NFYr + ty) * TX + tx]) - AT(fl[(r * NFYr + ty + 1) * TX + tx]), rhs[k][v]);
+          rhs[k][v] = low(mul_add(inv, num(fyv(r, ty, tx)) - num(fyv(r, ty + 1, tx)), num(rhs[k][v])));
         }
       }
     }
@@ -1049,7 +1063,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
           double in = b;
           if constexpr (KIND != kRkEuler) in = __ldg(qin + o + v * P.sv);
           if constexpr (kSplit) out = rk_combine_split(KIND, b, in, dtf, rhs[k][v]);
-          else out = rk_combine(KIND, b, in, dt, rhs[k][v]);
+          else out = rk_combine(KIND, num(b), num(in), num(dt), num(rhs[k][v]));
         }
         bad |= not_finite(out);
         qout[o + v * P.sv] = out;

@@ -87,6 +87,12 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
   constexpr int S = Sh::S, H = Sh::H, LA = Sh::LA, NP = Sh::NP;
   constexpr bool kSplit = sizeof(RT) == 4;
   using AT = RT;
+  // what the arithmetic runs on (Fma64 for the plain path)
+  using N = std::conditional_t<kSplit, float, Num64>;
+  N u0;
+  if constexpr (kSplit) u0 = 0.f;
+  else u0 = num64_unit(P.weno_eps);
+  auto num = [&](RT x) { return lift(x, u0); };
   constexpr int OA = DIR, OB = DIR == 0 ? 1 : 0, OC = DIR == 2 ? 1 : 2;  // axis index of a, b, c
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -114,20 +120,20 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
   else { b0 = blockIdx.x * TB; a0 = blockIdx.y * TA; c0 = blockIdx.z * TC; }
   const int na = P.n[OA], nb = P.n[OB], nc = P.n[OC];
 
-  RT gam_i[NF], pi_i[NF];
+  N gam_i[NF], pi_i[NF];
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
     if constexpr (kSplit) {
       gam_i[f] = P.gammas_f[f];
       pi_i[f] = P.pi_infs_f[f];
     } else {
-      gam_i[f] = P.gammas[f];
-      pi_i[f] = P.pi_infs[f];
+      gam_i[f] = num(P.gammas[f]);
+      pi_i[f] = num(P.pi_infs[f]);
     }
   }
-  RT eps;
+  N eps;
   if constexpr (kSplit) eps = P.weno_eps_f;
-  else eps = P.weno_eps;
+  else eps = num(P.weno_eps);
   // split WENO5 on a uniform grid: one coefficient record for the whole sweep
   const bool ua = Sh::NCOEF > 0 && U.on[DIR];
   (void)ua;
@@ -156,7 +162,7 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
     if constexpr (kSplit) {
       cons_to_prim_split<3, NF>(q, P, pr);
     } else {
-      cons_to_prim<3, NF>(q, P);
+      cons_to_prim<3, NF>(q, P, u0);
 #pragma unroll
       for (int v = 0; v < S; ++v) pr[v] = q[v];
     }
@@ -304,16 +310,17 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
   constexpr int NCA = TA + 2;
   // variable v of cell ca of pencil p; c: the cell's coefficient record
   auto recon = [&](const RT* __restrict__ c, const int ca, const int p, const int v) {
-    RT stc[5];
+    N stc[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
       const int o = k - 2;
-      stc[k] = (o >= -(WO / 2) && o <= WO / 2) ? sq[qi(v, p, ca + H - 1 + o)] : RT(0);
+      stc[k] = num(o >= -(WO / 2) && o <= WO / 2 ? sq[qi(v, p, ca + H - 1 + o)] : RT(0));
     }
-    RT vl, vr;
-    weno_cell<WO, RT>(c, stc, eps, vl, vr);
-    wl[wi(v, p, ca)] = vl;
-    wr[wi(v, p, ca)] = vr;
+    N vl, vr;
+    if constexpr (kSplit) weno_cell<WO, N>(c, stc, eps, vl, vr);
+    else weno_cell<WO, N>(NumCoef<N>{c, u0}, stc, eps, vl, vr);
+    wl[wi(v, p, ca)] = low(vl);
+    wr[wi(v, p, ca)] = low(vr);
   };
   if constexpr (kPair) {
     constexpr int NPR = S / 2;
@@ -365,7 +372,7 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
 #pragma unroll
       for (int k = 0; k < kNumCoef; ++k) c[k] = __ldg(P.coef[DIR] + k * P.cstride[DIR] + gi);
       char_weno_position<3, NF, WO, DIR>(
-          c, [&](int v, int o) { return sq[qi(v, p, ca + H - 1 + o)]; }, eps, P,
+          c, [&](int v, int o) { return sq[qi(v, p, ca + H - 1 + o)]; }, low(eps), P, u0,
           [&](int v) -> RT& { return wl[wi(v, p, ca)]; }, [&](int v) -> RT& { return wr[wi(v, p, ca)]; });
     }
   } else {
@@ -389,21 +396,21 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
   for (int it = tid; it < NP * NFA; it += NT) {
     const int f = it % NFA, p = it / NFA;
     const int gface = a0 - 1 + f;
-    RT qL[S], qR[S], F[S], us;
+    N qL[S], qR[S], F[S], us;
     const bool lfr = (gface == -1 && P.bc_beg[OA] == -4);
     const bool rfl = (gface == na - 1 && P.bc_end[OA] == -4);
 #pragma unroll
     for (int v = 0; v < S; ++v) {
-      const RT a = wr[wi(v, p, f)];
-      const RT b = wl[wi(v, p, f + 1)];
+      const N a = num(wr[wi(v, p, f)]);
+      const N b = num(wl[wi(v, p, f + 1)]);
       qL[v] = lfr ? b : a;
       qR[v] = rfl ? a : b;
     }
     if constexpr (kSplit) hllc_face_fast<3, NF, DIR>(qL, qR, gam_i, pi_i, F, us);
-    else hllc_face<3, NF, DIR, RT>(qL, qR, gam_i, pi_i, F, us);
+    else hllc_face<3, NF, DIR, N>(qL, qR, gam_i, pi_i, F, us);
 #pragma unroll
-    for (int v = 0; v < S; ++v) fl[(v * NP + p) * NFA + f] = F[v];
-    fl[(S * NP + p) * NFA + f] = us;
+    for (int v = 0; v < S; ++v) fl[(v * NP + p) * NFA + f] = low(F[v]);
+    fl[(S * NP + p) * NFA + f] = low(us);
   }
   __syncthreads();
 
@@ -428,35 +435,35 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
       int x, y, z;
       sweep_coords<DIR>(ga, gb, gc, x, y, z);
       const int64_t o = z * P.sz + y * P.sy + x;
-      const AT inv = narrow<AT>(__ldg(P.inv_d[DIR] + ga));
-      AT r[S];
+      const N inv = num(narrow<AT>(__ldg(P.inv_d[DIR] + ga)));
+      N r[S];
 #pragma unroll
       for (int v = 0; v < S; ++v) {
-        const AT diff = AT(fl[(v * NP + p) * NFA + ta]) - AT(fl[(v * NP + p) * NFA + ta + 1]);
-        r[v] = (DIR == 0) ? inv * diff : mul_add(inv, diff, rhs_buf[o + v * P.sv]);
+        const N diff = num(fl[(v * NP + p) * NFA + ta]) - num(fl[(v * NP + p) * NFA + ta + 1]);
+        r[v] = (DIR == 0) ? inv * diff : mul_add(inv, diff, num(rhs_buf[o + v * P.sv]));
       }
-      const AT du = AT(fl[(S * NP + p) * NFA + ta + 1]) - AT(fl[(S * NP + p) * NFA + ta]);
+      const N du = num(fl[(S * NP + p) * NFA + ta + 1]) - num(fl[(S * NP + p) * NFA + ta]);
 #pragma unroll
       for (int f = 0; f < NF; ++f) {
-        const AT a = AT(sq[qi(Q::ADV + f, p, ta + H)]);
+        const N a = num(sq[qi(Q::ADV + f, p, ta + H)]);
         r[Q::ADV + f] = mul_add(inv * a, du, r[Q::ADV + f]);
       }
       if constexpr (DIR < 2) {
 #pragma unroll
-        for (int v = 0; v < S; ++v) rhs_buf[o + v * P.sv] = r[v];
+        for (int v = 0; v < S; ++v) rhs_buf[o + v * P.sv] = low(r[v]);
         continue;
       }
 #pragma unroll
       for (int v = 0; v < S; ++v) {
         double out;
         if constexpr (KIND == kRhsOnly) {
-          out = widen(r[v]);
+          out = widen(low(r[v]));
         } else {
           const double b = __ldg(qbase + o + v * P.sv);
           double in = b;
           if constexpr (KIND != kRkEuler) in = __ldg(qin + o + v * P.sv);
           if constexpr (kSplit) out = rk_combine_split(KIND, b, in, dtf, r[v]);
-          else out = rk_combine(KIND, b, in, dt, r[v]);
+          else out = rk_combine(KIND, num(b), num(in), num(dt), r[v]);
         }
         bad |= not_finite(out);
         qout[o + v * P.sv] = out;

@@ -5,6 +5,7 @@
 // a CPU build of the reference with default flags fuses them.  The results
 // are no longer bit-identical to the contraction-off oracle; their distance
 // from it is measured by tests/test_fp64_fma.py and reported by bench.py.
+#define MFC_FP64_CONTRACT  // plain doubles, which -fmad=true contracts
 #include "mfc_launch.h"
 
 namespace mfc {
