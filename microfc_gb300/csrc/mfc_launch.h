@@ -13,6 +13,7 @@
 
 #include "../../include/mfc_gpu.h"
 #include "mfc_device.cuh"
+#include "mfc_flex.cuh"
 #include "mfc_stage.cuh"
 #include "mfc_sweep.cuh"
 
@@ -29,6 +30,8 @@ struct StageEntry {
   bool visc = false;  // compiled with the viscous terms
   bool tma = false;   // interior tiles staged by a TMA bulk tensor copy
   bool chr = false;   // WENO of the characteristic fields (MFC_RECON_CHARACTERISTIC)
+  // the tile of an nx x ny grid where the launch chooses it (else tx, ty)
+  void (*tile)(int nx, int ny, int* tx, int* ty) = nullptr;
 };
 
 // Launches a stage kernel with programmatic stream serialization, so that
@@ -122,6 +125,104 @@ StageEntry stage_entry() {
                     VISC,
                     TMA,
                     CHAR};
+}
+
+// The tile size of flex_kernel for an nx x ny grid: the one with the least
+// work on the busiest SM, ceil(tiles / 152) tiles of the largest size.  A
+// tile's cost in SM cycles, from the operation counts of the formulas and the
+// FP64 unit's measured rates: a phase takes 16.5 cycles per warp operation
+// once four warps are busy, but at least 64 per operation of one warp's chain
+// of items; loads, barriers and the block's launch take about 8000 more.
+// Candidates: the smallest tile of each number of columns and rows that fits
+// shared memory.  A pure function of the sizes, remembered per thread for the
+// last few grids (a search takes about 0.1 ms).
+template <int ND, int NF, int WO, int NT, bool VISC>
+void flex_plan(int nx, int ny, int* tx, int* ty) {
+  using Sh = FlexShape<ND, NF, WO>;
+  struct Memo {
+    int nx, ny, tx, ty;
+  };
+  thread_local Memo memo[8] = {};
+  thread_local unsigned next = 0;
+  for (const Memo& m : memo)
+    if (m.nx == nx && m.ny == ny) {
+      *tx = m.tx;
+      *ty = m.ty;
+      return;
+    }
+  constexpr int kSMs = 152, S = Sh::S, H = Sh::H, NW = NT / 32;
+  constexpr double kRate = 16.5, kChain = 64.0, kTile = 8000.0;
+  constexpr double both = WO == 5 ? 72 : WO == 3 ? 26 : 0, one = WO == 5 ? 53 : WO == 3 ? 18 : 0;
+  constexpr double face = VISC ? 160 : 95, prim = 17, cell = ND > 1 ? 14 : 9;
+  auto groups = [](int n) { return (n + 31) / 32; };
+  // total operations and number of groups of a phase; its longest chain
+  auto phase = [&](double ops, int g, double item) {
+    const double chain = kChain * item * ((g + NW - 1) / NW);
+    return ops * kRate > chain ? ops * kRate : chain;
+  };
+  auto cost = [&](int x, int y) {
+    const int gi = groups(S * x * y), gex = groups(S * y), gey = ND > 1 ? groups(S * x) : 0;
+    const int gf = groups((x + 1) * y) + (ND > 1 ? groups(x * (y + 1)) : 0);
+    const int gl = groups(x * y + 2 * H * (y + (ND > 1 ? x : 0)));
+    return phase(gl * prim, gl, prim) + phase(ND * gi * both + 2 * (gex + gey) * one, ND * gi + 2 * (gex + gey), both) +
+           phase(gf * face, gf, face) + phase(gi * cell, gi, cell) + kTile;
+  };
+  double best = 0.0;
+  *tx = 1;
+  *ty = 1;
+  for (int c = 1, last_x = 0; c <= nx; ++c) {
+    const int x = (nx + c - 1) / c;
+    if (x == last_x) continue;
+    last_x = x;
+    if (x < (ND > 1 ? 4 : 2)) break;
+    if (x > (ND > 1 ? 96 : 512)) continue;
+    for (int r = 1, last_y = 0; r <= ny; ++r) {
+      const int y = (ny + r - 1) / r;
+      if (y == last_y) continue;
+      last_y = y;
+      if (ND > 1 && (y < 4 || y > 96)) {
+        if (y < 4) break;
+        continue;
+      }
+      if (Sh::bytes(x, y) > kFlexSmemMax) continue;
+      const int64_t tiles = (int64_t)((nx + x - 1) / x) * ((ny + y - 1) / y);
+      const double t = double((tiles + kSMs - 1) / kSMs) * cost(x, y);
+      if (best == 0.0 || t < best) {
+        best = t;
+        *tx = x;
+        *ty = y;
+      }
+      if (ND == 1) break;
+    }
+  }
+  memo[next++ % 8] = {nx, ny, *tx, *ty};
+}
+
+template <int ND, int NF, int WO, int NT, bool VISC = false>
+StageEntry flex_entry() {
+  StageEntry e{};
+  e.nd = ND;
+  e.nf = NF;
+  e.wo = WO;
+  e.prec = MFC_PREC_FP64;
+  e.nt = NT;
+  e.smem = kFlexSmemMax;
+  e.kernels = 1;
+  e.prepare = [] {
+    return cudaFuncSetAttribute(&flex_kernel<ND, NF, WO, NT, VISC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kFlexSmemMax);
+  };
+  e.launch = [](const DevParams& P, const UniformCoef&, const double* qin, const double* qbase, double* qout,
+                double dt, int kind, cudaStream_t st) {
+    int tx, ty;
+    flex_plan<ND, NF, WO, NT, VISC>(P.n[0], P.n[1], &tx, &ty);
+    const dim3 grid((unsigned)((P.n[0] + tx - 1) / tx), (unsigned)((P.n[1] + ty - 1) / ty));
+    return launch_dependent(&flex_kernel<ND, NF, WO, NT, VISC>, grid, dim3(NT), FlexShape<ND, NF, WO>::bytes(tx, ty),
+                            st, P, qin, qbase, qout, dt, kind, tx, ty);
+  };
+  e.visc = VISC;
+  e.tile = &flex_plan<ND, NF, WO, NT, VISC>;
+  return e;
 }
 
 // 3-D: three directional sweeps per stage (mfc_sweep.cuh).  The x sweep uses
