@@ -999,7 +999,7 @@ int mfc_gpu_select_variant(mfc_gpu_ctx* c, int variant, int* tx, int* ty, int* t
     if (e.prepare() != cudaSuccess) return fail(MFC_ERR_CUDA, "tile variant does not fit on this device");
     c->stage = &e;
     int ex = e.tx, ey = e.ty;
-    if (e.tile) e.tile(c->n[0], c->n[1], &ex, &ey);
+    if (e.tile) e.tile(c->n, &ex, &ey);
     if (tx) *tx = ex;
     if (ty) *ty = ey;
     if (threads) *threads = e.nt;

@@ -30,8 +30,8 @@ struct StageEntry {
   bool visc = false;  // compiled with the viscous terms
   bool tma = false;   // interior tiles staged by a TMA bulk tensor copy
   bool chr = false;   // WENO of the characteristic fields (MFC_RECON_CHARACTERISTIC)
-  // the tile of an nx x ny grid where the launch chooses it (else tx, ty)
-  void (*tile)(int nx, int ny, int* tx, int* ty) = nullptr;
+  // the tile of a grid of n[0] x n[1] x n[2] cells where the launch chooses it (else tx, ty)
+  void (*tile)(const int* n, int* tx, int* ty) = nullptr;
 };
 
 // Launches a stage kernel with programmatic stream serialization, so that
@@ -127,76 +127,110 @@ StageEntry stage_entry() {
                     CHAR};
 }
 
-// The tile size of flex_kernel for an nx x ny grid: the one with the least
-// work on the busiest SM, ceil(tiles / 152) tiles of the largest size.  A
-// tile's cost in SM cycles, from the operation counts of the formulas and the
-// FP64 unit's measured rates: a phase takes 16.5 cycles per warp operation
-// once four warps are busy, but at least 64 per operation of one warp's chain
-// of items; loads, barriers and the block's launch take about 8000 more.
-// Candidates: the smallest tile of each number of columns and rows that fits
-// shared memory.  A pure function of the sizes, remembered per thread for the
-// last few grids (a search takes about 0.1 ms).
-template <int ND, int NF, int WO, int NT, bool VISC>
-void flex_plan(int nx, int ny, int* tx, int* ty) {
-  using Sh = FlexShape<ND, NF, WO>;
-  struct Memo {
-    int nx, ny, tx, ty;
-  };
-  thread_local Memo memo[8] = {};
-  thread_local unsigned next = 0;
-  for (const Memo& m : memo)
-    if (m.nx == nx && m.ny == ny) {
-      *tx = m.tx;
-      *ty = m.ty;
-      return;
-    }
-  constexpr int kSMs = 152, S = Sh::S, H = Sh::H, NW = NT / 32;
-  constexpr double kRate = 16.5, kChain = 64.0, kTile = 8000.0;
-  constexpr double both = WO == 5 ? 72 : WO == 3 ? 26 : 0, one = WO == 5 ? 53 : WO == 3 ? 18 : 0;
-  constexpr double face = VISC ? 160 : 95, prim = 17, cell = ND > 1 ? 14 : 9;
-  auto groups = [](int n) { return (n + 31) / 32; };
-  // total operations and number of groups of a phase; its longest chain
-  auto phase = [&](double ops, int g, double item) {
-    const double chain = kChain * item * ((g + NW - 1) / NW);
-    return ops * kRate > chain ? ops * kRate : chain;
-  };
-  auto cost = [&](int x, int y) {
-    const int gi = groups(S * x * y), gex = groups(S * y), gey = ND > 1 ? groups(S * x) : 0;
-    const int gf = groups((x + 1) * y) + (ND > 1 ? groups(x * (y + 1)) : 0);
-    const int gl = groups(x * y + 2 * H * (y + (ND > 1 ? x : 0)));
-    return phase(gl * prim, gl, prim) + phase(ND * gi * both + 2 * (gex + gey) * one, ND * gi + 2 * (gex + gey), both) +
-           phase(gf * face, gf, face) + phase(gi * cell, gi, cell) + kTile;
-  };
-  double best = 0.0;
-  *tx = 1;
-  *ty = 1;
+// Tile sizes of the flex kernels: the ones with the least work on the
+// busiest SM, ceil(tiles / 152) tiles of the largest size.  A tile's cost in
+// SM cycles, from the operation counts of the formulas and the FP64 unit's
+// measured rates: a phase takes 16.5 cycles per warp operation once four
+// warps are busy, but at least 64 per operation of one warp's chain of items;
+// loads, barriers and the block's launch take about 8000 more.  Candidates:
+// the smallest tile of each number of columns and rows that fits shared
+// memory.  A plan is a pure function of the sizes; each thread remembers
+// those of the last few grids (a search takes about 0.1 ms).
+namespace flex {
+constexpr int kSMs = 152;
+constexpr double kRate = 16.5, kChain = 64.0, kTile = 8000.0;
+constexpr double weno_ops(int wo) { return wo == 5 ? 72 : wo == 3 ? 26 : 0; }
+constexpr double weno_side_ops(int wo) { return wo == 5 ? 53 : wo == 3 ? 18 : 0; }
+inline int groups(int n) { return (n + 31) / 32; }
+// a phase of `ops` warp operations in g groups of at most `item` operations
+inline double phase(double ops, int g, double item, int warps) {
+  const double chain = kChain * item * ((g + warps - 1) / warps);
+  return ops * kRate > chain ? ops * kRate : chain;
+}
+
+// The sizes (x, y) that minimise ceil(tiles / 152) * cost(x, y) over grids
+// of nx x ny x layers cells cut into ceil(nx / x) * ceil(ny / y) * layers
+// tiles, with lo <= x <= hi_x, y <= hi_y and fits(x, y).
+struct Plan {
+  int key[3] = {0, 0, 0}, x = 0, y = 0;
+};
+template <class Cost, class Fits>
+Plan search(int nx, int ny, int layers, int lo_x, int hi_x, int lo_y, int hi_y, Cost&& cost, Fits&& fits) {
+  Plan best{{nx, ny, layers}, 1, 1};
+  double least = 0.0;
+  lo_x = lo_x < nx ? lo_x : nx;
+  lo_y = lo_y < ny ? lo_y : ny;
   for (int c = 1, last_x = 0; c <= nx; ++c) {
     const int x = (nx + c - 1) / c;
-    if (x == last_x) continue;
+    if (x == last_x || x > hi_x) continue;
     last_x = x;
-    if (x < (ND > 1 ? 4 : 2)) break;
-    if (x > (ND > 1 ? 96 : 512)) continue;
+    if (x < lo_x) break;
     for (int r = 1, last_y = 0; r <= ny; ++r) {
       const int y = (ny + r - 1) / r;
-      if (y == last_y) continue;
+      if (y == last_y || y > hi_y) continue;
       last_y = y;
-      if (ND > 1 && (y < 4 || y > 96)) {
-        if (y < 4) break;
-        continue;
-      }
-      if (Sh::bytes(x, y) > kFlexSmemMax) continue;
-      const int64_t tiles = (int64_t)((nx + x - 1) / x) * ((ny + y - 1) / y);
+      if (y < lo_y) break;
+      if (!fits(x, y)) continue;
+      const int64_t tiles = (int64_t)((nx + x - 1) / x) * ((ny + y - 1) / y) * layers;
       const double t = double((tiles + kSMs - 1) / kSMs) * cost(x, y);
-      if (best == 0.0 || t < best) {
-        best = t;
-        *tx = x;
-        *ty = y;
+      if (least == 0.0 || t < least) {
+        least = t;
+        best.x = x;
+        best.y = y;
       }
-      if (ND == 1) break;
     }
   }
-  memo[next++ % 8] = {nx, ny, *tx, *ty};
+  return best;
 }
+// The remembered plan of a grid, or a new search.
+template <class Search>
+Plan remembered(Plan (&memo)[8], unsigned& next, int nx, int ny, int layers, Search&& s) {
+  for (const Plan& m : memo)
+    if (m.key[0] == nx && m.key[1] == ny && m.key[2] == layers) return m;
+  return memo[next++ % 8] = s();
+}
+
+template <int ND, int NF, int WO, int NT, bool VISC>
+Plan plan(int nx, int ny) {
+  using Sh = FlexShape<ND, NF, WO>;
+  thread_local Plan memo[8];
+  thread_local unsigned next = 0;
+  return remembered(memo, next, nx, ny, 1, [&] {
+    constexpr int S = Sh::S, H = Sh::H, NW = NT / 32;
+    constexpr double both = weno_ops(WO), one = weno_side_ops(WO);
+    constexpr double face = VISC ? 160 : 95, prim = 17, cell = ND > 1 ? 14 : 9;
+    auto cost = [&](int x, int y) {
+      const int gi = groups(S * x * y), ge = groups(S * y) + (ND > 1 ? groups(S * x) : 0);
+      const int gf = groups((x + 1) * y) + (ND > 1 ? groups(x * (y + 1)) : 0);
+      const int gl = groups(x * y + 2 * H * (y + (ND > 1 ? x : 0)));
+      return phase(gl * prim, gl, prim, NW) + phase(ND * gi * both + 2 * ge * one, ND * gi + 2 * ge, both, NW) +
+             phase(gf * face, gf, face, NW) + phase(gi * cell, gi, cell, NW) + kTile;
+    };
+    return search(nx, ny, 1, ND > 1 ? 4 : 2, ND > 1 ? 96 : 512, ND > 1 ? 4 : 1, 96, cost,
+                  [](int x, int y) { return Sh::bytes(x, y) <= kFlexSmemMax; });
+  });
+}
+
+// x: cells along the sweep, y: pencils
+template <int NF, int WO, int NT, int DIR>
+Plan sweep_plan(int na, int nb, int nc) {
+  using Sh = FlexSweepShape<NF, WO, DIR>;
+  thread_local Plan memo[8];
+  thread_local unsigned next = 0;
+  return remembered(memo, next, na, nb, nc, [&] {
+    constexpr int S = Sh::S, H = Sh::H, NW = NT / 32;
+    constexpr double both = weno_ops(WO), one = weno_side_ops(WO);
+    constexpr double face = 100, prim = DIR == 0 ? 20 : 0, cell = DIR == 2 ? 10 : 4;
+    auto cost = [&](int a, int p) {
+      const int gi = groups(S * a * p), ge = groups(S * p), gf = groups((a + 1) * p), gl = groups((a + 2 * H) * p);
+      return phase(gl * prim, gl, prim, NW) + phase(gi * both + 2 * ge * one, gi + 2 * ge, both, NW) +
+             phase(gf * face, gf, face, NW) + phase(gi * cell, gi, cell, NW) + kTile;
+    };
+    // y and z: at least eight pencils, one 64-byte line of x per row
+    return search(na, nb, nc, 4, 512, DIR == 0 ? 1 : 8, 256, cost, [](int a, int p) { return Sh::bytes(a, p) <= kFlexSmemMax; });
+  });
+}
+}  // namespace flex
 
 template <int ND, int NF, int WO, int NT, bool VISC = false>
 StageEntry flex_entry() {
@@ -214,14 +248,59 @@ StageEntry flex_entry() {
   };
   e.launch = [](const DevParams& P, const UniformCoef&, const double* qin, const double* qbase, double* qout,
                 double dt, int kind, cudaStream_t st) {
-    int tx, ty;
-    flex_plan<ND, NF, WO, NT, VISC>(P.n[0], P.n[1], &tx, &ty);
-    const dim3 grid((unsigned)((P.n[0] + tx - 1) / tx), (unsigned)((P.n[1] + ty - 1) / ty));
-    return launch_dependent(&flex_kernel<ND, NF, WO, NT, VISC>, grid, dim3(NT), FlexShape<ND, NF, WO>::bytes(tx, ty),
-                            st, P, qin, qbase, qout, dt, kind, tx, ty);
+    const flex::Plan t = flex::plan<ND, NF, WO, NT, VISC>(P.n[0], P.n[1]);
+    const dim3 grid((unsigned)((P.n[0] + t.x - 1) / t.x), (unsigned)((P.n[1] + t.y - 1) / t.y));
+    return launch_dependent(&flex_kernel<ND, NF, WO, NT, VISC>, grid, dim3(NT), FlexShape<ND, NF, WO>::bytes(t.x, t.y),
+                            st, P, qin, qbase, qout, dt, kind, t.x, t.y);
   };
   e.visc = VISC;
-  e.tile = &flex_plan<ND, NF, WO, NT, VISC>;
+  e.tile = [](const int* n, int* tx, int* ty) {
+    const flex::Plan t = flex::plan<ND, NF, WO, NT, VISC>(n[0], n[1]);
+    *tx = t.x;
+    *ty = t.y;
+  };
+  return e;
+}
+
+// 3-D: three flex sweeps per stage.
+template <int NF, int WO, int NT>
+StageEntry flex_sweep_entry() {
+  StageEntry e{};
+  e.nd = 3;
+  e.nf = NF;
+  e.wo = WO;
+  e.prec = MFC_PREC_FP64;
+  e.nt = NT;
+  e.smem = kFlexSmemMax;
+  e.kernels = 3;
+  e.prepare = [] {
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t r = cudaFuncSetAttribute(&flex_sweep_kernel<NF, WO, NT, 0>, attr, (int)kFlexSmemMax);
+    if (r == cudaSuccess) r = cudaFuncSetAttribute(&flex_sweep_kernel<NF, WO, NT, 1>, attr, (int)kFlexSmemMax);
+    if (r == cudaSuccess) r = cudaFuncSetAttribute(&flex_sweep_kernel<NF, WO, NT, 2>, attr, (int)kFlexSmemMax);
+    return r;
+  };
+  e.launch = [](const DevParams& P, const UniformCoef&, const double* qin, const double* qbase, double* qout,
+                double dt, int kind, cudaStream_t st) {
+    auto sweep = [&](auto dir) {
+      constexpr int D = decltype(dir)::value;
+      constexpr int A = D, B = D == 0 ? 1 : 0, C = D == 2 ? 1 : 2;
+      const flex::Plan t = flex::sweep_plan<NF, WO, NT, D>(P.n[A], P.n[B], P.n[C]);
+      const unsigned tiles =
+          (unsigned)((P.n[A] + t.x - 1) / t.x) * (unsigned)((P.n[B] + t.y - 1) / t.y) * (unsigned)P.n[C];
+      return launch_dependent(&flex_sweep_kernel<NF, WO, NT, D>, dim3(tiles), dim3(NT),
+                              FlexSweepShape<NF, WO, D>::bytes(t.x, t.y), st, P, qin, qbase, qout, dt, kind, t.x, t.y);
+    };
+    cudaError_t r = sweep(std::integral_constant<int, 0>{});
+    if (r == cudaSuccess) r = sweep(std::integral_constant<int, 1>{});
+    if (r == cudaSuccess) r = sweep(std::integral_constant<int, 2>{});
+    return r;
+  };
+  e.tile = [](const int* n, int* tx, int* ty) {  // the x sweep's
+    const flex::Plan t = flex::sweep_plan<NF, WO, NT, 0>(n[0], n[1], n[2]);
+    *tx = t.x;
+    *ty = t.y;
+  };
   return e;
 }
 

@@ -4,14 +4,13 @@
 namespace mfc {
 
 void register_stage_3d_fp64(std::vector<StageEntry>& r) {
-  r.push_back(Sweep3D<2, 5, double, 32, 4, 2, 16, 16, 256>::entry());
-  r.push_back(Sweep3D<2, 5, double, 32, 4, 2, 16, 16, 256, true>::entry());  // TMA-staged tiles
-  // 320 threads at 96 registers, two blocks per SM (20 warps): 7.09e7
-  // cell-updates/s at 256^3 against 7.02e7 for 256 threads
+  r.push_back(flex_sweep_entry<2, 5, 640>());
+  // fixed tiles, TMA-staged: even with the sized ones where the grid is a
+  // multiple of both tiles (26.05 and 26.01 ms a step at 128^3), slower elsewhere
   r.push_back(Sweep3D<2, 5, double, 32, 4, 2, 16, 16, 320, true, 2, false, 2>::entry());
-  r.push_back(Sweep3D<1, 5, double, 32, 4, 2, 16, 16, 256>::entry());
-  r.push_back(Sweep3D<2, 3, double, 32, 4, 2, 16, 16, 256>::entry());
-  r.push_back(Sweep3D<2, 1, double, 32, 4, 2, 16, 16, 256>::entry());
+  r.push_back(flex_sweep_entry<1, 5, 640>());
+  r.push_back(flex_sweep_entry<2, 3, 512>());
+  r.push_back(flex_sweep_entry<2, 1, 512>());
 }
 
 }  // namespace mfc

@@ -39,3 +39,14 @@ def test_2d_sizes(nx, ny, bcx, bcy, viscous):
         c = c.replace(re_shear=(10.0, 500.0), re_bulk=(0.0, 200.0))
     got, want = _run(c, 2)
     assert np.array_equal(got.view(np.uint64), want.view(np.uint64))
+
+
+@pytest.mark.parametrize("order", [1, 3, 5])
+@pytest.mark.parametrize("nx,ny,nz,bcx,bcy,bcz",
+                         [(25, 26, 27, (-3, -3), (-2, -4), (-1, -1)), (161, 25, 33, (-4, -2), (-1, -1), (-2, -3)),
+                          (31, 97, 25, (-2, -3), (-4, -4), (-3, -4))])
+def test_3d_sizes(nx, ny, nz, bcx, bcy, bcz, order):
+    c = cases.shock_bubble_3d(N=28, steps=2, precision="fp64")
+    c = c.replace(m=nx - 1, n=ny - 1, p=nz - 1, dt=c.dt / 8, bc_x=bcx, bc_y=bcy, bc_z=bcz, weno_order=order)
+    got, want = _run(c, 2)
+    assert np.array_equal(got.view(np.uint64), want.view(np.uint64))
