@@ -4,36 +4,22 @@
 namespace mfc {
 
 void register_ensemble_fp32(std::vector<EnsembleEntry>& r) {
-  r.push_back(ensemble_entry<2, 5, float, 32, 16, 256>());
-  r.push_back(ensemble_entry<2, 5, float, 16, 16, 256>());
-  r.push_back(ensemble_entry<2, 5, float, 32, 8, 256>());
-  r.push_back(ensemble_entry<2, 5, float, 32, 32, 512>());
-  r.push_back(ensemble_entry<2, 5, float, 64, 8, 256>());
-  r.push_back(ensemble_entry<2, 5, float, 16, 16, 256, false, 4>());
-  r.push_back(ensemble_entry<2, 5, float, 16, 16, 256, false, 5>());
-  // interior tiles staged by one TMA bulk tensor copy
-  r.push_back(ensemble_entry<2, 5, float, 16, 16, 256, false, 5, true>());
+  // interior tiles loaded by one TMA bulk tensor copy; the first is the default
+  r.push_back(ensemble_entry<2, float, 16, 16, 256, 4, 9, 9, false, true>());
+  r.push_back(ensemble_entry<2, float, 16, 16, 256, 4, 9, 9>());
+  r.push_back(ensemble_entry<2, float, 8, 8, 160, 6, 2, 2, false, true>());
   // with the viscous terms (mfc_gpu_ensemble_set_viscosity)
-  r.push_back(ensemble_entry<2, 5, float, 16, 16, 256, false, 1, false, true>());
-  r.push_back(ensemble_entry<2, 5, float, 32, 16, 256, false, 1, false, true>());
+  r.push_back(ensemble_entry<2, float, 16, 16, 256, 4, 9, 9, false, false, true>());
+  r.push_back(ensemble_entry<2, float, 16, 16, 256, 3, 9, 9, false, false, true>());
 }
 
-}  // namespace mfc
-
-namespace mfc {
-
 void register_ensemble_gated(std::vector<EnsembleEntry>& r) {
-  r.push_back(ensemble_entry<2, 5, float, 32, 16, 256, true>());
-  r.push_back(ensemble_entry<2, 5, float, 16, 16, 256, true>());
-  r.push_back(ensemble_entry<2, 5, float, 32, 32, 512, true>());
-  // register-capped 16x16 tiles: four or five blocks per SM
-  r.push_back(ensemble_entry<2, 5, float, 16, 16, 256, true, 4>());
-  r.push_back(ensemble_entry<2, 5, float, 16, 16, 256, true, 5>());
-  // interior tiles staged by one TMA bulk tensor copy (four blocks per SM:
-  // the five-block cap spills the TMA kernel's registers)
-  r.push_back(ensemble_entry<2, 5, float, 16, 16, 256, true, 4, true>());
+  // interior tiles loaded by one TMA bulk tensor copy; the first is the default
+  r.push_back(ensemble_entry<2, float, 16, 16, 256, 4, 9, 9, true, true>());
+  r.push_back(ensemble_entry<2, float, 16, 16, 256, 4, 9, 9, true>());
+  r.push_back(ensemble_entry<2, float, 16, 16, 256, 3, 9, 9, true, true>());
   // with the viscous terms (mfc_gpu_ensemble_set_viscosity)
-  r.push_back(ensemble_entry<2, 5, float, 16, 16, 256, true, 1, false, true>());
+  r.push_back(ensemble_entry<2, float, 16, 16, 256, 4, 9, 9, true, false, true>());
 }
 
 }  // namespace mfc

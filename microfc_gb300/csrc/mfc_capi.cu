@@ -167,6 +167,12 @@ struct mfc_gpu_ctx {
   void* gate_w = nullptr;       // MFC_PREC_GATED: FP16 gate parameters
   uint8_t* gate_flags = nullptr;  // MFC_PREC_GATED: a step's first-stage gate decisions
   bool gate_ready = false;
+  // split and gated 2-D WENO5: the primitive pairs of the last stage's output
+  // (prim[prim_at]; of register prim_of, or of none), and the buffer that the
+  // next stage writes them to
+  mfc::f32x2* prim[2] = {nullptr, nullptr};
+  int prim_at = 0;
+  const double* prim_of = nullptr;
   unsigned long long* monitor = nullptr;  // max ICFL of the monitored steps (double bits)
   bool monitor_on = false;
   double* tables = nullptr;     // inv_d and coefficient tables
@@ -257,7 +263,21 @@ int launch_stage(mfc_gpu_ctx* c, const double* qin, const double* qbase, double*
     if (g != cudaSuccess) return fail(MFC_ERR_CUDA, std::string("viscous gradients: ") + cudaGetErrorString(g));
     c->launches += c->nd == 1 ? 3 : 4;
   }
-  cudaError_t e = c->stage->launch(P, c->ucoef, qin, qbase, qout, dt, kind, c->stream);
+  cudaError_t e;
+  if (c->prim[0] != nullptr && c->stage->launch_prims != nullptr) {
+    const bool keep = kind != mfc::kRhsOnly;  // an RHS evaluation makes no state
+    const int64_t pitch = mfc::prim_pitch(c->n[0]);
+    const mfc::PrimPairs B{c->prim_of == qin ? c->prim[c->prim_at] : nullptr,
+                           keep ? c->prim[c->prim_at ^ 1] : nullptr, pitch, pitch * c->n[1]};
+    e = c->stage->launch_prims(P, c->ucoef, qin, qbase, qout, dt, kind, B, c->stream);
+    if (keep) {
+      c->prim_at ^= 1;
+      c->prim_of = e == cudaSuccess ? qout : nullptr;
+    }
+  } else {
+    e = c->stage->launch(P, c->ucoef, qin, qbase, qout, dt, kind, c->stream);
+    if (kind != mfc::kRhsOnly) c->prim_of = nullptr;  // the registers change, the pairs do not
+  }
   if (e != cudaSuccess) return fail(MFC_ERR_CUDA, std::string("stage launch: ") + cudaGetErrorString(e));
   c->launches += c->stage->kernels;
   return MFC_OK;
@@ -413,6 +433,16 @@ int mfc_gpu_init(const mfc_params* p, mfc_gpu_ctx** out) {
   if (p->precision == MFC_PREC_GATED &&
       (e = cudaMalloc(&c->gate_flags, mfc::gate_flag_bytes(c->n[0], c->n[1]))) != cudaSuccess)
     return cleanup(fail(MFC_ERR_NOMEM, cudaGetErrorString(e)));
+  // 2-D split and gated: two buffers of primitive pairs, the next stage's
+  // input and output (not with processor boundaries, whose ghost cells come
+  // as conservative values)
+  if (c->nd == 2 && p->weno_order == 5 && (p->precision == MFC_PREC_SPLIT || p->precision == MFC_PREC_GATED) &&
+      p->bc_x_beg < 0 && p->bc_x_end < 0 && p->bc_y_beg < 0 && p->bc_y_end < 0) {
+    const size_t bytes = sizeof(mfc::f32x2) * (size_t)((c->S + 1) / 2) * c->n[1] * mfc::prim_pitch(c->n[0]);
+    for (int k = 0; k < 2; ++k)
+      if ((e = cudaMalloc(&c->prim[k], bytes)) != cudaSuccess)
+        return cleanup(fail(MFC_ERR_NOMEM, cudaGetErrorString(e)));
+  }
   // 3-D: the partial RHS, then the primitives the x sweep stores (S x sv
   // values each, in the reconstruction type: FP64 at most)
   if (c->nd == 3 && (e = cudaMalloc(&c->work, sizeof(double) * c->reg_elems * 2)) != cudaSuccess)
@@ -500,6 +530,7 @@ int mfc_gpu_sys_size(const mfc_gpu_ctx* c) { return c ? c->S : 0; }
 
 int mfc_gpu_upload(mfc_gpu_ctx* c, int var, const double* host_sf, int64_t ld_y, int64_t ld_z) {
   if (!c || !host_sf) return fail(MFC_ERR_INVALID, "NULL argument");
+  c->prim_of = nullptr;
   int rc = copy_var(c, c->reg[0], var, host_sf, nullptr, ld_y, ld_z);
   if (rc) return rc;
   MFC_CUDA(cudaStreamSynchronize(c->stream));
@@ -522,6 +553,7 @@ int mfc_gpu_download(mfc_gpu_ctx* c, int var, double* host_sf, int64_t ld_y, int
 // one contiguous block like the host array, and one linear copy moves it
 int mfc_gpu_upload_state(mfc_gpu_ctx* c, const double* host_q) {
   if (!c || !host_q) return fail(MFC_ERR_INVALID, "NULL argument");
+  c->prim_of = nullptr;
   const size_t rows = (size_t)c->S * c->n[1] * c->n[2];
   if (c->sy == c->n[0])
     MFC_CUDA(cudaMemcpyAsync(c->reg[0], host_q, rows * c->n[0] * 8, cudaMemcpyHostToDevice, c->stream));
@@ -534,6 +566,7 @@ int mfc_gpu_upload_state(mfc_gpu_ctx* c, const double* host_q) {
 
 int mfc_gpu_generate_ic(mfc_gpu_ctx* c, const mfc_patch* patches, int num_patches, const double* domain) {
   if (!c) return fail(MFC_ERR_INVALID, "NULL context");
+  c->prim_of = nullptr;
   mfc::IcTarget t{c->nd,
                   c->prm.num_fluids,
                   {c->n[0], c->n[1], c->n[2]},
@@ -947,6 +980,7 @@ int mfc_gpu_tune(mfc_gpu_ctx* c, int reps, int* variant_out, double* ms_out) {
     MFC_CUDA(mfc::visc_gradients_launch(c->nd, c->prm.num_fluids, c->prm.precision != MFC_PREC_FP64, c->dev, c->vg,
                                         c->reg[0], c->stream));
   MFC_CUDA(cudaStreamSynchronize(c->stream));
+  c->prim_of = nullptr;  // the timed launches use the pairs' buffers
   const mfc::StageEntry* best = nullptr;
   int idx = -1, best_idx = -1;
   float best_ms = 0.f;
@@ -965,12 +999,20 @@ int mfc_gpu_tune(mfc_gpu_ctx* c, int reps, int* variant_out, double* ms_out) {
       continue;
     ++idx;
     if (e.prepare() != cudaSuccess) continue;
-    // first-stage launches read register 0 and write register 1 only
-    if (e.launch(c->dev, c->ucoef, c->reg[0], c->reg[0], c->reg[1], 0.0, mfc::kRkEuler, c->stream) != cudaSuccess)
-      continue;
+    // first-stage launches read register 0 and write register 1 only; with
+    // primitive pairs (of the same state, dt being 0) after the first
+    const int64_t pitch = mfc::prim_pitch(c->n[0]);
+    mfc::PrimPairs B{nullptr, c->prim[0], pitch, pitch * c->n[1]};
+    auto once = [&] {
+      if (c->prim[0] != nullptr && e.launch_prims != nullptr)
+        return e.launch_prims(c->dev, c->ucoef, c->reg[0], c->reg[0], c->reg[1], 0.0, mfc::kRkEuler, B, c->stream);
+      return e.launch(c->dev, c->ucoef, c->reg[0], c->reg[0], c->reg[1], 0.0, mfc::kRkEuler, c->stream);
+    };
+    if (once() != cudaSuccess) continue;
+    B.in = c->prim[0];
+    B.out = c->prim[1];
     cudaEventRecord(a, c->stream);
-    for (int r = 0; r < reps; ++r)
-      e.launch(c->dev, c->ucoef, c->reg[0], c->reg[0], c->reg[1], 0.0, mfc::kRkEuler, c->stream);
+    for (int r = 0; r < reps; ++r) once();
     cudaEventRecord(b, c->stream);
     if (cudaEventSynchronize(b) != cudaSuccess) break;
     float ms = 0.f;
@@ -1013,11 +1055,11 @@ int mfc_gpu_select_variant(mfc_gpu_ctx* c, int variant, int* tx, int* ty, int* t
     if (++idx != variant) continue;
     if (e.prepare() != cudaSuccess) return fail(MFC_ERR_CUDA, "tile variant does not fit on this device");
     c->stage = &e;
-    int ex = e.tx, ey = e.ty;
-    if (e.tile) e.tile(c->n, &ex, &ey);
+    int ex = e.tx, ey = e.ty, et = e.nt;
+    if (e.tile) e.tile(c->n, &ex, &ey, &et);
     if (tx) *tx = ex;
     if (ty) *ty = ey;
-    if (threads) *threads = e.nt;
+    if (threads) *threads = et;
     return MFC_OK;
   }
   return fail(MFC_ERR_INVALID, "no such tile variant for this configuration");
@@ -1120,6 +1162,8 @@ int mfc_gpu_finalize(mfc_gpu_ctx* c) {
   cudaFree(c->tables);
   cudaFree(c->status);
   cudaFree(c->work);
+  cudaFree(c->prim[0]);
+  cudaFree(c->prim[1]);
   cudaFree(c->scratch);
   cudaFree(c->vg.vel);
   cudaFree(c->vg.g);

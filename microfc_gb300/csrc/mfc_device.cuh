@@ -176,10 +176,28 @@ __device__ __forceinline__ float d2f_bits(double x) {
   return __uint_as_float(d2f_trunc_word((uint32_t)__double2hiint(x), (uint32_t)__double2loint(x)));
 }
 
+// d2f_bits for values that go on into arithmetic of the split units, which
+// flush subnormals (-ftz=true): two clamps in place of two compares and
+// selects; a result below the smallest normal float keeps subnormal bits
+// instead of becoming zero.
+__device__ __forceinline__ float d2f_ftz(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t a = min(max(hi & 0x7fffffffu, 0x38000000u), 0x47f00000u);
+  const uint32_t t = min(__funnelshift_l(lo, a - 0x38000000u, 3), 0x7f800000u);
+  return __uint_as_float(t | (hi & 0x80000000u));
+}
+
 __device__ __forceinline__ double f2d_bits(float f) {
   const uint32_t b = __float_as_uint(f);
   const uint32_t lo = (b & 0x7fffffffu) < 0x00800000u ? 0u : (b << 29);
   return __hiloint2double((int)f2d_high_word(b), (int)lo);
+}
+
+// f2d_bits of a result of the split units' arithmetic, which is never
+// subnormal: only zero needs a select, in the high word.
+__device__ __forceinline__ double f2d_ftz(float f) {
+  const uint32_t b = __float_as_uint(f);
+  return __hiloint2double((int)f2d_high_word(b), (int)(b << 29));
 }
 
 // Programmatic dependent launch.  The single-case stage kernels are launched
@@ -313,10 +331,12 @@ __device__ __forceinline__ float div_rn(float a, const DivisorF32& d) { return a
 struct Fma64 {
   double v, one, nz;
 };
-// The two constants, opaque to the compiler (eps is a run-time parameter,
-// finite and positive), so that they stay in registers.
-__device__ __forceinline__ Fma64 fma64_unit(double eps) {
-  return {0.0, __fma_rn(eps, 0.0, 1.0), __dmul_rn(eps, -0.0)};
+// The two constants, made from a loaded value (the sign of an inverse cell
+// width: 0), so that the compiler can neither fold them into constant
+// operands nor compute them again at each use when registers are short.
+__device__ __forceinline__ Fma64 fma64_unit(const double* inv_width) {
+  const int s = __double2hiint(__ldg(inv_width)) >> 31;
+  return {0.0, __hiloint2double(0x3ff00000 | s, s), __hiloint2double((int)0x80000000 | s, s)};
 }
 __device__ __forceinline__ Fma64 operator+(const Fma64& a, const Fma64& b) {
   return {__fma_rn(a.v, a.one, b.v), a.one, a.nz};
@@ -360,10 +380,10 @@ __device__ __forceinline__ Fma64 num_sqrt(const Fma64& a) { return {sqrt(a.v), a
 // compiler fuses.
 #ifdef MFC_FP64_CONTRACT
 using Num64 = double;
-__device__ __forceinline__ Num64 num64_unit(double) { return 0.0; }
+__device__ __forceinline__ Num64 num64_unit(const double*) { return 0.0; }
 #else
 using Num64 = Fma64;
-__device__ __forceinline__ Num64 num64_unit(double eps) { return fma64_unit(eps); }
+__device__ __forceinline__ Num64 num64_unit(const double* inv_width) { return fma64_unit(inv_width); }
 #endif
 
 // A coefficient record read as numbers.
@@ -471,31 +491,42 @@ __device__ __forceinline__ void monitor_max(unsigned long long* w, double v) {
 // p = (float)((E - Pi) - (double)KE) / Gamma.
 // GB300's FP64 pipe bounds the split stage, and this conversion runs on every
 // halo cell as well (1.75x the interior for 16x16 tiles).
+// The FP64 operations are DFMAs of three registers where they can be (Fma64:
+// 16 instead of 19 SM cycles each; one: the register holding 1.0), and a fluid without pi_inf (an ideal gas) adds none: its
+// products are zeros, whose sum changes nothing while the state is finite.
 template <int ND, int NF>
 __device__ __forceinline__ void cons_to_prim_split(const double (&q)[Eqs<ND, NF>::S], const DevParams& P,
-                                                   float (&out)[Eqs<ND, NF>::S]) {
+                                                   double one, float (&out)[Eqs<ND, NF>::S]) {
   using Q = Eqs<ND, NF>;
-  double pinf = 0.0;
   float rho = 0.f, gam = 0.f;
+  double e = q[Q::E];
+  bool any = false;
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
-    out[f] = d2f_bits(q[f]);
-    out[Q::ADV + f] = d2f_bits(q[Q::ADV + f]);
+    out[f] = d2f_ftz(q[f]);
+    out[Q::ADV + f] = d2f_ftz(q[Q::ADV + f]);
     rho = rho + out[f];
     gam = fmaf(out[Q::ADV + f], d2f_bits(P.gammas[f]), gam);
-    pinf = fma(q[Q::ADV + f], P.pi_infs[f], pinf);
+    any |= __double_as_longlong(P.pi_infs[f]) != 0;  // integer: a comparison would occupy the FP64 unit
+  }
+  if (any) {
+    double pinf = 0.0;
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+      if (__double_as_longlong(P.pi_infs[f]) != 0) pinf = __fma_rn(q[Q::ADV + f], P.pi_infs[f], pinf);
+    e = __fma_rn(-pinf, one, e);
   }
   rho = fmaxf(rho, 1e-16f);
   const float irho = __fdividef(1.f, rho);
   float m2 = 0.f;
 #pragma unroll
   for (int d = 0; d < ND; ++d) {
-    const float m = d2f_bits(q[Q::MOM + d]);
+    const float m = d2f_ftz(q[Q::MOM + d]);
     out[Q::MOM + d] = m * irho;
     m2 = fmaf(m, m, m2);
   }
-  const double dE = (q[Q::E] - pinf) - f2d_bits(0.5f * m2 * irho);
-  out[Q::E] = __fdividef(d2f_bits(dE), gam);
+  const double dE = __fma_rn(-f2d_bits(0.5f * m2 * irho), one, e);
+  out[Q::E] = __fdividef(d2f_ftz(dE), gam);
 }
 
 // ---------------------------------------------------------------------------
@@ -547,10 +578,11 @@ __device__ __forceinline__ f32x2 f2_rcp(f32x2 a) {
 // so nothing grows beyond the operands' range.  Mathematically identical to
 // weno_cell; rounding differs.  C(k) returns coefficient k of the cell's
 // record as a (c, c) pair.
+// The form on the cell's value v and the differences of its stencil (d1 =
+// v[4] - v[3] .. dm2 = v[1] - v[0]), which neighbouring cells share.
 template <class Coef>
-__device__ __forceinline__ void weno5_pair_fast(const Coef& C, const f32x2 (&v)[5], f32x2 eps, f32x2& vL,
-                                                f32x2& vR) {
-  const f32x2 d1 = f2_sub(v[4], v[3]), d0 = f2_sub(v[3], v[2]), dm1 = f2_sub(v[2], v[1]), dm2 = f2_sub(v[1], v[0]);
+__device__ __forceinline__ void weno5_pair_diffs(const Coef& C, f32x2 v, f32x2 d1, f32x2 d0, f32x2 dm1, f32x2 dm2,
+                                                 f32x2 eps, f32x2& vL, f32x2& vR) {
   const f32x2 b0 = f2_fma(d1, f2_fma(C(kBeta + 0), d1, f2_mul(C(kBeta + 1), d0)), f2_fma(f2_mul(C(kBeta + 2), d0), d0, eps));
   const f32x2 b1 = f2_fma(d0, f2_fma(C(kBeta + 3), d0, f2_mul(C(kBeta + 4), dm1)), f2_fma(f2_mul(C(kBeta + 5), dm1), dm1, eps));
   const f32x2 b2 = f2_fma(dm1, f2_fma(C(kBeta + 6), dm1, f2_mul(C(kBeta + 7), dm2)), f2_fma(f2_mul(C(kBeta + 8), dm2), dm2, eps));
@@ -558,15 +590,20 @@ __device__ __forceinline__ void weno5_pair_fast(const Coef& C, const f32x2 (&v)[
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
     const int kP = side ? kPR : kPL, kD = side ? kDR : kDL;
-    const f32x2 p0 = f2_fma(C(kP + 1), d0, f2_fma(C(kP + 0), d1, v[2]));
-    const f32x2 p1 = f2_fma(C(kP + 3), dm1, f2_fma(C(kP + 2), d0, v[2]));
-    const f32x2 p2 = f2_fma(C(kP + 5), dm2, f2_fma(C(kP + 4), dm1, v[2]));
+    const f32x2 p0 = f2_fma(C(kP + 1), d0, f2_fma(C(kP + 0), d1, v));
+    const f32x2 p1 = f2_fma(C(kP + 3), dm1, f2_fma(C(kP + 2), d0, v));
+    const f32x2 p2 = f2_fma(C(kP + 5), dm2, f2_fma(C(kP + 4), dm1, v));
     const f32x2 a0 = f2_mul(C(kD + 0), r0), a1 = f2_mul(C(kD + 1), r1), a2 = f2_mul(C(kD + 2), r2);
     const f32x2 is = f2_rcp(f2_add(f2_add(a0, a1), a2));
     const f32x2 val = f2_fma(f2_mul(a2, is), p2, f2_fma(f2_mul(a1, is), p1, f2_mul(f2_mul(a0, is), p0)));
     if (side) vR = val;
     else vL = val;
   }
+}
+template <class Coef>
+__device__ __forceinline__ void weno5_pair_fast(const Coef& C, const f32x2 (&v)[5], f32x2 eps, f32x2& vL,
+                                                f32x2& vR) {
+  weno5_pair_diffs(C, v[2], f2_sub(v[4], v[3]), f2_sub(v[3], v[2]), f2_sub(v[2], v[1]), f2_sub(v[1], v[0]), eps, vL, vR);
 }
 
 // WENO reconstruction of one cell from its stencil, m_weno.fpp:391-536.
@@ -943,14 +980,16 @@ __device__ __forceinline__ double rk_combine(int kind, const N& base, const N& i
 // 2 (q2 - q0 + dt r)/3 for RK3.  The increment is small next to the state,
 // so it is formed in FP32 from the FP32 right-hand side and the FP64
 // difference of the registers, and the state accumulates in FP64: one or two
-// FP64 operations per value instead of two or three.
-__device__ __forceinline__ double rk_combine_split(int kind, double base, double in, float dt, float r) {
+// FP64 operations per value instead of two or three, as three-register DFMAs
+// (Fma64; one: the register holding 1.0).
+__device__ __forceinline__ double rk_combine_split(int kind, double base, double in, float dt, float r, double one) {
+  auto diff = [&] { return d2f_ftz(__fma_rn(-base, one, in)); };
   switch (kind) {
-    case kRkEuler: return base + f2d_bits(dt * r);
-    case kRk2Final: return base + f2d_bits(0.5f * fmaf(dt, r, d2f_bits(in - base)));
-    case kRk3Mid: return base + f2d_bits(0.25f * fmaf(dt, r, d2f_bits(in - base)));
-    case kRk3Final: return base + f2d_bits((2.0f / 3.0f) * fmaf(dt, r, d2f_bits(in - base)));
-    default: return f2d_bits(r);
+    case kRkEuler: return __fma_rn(base, one, f2d_ftz(dt * r));
+    case kRk2Final: return __fma_rn(base, one, f2d_ftz(0.5f * fmaf(dt, r, diff())));
+    case kRk3Mid: return __fma_rn(base, one, f2d_ftz(0.25f * fmaf(dt, r, diff())));
+    case kRk3Final: return __fma_rn(base, one, f2d_ftz((2.0f / 3.0f) * fmaf(dt, r, diff())));
+    default: return f2d_ftz(r);
   }
 }
 

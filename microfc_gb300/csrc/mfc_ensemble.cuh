@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "mfc_device.cuh"
+#include "mfc_pair.cuh"
 #include "mfc_stage.cuh"
 
 namespace mfc {
@@ -41,15 +42,15 @@ static_assert(sizeof(EnsParams) <= 32764, "ensemble parameters must fit the kern
 // TMA: interior tiles arrive by one bulk tensor copy; the block initialises
 // its mbarrier once and alternates its phase per copied tile.
 // VISC: every case carries its viscosity parameters (DevParams::visc).
-template <int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, bool TMA, bool VISC = false>
+// RT float: pair_tile with runs of RX and RY cells; double: stage_tile.
+template <int NF, class RT, int TX, int TY, int NT, int RX, int RY, bool GATE, bool TMA, bool VISC>
 __device__ __forceinline__ void ensemble_walk(const EnsParams& E) {
-  static_assert(!VISC || !TMA, "the viscous ensemble kernels load their tiles plainly");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  static_assert(!TMA || (sizeof(RT) == 4 && !VISC), "TMA loads are compiled for the inviscid split kernels");
+  extern __shared__ __align__(128) unsigned char smem_raw[];
   uint32_t parity = 0;
   if constexpr (TMA) {
     if (E.maps != nullptr && threadIdx.x == 0)
-      mbar_init(smem_addr(tma_staging<2, NF, WO, RT, TX, TY>(smem_raw) + tma_stage_bytes<2, NF, WO, RT, TX, TY>()),
-                1);
+      mbar_init(smem_addr(pair_staging<2, NF, TX, TY, VISC>(smem_raw) + PairShape<2, NF, TX, TY, VISC>::kStageBytes), 1);
     __syncthreads();
   }
   for (int t = blockIdx.x; t < E.total_tiles; t += gridDim.x) {
@@ -75,28 +76,19 @@ __device__ __forceinline__ void ensemble_walk(const EnsParams& E) {
       in = C.reg[2], out = C.reg[0], kind = kRk3Final, reg = 2;
     }
     const TileMap* T = (TMA && E.maps != nullptr) ? E.maps + reg * E.num_cases + lo : nullptr;
-    stage_tile<2, NF, WO, RT, TX, TY, NT, GATE, VISC, UniformCoefT<2>, TMA>(
-        C.P, in, C.reg[0], out, E.last_step ? C.dt_last : C.dt, kind, x0, y0, smem_raw, &E.U, T, &parity);
+    const double dt = E.last_step ? C.dt_last : C.dt;
+    if constexpr (sizeof(RT) == 4)
+      pair_tile<2, NF, TX, TY, NT, GATE, VISC, UniformCoefT<2>, TMA, RX, RY>(
+          C.P, in, C.reg[0], out, dt, kind, x0, y0, smem_raw, &E.U, PrimPairs{}, T, &parity);
+    else
+      stage_tile<2, NF, 5, RT, TX, TY, NT, VISC>(C.P, in, C.reg[0], out, dt, kind, x0, y0, smem_raw);
     __syncthreads();  // the next tile reuses the shared memory
   }
 }
 
-template <int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, bool TMA, bool VISC = false>
-__global__ void __launch_bounds__(NT) ensemble_stage_kernel(const __grid_constant__ EnsParams E) {
-  ensemble_walk<NF, WO, RT, TX, TY, NT, GATE, TMA, VISC>(E);
-}
-
-// The same with the registers capped so that MINB blocks fit on an SM.
-template <int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, int MINB, bool TMA>
-__global__ void __launch_bounds__(NT, MINB) ensemble_stage_kernel_mb(const __grid_constant__ EnsParams E) {
-  ensemble_walk<NF, WO, RT, TX, TY, NT, GATE, TMA>(E);
-}
-
-template <int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, int MINB, bool TMA, bool VISC = false>
-constexpr auto ensemble_func() {
-  static_assert(!VISC || MINB == 1, "register-capped ensemble variants are inviscid");
-  if constexpr (MINB > 1) return &ensemble_stage_kernel_mb<NF, WO, RT, TX, TY, NT, GATE, MINB, TMA>;
-  else return &ensemble_stage_kernel<NF, WO, RT, TX, TY, NT, GATE, TMA, VISC>;
+template <int NF, class RT, int TX, int TY, int NT, int MINB, int RX, int RY, bool GATE, bool TMA, bool VISC>
+__global__ void __launch_bounds__(NT, MINB) ensemble_stage_kernel(const __grid_constant__ EnsParams E) {
+  ensemble_walk<NF, RT, TX, TY, NT, RX, RY, GATE, TMA, VISC>(E);
 }
 
 struct EnsembleEntry {
@@ -110,37 +102,37 @@ struct EnsembleEntry {
   bool visc;   // compiled with the viscous terms
 };
 
-template <int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, int MINB = 1, bool TMA = false,
-          bool VISC = false>
-cudaError_t ensemble_launch(const EnsParams& E, int grid, size_t smem, cudaStream_t st) {
-  ensemble_func<NF, WO, RT, TX, TY, NT, GATE, MINB, TMA, VISC>()<<<grid, NT, smem, st>>>(E);
-  return cudaGetLastError();
-}
-
-template <int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, bool TMA, bool VISC = false>
-constexpr size_t ensemble_smem(bool shared_coef) {
-  return stage_smem_total<2, NF, WO, RT, TX, TY, NT, GATE, VISC, TMA>(shared_coef);
-}
-
-// prec: 0 FP64, 1 split, 2 split with the learned gate
-template <int NF, int WO, class RT, int TX, int TY, int NT, bool GATE = false, int MINB = 1, bool TMA = false,
-          bool VISC = false>
+// MINB: blocks per SM that the registers must allow; RX, RY: run lengths of
+// the split kernels.
+template <int NF, class RT, int TX, int TY, int NT, int MINB, int RX = 1, int RY = 1, bool GATE = false,
+          bool TMA = false, bool VISC = false>
 EnsembleEntry ensemble_entry() {
-  using Sh = StageShape<2, NF, WO, RT, TX, TY>;
-  return EnsembleEntry{NF,
-                       WO,
-                       sizeof(RT) == 8 ? 0 : (GATE ? 2 : 1),
-                       TX,
-                       TY,
-                       NT,
-                       ensemble_smem<NF, WO, RT, TX, TY, NT, GATE, TMA, VISC>(false),
-                       ensemble_smem<NF, WO, RT, TX, TY, NT, GATE, TMA, VISC>(true),
-                       reinterpret_cast<const void*>(ensemble_func<NF, WO, RT, TX, TY, NT, GATE, MINB, TMA, VISC>()),
-                       &ensemble_launch<NF, WO, RT, TX, TY, NT, GATE, MINB, TMA, VISC>,
-                       TMA,
-                       TmaBox<TX, Sh::H>::kWidth,
-                       Sh::LY,
-                       VISC};
+  struct K {
+    static constexpr auto func() { return &ensemble_stage_kernel<NF, RT, TX, TY, NT, MINB, RX, RY, GATE, TMA, VISC>; }
+    static constexpr size_t smem(bool shared_coef) {
+      if constexpr (sizeof(RT) == 4) return pair_smem<2, NF, TX, TY, NT, GATE, VISC, TMA>(shared_coef);
+      else return stage_smem_total<2, NF, 5, RT, TX, TY, VISC, false>();
+    }
+  };
+  EnsembleEntry e{};
+  e.nf = NF;
+  e.wo = 5;
+  e.prec = sizeof(RT) == 8 ? 0 : (GATE ? 2 : 1);
+  e.tx = TX;
+  e.ty = TY;
+  e.nt = NT;
+  e.smem = K::smem(false);
+  e.smem_shared_coef = K::smem(true);
+  e.func = reinterpret_cast<const void*>(K::func());
+  e.launch = [](const EnsParams& E, int grid, size_t smem, cudaStream_t st) {
+    K::func()<<<grid, NT, smem, st>>>(E);
+    return cudaGetLastError();
+  };
+  e.tma = TMA;
+  e.box_w = TmaBox<TX, 3>::kWidth;
+  e.box_h = TY + 6;
+  e.visc = VISC;
+  return e;
 }
 
 void register_ensemble_fp64(std::vector<EnsembleEntry>& r);

@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(NT) flex_kernel(const DevParams P, const doubl
   const int LX = tw + 2 * H, LY = ND > 1 ? th + 2 * H : 1, LXY = LX * LY;
   const int NCX = tw + 2, NCY = ND > 1 ? th + 2 : 0;
   const int HY = ND > 1 ? H : 0;
-  const N u0 = num64_unit(P.weno_eps);
+  const N u0 = num64_unit(P.inv_d[0]);
   auto num = [&](double x) { return lift(x, u0); };
   // x values: position c = 0 .. tw+1 (cell x0-1+c) of row; y values: position c of column
   auto wxi = [&](int v, int row, int c) { return (v * th + row) * NCX + c; };
@@ -122,34 +122,9 @@ __global__ void __launch_bounds__(NT) flex_kernel(const DevParams P, const doubl
     // tile that the viscous cross derivatives use
     const bool hx = lx < H || lx >= H + tw, hy = ND > 1 && (ly < H || ly >= H + th);
     if (hx && hy && !(VISC && (lx == H - 1 || lx == H + tw) && (ly == H - 1 || ly == H + th))) continue;
-    bool fx = false, fy = false;
-    const int rx = x0 - H + lx, ry = ND > 1 ? y0 - H + ly : 0;
-    // processor boundaries: ghost cells come from the neighbour's halo buffer
-    // (y strips are nx + 2 wide: the x ghost cells -1 and nx first and last;
-    // the depth stays below H, since the tile's halo is H deep)
-    const int px = rx < 0 ? (P.bc_beg[0] >= 0 ? 0 : -1) : (rx >= nx && P.bc_end[0] >= 0 ? 1 : -1);
-    const int py = ND > 1 ? (ry < 0 ? (P.bc_beg[1] >= 0 ? 0 : -1) : (ry >= ny && P.bc_end[1] >= 0 ? 1 : -1)) : -1;
-    const double* src;
-    int64_t vs = P.sv;
-    if (px >= 0 && py >= 0) {
-      const int d = py == 0 ? -1 - ry : ry - ny;
-      src = P.halo[2 + py] + (int64_t)d * (nx + 2) + (px == 0 ? 0 : nx + 1);
-      vs = (int64_t)H * (nx + 2);
-    } else if (px >= 0) {
-      const int d = px == 0 ? -1 - rx : rx - nx;
-      const int yy = ND > 1 ? map_cell(ry, ny, P.bc_beg[1], P.bc_end[1], &fy) : 0;
-      src = P.halo[px] + (int64_t)yy * H + d;
-      vs = (int64_t)ny * H;
-    } else if (py >= 0) {
-      const int d = py == 0 ? -1 - ry : ry - ny;
-      const int xx = map_cell(rx, nx, P.bc_beg[0], P.bc_end[0], &fx);
-      src = P.halo[2 + py] + (int64_t)d * (nx + 2) + xx + 1;
-      vs = (int64_t)H * (nx + 2);
-    } else {
-      const int gx = map_cell(rx, nx, P.bc_beg[0], P.bc_end[0], &fx);
-      const int gy = ND > 1 ? map_cell(ry, ny, P.bc_beg[1], P.bc_end[1], &fy) : 0;
-      src = qin + (int64_t)gy * P.sy + gx;
-    }
+    bool fx, fy;
+    int64_t vs;
+    const double* src = tile_cell<ND, H>(P, qin, x0 - H + lx, ND > 1 ? y0 - H + ly : 0, vs, fx, fy);
     double q[S];
 #pragma unroll
     for (int v = 0; v < S; ++v) q[v] = __ldg(src + v * vs);
@@ -467,7 +442,7 @@ __global__ void __launch_bounds__(NT) flex_sweep_kernel(const DevParams P, const
   double* const wl = sq + S * tb * (ta + 2 * H);
   double* const wr = wl + S * NP * NCA;
   double* const cf = wl + 2 * S * tb * (ta + 2);  // [kNumCoef][NCA]
-  const N u0 = num64_unit(P.weno_eps);
+  const N u0 = num64_unit(P.inv_d[0]);
   auto num = [&](double x) { return lift(x, u0); };
   const int sa = DIR == 0 ? 1 : NP;  // stride along the sweep
   auto qi = [&](int v, int p, int la) { return DIR == 0 ? (v * NP + p) * LA + la : (v * LA + la) * NP + p; };

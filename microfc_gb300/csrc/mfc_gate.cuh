@@ -83,16 +83,16 @@ __device__ __forceinline__ double weno5_weight_deviation(const double* __restric
 }
 
 // WENO5 with the optimal linear weights d_k (the gate's "smooth" branch),
-// two variables at once (weno5_pair_fast's packed pairs).
+// two variables at once (weno5_pair_diffs' packed pairs).
 template <class Coef>
-__device__ __forceinline__ void weno5_pair_linear(const Coef& C, const f32x2 (&v)[5], f32x2& vL, f32x2& vR) {
-  const f32x2 d1 = f2_sub(v[4], v[3]), d0 = f2_sub(v[3], v[2]), dm1 = f2_sub(v[2], v[1]), dm2 = f2_sub(v[1], v[0]);
+__device__ __forceinline__ void weno5_pair_linear(const Coef& C, f32x2 v, f32x2 d1, f32x2 d0, f32x2 dm1, f32x2 dm2,
+                                                  f32x2& vL, f32x2& vR) {
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
     const int kP = side ? kPR : kPL, kD = side ? kDR : kDL;
-    const f32x2 p0 = f2_fma(C(kP + 1), d0, f2_fma(C(kP + 0), d1, v[2]));
-    const f32x2 p1 = f2_fma(C(kP + 3), dm1, f2_fma(C(kP + 2), d0, v[2]));
-    const f32x2 p2 = f2_fma(C(kP + 5), dm2, f2_fma(C(kP + 4), dm1, v[2]));
+    const f32x2 p0 = f2_fma(C(kP + 1), d0, f2_fma(C(kP + 0), d1, v));
+    const f32x2 p1 = f2_fma(C(kP + 3), dm1, f2_fma(C(kP + 2), d0, v));
+    const f32x2 p2 = f2_fma(C(kP + 5), dm2, f2_fma(C(kP + 4), dm1, v));
     const f32x2 val = f2_fma(C(kD + 2), p2, f2_fma(C(kD + 1), p1, f2_mul(C(kD + 0), p0)));
     if (side) vR = val;
     else vL = val;

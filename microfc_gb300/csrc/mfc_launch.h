@@ -14,6 +14,7 @@
 #include "../../include/mfc_gpu.h"
 #include "mfc_device.cuh"
 #include "mfc_flex.cuh"
+#include "mfc_pair.cuh"
 #include "mfc_stage.cuh"
 #include "mfc_sweep.cuh"
 
@@ -30,8 +31,11 @@ struct StageEntry {
   bool visc = false;  // compiled with the viscous terms
   bool tma = false;   // interior tiles staged by a TMA bulk tensor copy
   bool chr = false;   // WENO of the characteristic fields (MFC_RECON_CHARACTERISTIC)
-  // the tile of a grid of n[0] x n[1] x n[2] cells where the launch chooses it (else tx, ty)
-  void (*tile)(const int* n, int* tx, int* ty) = nullptr;
+  // the same launch with primitive pairs (mfc_pair.cuh); null: the kernel has no use for them
+  cudaError_t (*launch_prims)(const DevParams& P, const UniformCoef& U, const double* qin, const double* qbase,
+                              double* qout, double dt, int kind, const PrimPairs& B, cudaStream_t st) = nullptr;
+  // the tile and threads of a grid of n[0] x n[1] x n[2] cells where the launch chooses them (else tx, ty, nt)
+  void (*tile)(const int* n, int* tx, int* ty, int* nt) = nullptr;
 };
 
 // Launches a stage kernel with programmatic stream serialization, so that
@@ -53,78 +57,141 @@ cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// MINB > 1 selects the register-capped kernel (stage_kernel_mb); TMA the
-// kernel that stages interior tiles with a bulk tensor copy; FMA the
-// instantiations compiled with multiply-add contraction (MFC_PREC_FP64_FMA).
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, int MINB, bool VISC, bool TMA = false,
-          bool FMA = false, bool CHAR = false>
-constexpr auto stage_func() {
-  static_assert(MINB == 1 || !VISC || !TMA, "register-capped viscous variants load their tiles without TMA");
-  static_assert(!TMA || (ND == 2 && !VISC), "TMA staging is compiled for the inviscid 2-D kernel");
-  static_assert(!CHAR || (!TMA && MINB == 1), "characteristic-field WENO uses the plain stage kernel");
-  if constexpr (TMA && MINB > 1) return &stage_kernel_tma_mb<ND, NF, WO, RT, TX, TY, NT, GATE, MINB, FMA>;
-  else if constexpr (TMA) return &stage_kernel_tma<ND, NF, WO, RT, TX, TY, NT, GATE, FMA>;
-  else if constexpr (MINB > 1) return &stage_kernel_mb<ND, NF, WO, RT, TX, TY, NT, GATE, MINB, FMA, VISC>;
-  else return &stage_kernel<ND, NF, WO, RT, TX, TY, NT, GATE, VISC, FMA, CHAR>;
-}
-
-// Dynamic shared memory of a launch: without the coefficient records on a
-// uniform grid; a TMA kernel's records sit past its staging area.
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, bool VISC, bool TMA>
-constexpr size_t stage_launch_smem(bool shared_coef) {
-  return stage_smem_total<ND, NF, WO, RT, TX, TY, NT, GATE, VISC, TMA>(shared_coef);
-}
-
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE = false, int MINB = 1, bool VISC = false,
-          bool TMA = false, bool FMA = false, bool CHAR = false>
-cudaError_t stage_prepare() {
-  return cudaFuncSetAttribute(stage_func<ND, NF, WO, RT, TX, TY, NT, GATE, MINB, VISC, TMA, FMA, CHAR>(),
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)stage_launch_smem<ND, NF, WO, RT, TX, TY, NT, GATE, VISC, TMA>(false));
-}
-
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE = false, int MINB = 1, bool VISC = false,
-          bool TMA = false, bool FMA = false, bool CHAR = false>
-cudaError_t stage_launch(const DevParams& P, const UniformCoef& U, const double* qin, const double* qbase,
-                         double* qout, double dt, int kind, cudaStream_t st) {
-  const dim3 grid((unsigned)((P.n[0] + TX - 1) / TX), ND > 1 ? (unsigned)((P.n[1] + TY - 1) / TY) : 1u, 1u);
-  // a uniform grid stages no coefficient records: launch without their share
-  const bool shared_coef = U.on[0] && (ND < 2 || U.on[1]);
-  const size_t smem = stage_launch_smem<ND, NF, WO, RT, TX, TY, NT, GATE, VISC, TMA>(shared_coef);
-  if constexpr (TMA) {
-    // the map of this launch's input register; without one (a layout the
-    // copy engine does not take) every tile takes the plain loads
-    using Sh = StageShape<ND, NF, WO, RT, TX, TY>;
-    TileMap T{};
-    encode_tile_map(T, qin, P.n[0], P.n[1], Sh::S, P.sy, P.sv, TmaBox<TX, Sh::H>::kWidth, Sh::LY);
-    return launch_dependent(stage_func<ND, NF, WO, RT, TX, TY, NT, GATE, MINB, VISC, TMA, FMA, CHAR>(), grid, dim3(NT), smem,
-                            st, P, U, T, qin, qbase, qout, dt, kind);
-  } else {
-    return launch_dependent(stage_func<ND, NF, WO, RT, TX, TY, NT, GATE, MINB, VISC, TMA, FMA, CHAR>(), grid, dim3(NT), smem,
-                            st, P, U, qin, qbase, qout, dt, kind);
-  }
-}
-
-// prec of a registry entry: 0 FP64, 1 split, 2 split with the learned gate,
-// 3 FP64 with multiply-add contraction
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE = false, int MINB = 1, bool VISC = false,
-          bool TMA = false, bool FMA = false, bool CHAR = false>
+// TMA selects the kernel that stages interior tiles with a bulk tensor copy;
+// FMA the instantiations compiled with multiply-add contraction
+// (MFC_PREC_FP64_FMA); CHAR WENO of the characteristic fields.
+template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool TMA = false, bool FMA = false,
+          bool CHAR = false>
 StageEntry stage_entry() {
   static_assert(!FMA || sizeof(RT) == 8, "the contracted variant is FP64");
-  return StageEntry{ND,
-                    NF,
-                    WO,
-                    FMA ? 3 : sizeof(RT) == 8 ? 0 : (GATE ? 2 : 1),
-                    TX,
-                    TY,
-                    NT,
-                    stage_launch_smem<ND, NF, WO, RT, TX, TY, NT, GATE, VISC, TMA>(false),
-                    1,
-                    &stage_prepare<ND, NF, WO, RT, TX, TY, NT, GATE, MINB, VISC, TMA, FMA, CHAR>,
-                    &stage_launch<ND, NF, WO, RT, TX, TY, NT, GATE, MINB, VISC, TMA, FMA, CHAR>,
-                    VISC,
-                    TMA,
-                    CHAR};
+  static_assert(!TMA || (ND == 2 && !CHAR), "TMA staging is compiled for the inviscid 2-D kernel");
+  struct K {
+    static constexpr auto func() {
+      if constexpr (TMA) return &stage_kernel_tma<ND, NF, WO, RT, TX, TY, NT, FMA>;
+      else return &stage_kernel<ND, NF, WO, RT, TX, TY, NT, FMA, CHAR>;
+    }
+    static constexpr size_t smem() { return stage_smem_total<ND, NF, WO, RT, TX, TY, false, TMA>(); }
+  };
+  StageEntry e{};
+  e.nd = ND;
+  e.nf = NF;
+  e.wo = WO;
+  e.prec = FMA ? MFC_PREC_FP64_FMA : sizeof(RT) == 8 ? MFC_PREC_FP64 : MFC_PREC_SPLIT;
+  e.tx = TX;
+  e.ty = TY;
+  e.nt = NT;
+  e.smem = K::smem();
+  e.kernels = 1;
+  e.prepare = [] {
+    return cudaFuncSetAttribute(K::func(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::smem());
+  };
+  e.launch = [](const DevParams& P, const UniformCoef&, const double* qin, const double* qbase, double* qout,
+                double dt, int kind, cudaStream_t st) {
+    const dim3 grid((unsigned)((P.n[0] + TX - 1) / TX), ND > 1 ? (unsigned)((P.n[1] + TY - 1) / TY) : 1u);
+    if constexpr (TMA) {
+      // the map of this launch's input register; without one (a layout the
+      // copy engine does not take) every tile takes the plain loads
+      using Sh = StageShape<ND, NF, WO, RT, TX, TY>;
+      TileMap T{};
+      encode_tile_map(T, qin, P.n[0], P.n[1], Sh::S, P.sy, P.sv, TmaBox<TX, Sh::H>::kWidth, Sh::LY);
+      return launch_dependent(K::func(), grid, dim3(NT), K::smem(), st, P, T, qin, qbase, qout, dt, kind);
+    } else {
+      return launch_dependent(K::func(), grid, dim3(NT), K::smem(), st, P, qin, qbase, qout, dt, kind);
+    }
+  };
+  e.tma = TMA;
+  e.chr = CHAR;
+  return e;
+}
+
+// The split WENO5 kernels of 1-D and 2-D cases (mfc_pair.cuh).
+template <int ND, int NF, int TX, int TY, int NT, int MINB, int RX, int RY, bool GATE = false, bool VISC = false,
+          bool TMA = false>
+StageEntry pair_entry() {
+  static_assert(!TMA || ND == 2, "TMA loads are compiled for the 2-D kernel");
+  struct K {
+    static constexpr auto func() {
+      if constexpr (TMA) return &pair_kernel_tma<NF, TX, TY, NT, GATE, VISC, MINB, RX, RY>;
+      else return &pair_kernel<ND, NF, TX, TY, NT, GATE, VISC, MINB, RX, RY>;
+    }
+  };
+  StageEntry e{};
+  e.nd = ND;
+  e.nf = NF;
+  e.wo = 5;
+  e.prec = GATE ? MFC_PREC_GATED : MFC_PREC_SPLIT;
+  e.tx = TX;
+  e.ty = TY;
+  e.nt = NT;
+  e.smem = pair_smem<ND, NF, TX, TY, NT, GATE, VISC, TMA>(false);
+  e.kernels = 1;
+  e.prepare = [] {
+    return cudaFuncSetAttribute(K::func(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)pair_smem<ND, NF, TX, TY, NT, GATE, VISC, TMA>(false));
+  };
+  e.launch_prims = [](const DevParams& P, const UniformCoef& U, const double* qin, const double* qbase, double* qout,
+                      double dt, int kind, const PrimPairs& B, cudaStream_t st) {
+    const dim3 grid((unsigned)((P.n[0] + TX - 1) / TX), ND > 1 ? (unsigned)((P.n[1] + TY - 1) / TY) : 1u);
+    // a uniform grid stages no coefficient records: launch without their share
+    const size_t smem = pair_smem<ND, NF, TX, TY, NT, GATE, VISC, TMA>(U.on[0] && (ND < 2 || U.on[1]));
+    if constexpr (TMA) {
+      // the map of this launch's input; without one (a layout the copy engine
+      // does not take) every tile takes the plain loads
+      using Sh = PairShape<ND, NF, TX, TY, VISC>;
+      TileMap T{};
+      if (B.in != nullptr)
+        encode_tile_map(T, reinterpret_cast<const double*>(B.in), (int)B.pitch, P.n[1], Sh::NPR, B.pitch, B.plane,
+                        Sh::LX, Sh::LY);
+      else
+        encode_tile_map(T, qin, P.n[0], P.n[1], Sh::S, P.sy, P.sv, TmaBox<TX, Sh::H>::kWidth, Sh::LY);
+      return launch_dependent(K::func(), grid, dim3(NT), smem, st, P, U, T, qin, qbase, qout, dt, kind, B);
+    } else {
+      return launch_dependent(K::func(), grid, dim3(NT), smem, st, P, U, qin, qbase, qout, dt, kind, B);
+    }
+  };
+  e.launch = [](const DevParams& P, const UniformCoef& U, const double* qin, const double* qbase, double* qout,
+                double dt, int kind, cudaStream_t st) {
+    return pair_entry<ND, NF, TX, TY, NT, MINB, RX, RY, GATE, VISC, TMA>().launch_prims(P, U, qin, qbase, qout, dt, kind,
+                                                                                        PrimPairs{}, st);
+  };
+  e.visc = VISC;
+  e.tma = TMA;
+  return e;
+}
+
+// Two pair entries as one: tiles of 8x8 cells where 16x16 ones are too few
+// to fill the chip (kSmallTiles of them or less), else 16x16.  Where the line
+// lies (us a step, 8x8 and 16x16): 100x50 (28 tiles) 14.6 and 19.0, 333x167
+// (231) 22.5 and 27.9, 400x200 (325) 31.9 and 31.9, 512x256 (512) 45.4 and
+// 37.5.
+constexpr int64_t kSmallTiles = 320;
+template <class Small, class Large>
+StageEntry sized_entry(const Small&, const Large&) {
+  StageEntry e = Large::entry();
+  e.prepare = [] {
+    const cudaError_t r = Small::entry().prepare();
+    return r != cudaSuccess ? r : Large::entry().prepare();
+  };
+  struct Pick {
+    static bool small(const int* n) {
+      return (int64_t)((n[0] + 15) / 16) * ((n[1] + 15) / 16) <= kSmallTiles;
+    }
+  };
+  e.launch = [](const DevParams& P, const UniformCoef& U, const double* qin, const double* qbase, double* qout,
+                double dt, int kind, cudaStream_t st) {
+    return (Pick::small(P.n) ? Small::entry() : Large::entry()).launch(P, U, qin, qbase, qout, dt, kind, st);
+  };
+  e.launch_prims = [](const DevParams& P, const UniformCoef& U, const double* qin, const double* qbase, double* qout,
+                      double dt, int kind, const PrimPairs& B, cudaStream_t st) {
+    return (Pick::small(P.n) ? Small::entry() : Large::entry()).launch_prims(P, U, qin, qbase, qout, dt, kind, B, st);
+  };
+  e.tile = [](const int* n, int* tx, int* ty, int* nt) {
+    const StageEntry c = Pick::small(n) ? Small::entry() : Large::entry();
+    *tx = c.tx;
+    *ty = c.ty;
+    *nt = c.nt;
+  };
+  return e;
 }
 
 // Tile sizes of the flex kernels: the ones with the least work on the
@@ -254,10 +321,11 @@ StageEntry flex_entry() {
                             st, P, qin, qbase, qout, dt, kind, t.x, t.y);
   };
   e.visc = VISC;
-  e.tile = [](const int* n, int* tx, int* ty) {
+  e.tile = [](const int* n, int* tx, int* ty, int* nt) {
     const flex::Plan t = flex::plan<ND, NF, WO, NT, VISC>(n[0], n[1]);
     *tx = t.x;
     *ty = t.y;
+    *nt = NT;
   };
   return e;
 }
@@ -296,10 +364,11 @@ StageEntry flex_sweep_entry() {
     if (r == cudaSuccess) r = sweep(std::integral_constant<int, 2>{});
     return r;
   };
-  e.tile = [](const int* n, int* tx, int* ty) {  // the x sweep's
+  e.tile = [](const int* n, int* tx, int* ty, int* nt) {  // the x sweep's
     const flex::Plan t = flex::sweep_plan<NF, WO, NT, 0>(n[0], n[1], n[2]);
     *tx = t.x;
     *ty = t.y;
+    *nt = NT;
   };
   return e;
 }

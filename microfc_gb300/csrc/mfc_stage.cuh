@@ -20,7 +20,6 @@
 #include <type_traits>
 
 #include "mfc_device.cuh"
-#include "mfc_gate.cuh"
 #include "mfc_tma.cuh"
 
 namespace mfc {
@@ -78,15 +77,10 @@ struct StageShape {
   static constexpr int TYE = (ND > 1) ? TY : 1;
   static constexpr int LX = TX + 2 * H;
   static constexpr int LY = (ND > 1) ? TY + 2 * H : 1;
-  // split WENO5 keeps the primitive variables and the WENO values in
-  // interleaved pairs (2p, 2p+1), reconstructed two at a time with packed
-  // FP32 instructions; SP counts the variables with the padding one
-  static constexpr bool PAIR = sizeof(RT) == 4 && WO == 5;
-  static constexpr int SP = PAIR ? (S + 1) / 2 * 2 : S;
-  static constexpr int NQ = SP * LY * LX;  // primitive tile
+  static constexpr int NQ = S * LY * LX;  // primitive tile
   // WENO outputs (left and right face values), x and y layouts share space
-  static constexpr int NWX = SP * TYE * (TX + 2);
-  static constexpr int NWY = (ND > 1) ? SP * (TY + 2) * TX : 0;
+  static constexpr int NWX = S * TYE * (TX + 2);
+  static constexpr int NWY = (ND > 1) ? S * (TY + 2) * TX : 0;
   static constexpr int NW = NWX > NWY ? NWX : NWY;
   // fluxes + interface velocity (+ the viscous x-momentum, y-momentum and
   // energy source fluxes)
@@ -94,40 +88,59 @@ struct StageShape {
   static constexpr int NFX = NR * TYE * (TX + 1);
   static constexpr int NFY = (ND > 1) ? NR * (TY + 1) * TX : 0;
   static constexpr int NFL = NFX > NFY ? NFX : NFY;
-  // split precision: the tile's WENO coefficients, converted to FP32 once and
-  // stored as one 16-byte aligned record of kCoefRec floats per cell, so that
-  // a WENO evaluation loads them with 7 vector loads
   static constexpr int NCX = TX + 2, NCY = (ND > 1) ? TY + 2 : 0;
-  static constexpr int NCOEF = (sizeof(RT) == 4 && WO == 5) ? kCoefRec * (NCX + NCY) : 0;
   // FP64 WENO5: the tile's coefficients as doubles in [k][cell] order (x
   // cells, then y cells), staged once per tile so that the reconstructions
   // read them from shared memory instead of issuing kNumCoef global loads
   // each
-  static constexpr int NCOEF64 = (sizeof(RT) == 8 && WO == 5) ? kNumCoef * (NCX + NCY) : 0;
+  static constexpr int NCOEF = (sizeof(RT) == 8 && WO == 5) ? kNumCoef * (NCX + NCY) : 0;
   // offsets (in RT elements) of the arrays, each rounded up to 16 bytes
   static constexpr int align16(int n) { return (n * int(sizeof(RT)) + 15) / 16 * 16 / int(sizeof(RT)); }
   static constexpr int OW = align16(NQ), OF = OW + 2 * align16(NW), OC = OF + align16(NFL);
-  // layout: [primitive tile, WENO values, fluxes][learned gate][coefficient
-  // records]; the records come last so that a uniform grid, which never
-  // stages them, can launch without their share
+  // layout: primitive tile, WENO values, fluxes, coefficients
   static constexpr size_t kMainBytes = sizeof(RT) * size_t(OC);
-  static constexpr size_t kCoefBytes = sizeof(RT) * size_t(NCOEF + NCOEF64);
+  static constexpr size_t kCoefBytes = sizeof(RT) * size_t(NCOEF);
   static constexpr size_t kSmemBytes = kMainBytes + kCoefBytes;
 };
 
-// Shared memory of the learned gate.  Its own region holds one flag per
-// (cell, direction) reconstructed by the tile.  The gate phase's scratch --
-// one 16x16 FP16 input block per warp, then the MLP's lane fragments
-// (kGateFragWords words per lane, word-major) -- lives in the WENO value
-// arrays, which are not written before the gate phase ends.
-template <int ND, int TX, int TY, int NT>
-struct GateShape {
-  static constexpr int NGX = (TX + 2) * ((ND > 1) ? TY : 1);
-  static constexpr int NGY = (ND > 1) ? TX * (TY + 2) : 0;
-  static constexpr size_t kFragOff = size_t(NT / 32) * 512;
-  static constexpr size_t kScratchBytes = kFragOff + size_t(kGateFragWords) * 32 * 4;
-  static constexpr size_t kBytes = ((NGX + NGY + 15) / 16) * 16;
-};
+// Where a tile finds the cell (rx, ry), inside the domain or up to H cells
+// outside: the interior cell that a ghost cell mirrors (fx, fy: the normal
+// momentum changes sign), or the halo buffer of a processor boundary.  vs:
+// the stride between variables there.  Cells of partial edge tiles beyond the
+// first H ghosts are never stored: their depth is clamped.  y strips are
+// nx + 2 wide (the x ghost cells -1 and nx of the neighbour's rows come first
+// and last).
+template <int ND, int H>
+__device__ __forceinline__ const double* tile_cell(const DevParams& P, const double* __restrict__ qin, const int rx,
+                                                   const int ry, int64_t& vs, bool& fx, bool& fy) {
+  const int nx = P.n[0], ny = P.n[1];
+  fx = fy = false;
+  vs = P.sv;
+  const int px = rx < 0 ? (P.bc_beg[0] >= 0 ? 0 : -1) : (rx >= nx && P.bc_end[0] >= 0 ? 1 : -1);
+  const int py = ND > 1 ? (ry < 0 ? (P.bc_beg[1] >= 0 ? 0 : -1) : (ry >= ny && P.bc_end[1] >= 0 ? 1 : -1)) : -1;
+  if (px >= 0 && py >= 0) {
+    // between two processor boundaries (the viscous corner cells): the
+    // diagonal neighbour's cell, forwarded by the y neighbour
+    const int d = min(py == 0 ? -1 - ry : ry - ny, H - 1);
+    vs = (int64_t)H * (nx + 2);
+    return P.halo[2 + py] + (int64_t)d * (nx + 2) + (px == 0 ? 0 : nx + 1);
+  }
+  if (px >= 0) {
+    const int d = min(px == 0 ? -1 - rx : rx - nx, H - 1);
+    const int yy = ND > 1 ? map_cell(ry, ny, P.bc_beg[1], P.bc_end[1], &fy) : 0;
+    vs = (int64_t)ny * H;
+    return P.halo[px] + (int64_t)yy * H + d;
+  }
+  if (py >= 0) {
+    const int d = min(py == 0 ? -1 - ry : ry - ny, H - 1);
+    const int xx = map_cell(rx, nx, P.bc_beg[0], P.bc_end[0], &fx);
+    vs = (int64_t)H * (nx + 2);
+    return P.halo[2 + py] + (int64_t)d * (nx + 2) + xx + 1;
+  }
+  const int gx = map_cell(rx, nx, P.bc_beg[0], P.bc_end[0], &fx);
+  const int gy = ND > 1 ? map_cell(ry, ny, P.bc_beg[1], P.bc_end[1], &fy) : 0;
+  return qin + gy * P.sy + gx;
+}
 
 // The TMA staging area of a stage tile (2-D): after the primitive tile,
 // 128-byte aligned, the box of all variables, then its mbarrier and a flag.
@@ -143,14 +156,13 @@ constexpr uint32_t tma_stage_bytes() {
   return uint32_t(TmaBox<TX, Sh::H>::kWidth) * Sh::LY * Sh::S * 8;
 }
 
-// Offset of the split path's coefficient records in a block's shared
-// memory: after the main arrays and the gate's flags, and after the TMA
-// staging area (worst-case alignment) of a TMA kernel, so that records
-// staged before the copy lands are not overwritten.
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, bool VISC, bool TMA>
+// Offset of the coefficients in a block's shared memory: after the main arrays
+// and, in a TMA kernel, after the staging area (worst-case alignment), so that
+// coefficients staged before the copy lands are not overwritten.
+template <int ND, int NF, int WO, class RT, int TX, int TY, bool VISC, bool TMA>
 constexpr size_t stage_coef_offset() {
   using Sh = StageShape<ND, NF, WO, RT, TX, TY, VISC>;
-  size_t o = Sh::kMainBytes + (GATE ? GateShape<ND, TX, TY, NT>::kBytes : 0);
+  size_t o = Sh::kMainBytes;
   if constexpr (TMA) {
     const size_t t =
         (sizeof(RT) * size_t(Sh::OW) + 128 + tma_stage_bytes<ND, NF, WO, RT, TX, TY>() + 16 + 15) / 16 * 16;
@@ -159,14 +171,11 @@ constexpr size_t stage_coef_offset() {
   return o;
 }
 
-// Dynamic shared memory of one block: without the split path's coefficient
-// records when the grid is uniform (every direction reads the shared
-// record); the FP64 coefficients are always staged.
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, bool VISC, bool TMA>
-constexpr size_t stage_smem_total(bool shared_coef) {
-  using Sh = StageShape<ND, NF, WO, RT, TX, TY, VISC>;
-  return stage_coef_offset<ND, NF, WO, RT, TX, TY, NT, GATE, VISC, TMA>() +
-         (shared_coef && Sh::NCOEF64 == 0 ? 0 : Sh::kCoefBytes);
+// Dynamic shared memory of one block.
+template <int ND, int NF, int WO, class RT, int TX, int TY, bool VISC, bool TMA>
+constexpr size_t stage_smem_total() {
+  return stage_coef_offset<ND, NF, WO, RT, TX, TY, VISC, TMA>() +
+         StageShape<ND, NF, WO, RT, TX, TY, VISC>::kCoefBytes;
 }
 
 // WENO of the characteristic fields at one position (FP64): the stencil of
@@ -250,17 +259,15 @@ __device__ __forceinline__ void char_weno_position(const double (&c)[kCoefRec], 
 // One tile of one RK stage; the tile's first cell is (x0, y0).  Used by the
 // single-case kernel (one tile per block) and by the ensemble kernel (many
 // tiles of many cases per persistent block).  smem_raw must hold
-// stage_smem_total() (of shared_coef = true when U covers every
-// direction).
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE = false, bool VISC = false,
-          class UC = UniformCoef, bool TMA = false, bool CHAR = false>
+// stage_smem_total().
+template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool VISC = false, bool TMA = false,
+          bool CHAR = false>
 __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __restrict__ qin,
                                            const double* __restrict__ qbase, double* __restrict__ qout,
                                            const double dt, const int kind, const int x0, const int y0,
-                                           unsigned char* smem_raw, const UC* U = nullptr,
-                                           const TileMap* T = nullptr, uint32_t* tma_parity = nullptr) {
-  static_assert(!GATE || (sizeof(RT) == 4 && WO == 5), "the learned gate runs on the split-precision WENO5 path");
-  static_assert(!CHAR || (sizeof(RT) == 8 && WO > 1 && !VISC && !GATE && ND < 3),
+                                           unsigned char* smem_raw, const TileMap* T = nullptr) {
+  static_assert(sizeof(RT) == 8 || WO < 5, "split-precision WENO5 is pair_tile (mfc_pair.cuh)");
+  static_assert(!CHAR || (sizeof(RT) == 8 && WO > 1 && !VISC && ND < 3),
                 "characteristic-field WENO is compiled for the inviscid FP64 1-D/2-D WENO3/5 kernel");
   using Sh = StageShape<ND, NF, WO, RT, TX, TY, VISC>;
   using Q = Eqs<ND, NF>;
@@ -274,29 +281,23 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
   using N = std::conditional_t<kSplit, float, Num64>;
   N u0;
   if constexpr (kSplit) u0 = 0.f;
-  else u0 = num64_unit(P.weno_eps);
+  else u0 = num64_unit(P.inv_d[0]);
   auto num = [&](RT x) { return lift(x, u0); };
+  const double one = kSplit ? fma64_unit(P.inv_d[0]).one : 1.0;  // split: the FP64 sums' register operand
+  (void)one;
 
-  RT* sq = reinterpret_cast<RT*>(smem_raw);  // [S][LY][LX] primitive ([S/2][LY][LX][2] in pairs)
+  RT* sq = reinterpret_cast<RT*>(smem_raw);  // [S][LY][LX] primitive
   RT* wl = sq + Sh::OW;                       // left-face values
   RT* wr = wl + Sh::align16(Sh::NW);          // right-face values
   RT* fl = sq + Sh::OF;                       // fluxes [S+1][...]
-  // split: FP32 x coefficients [TX+2][kCoefRec], after the gate's share
-  RT* scx = reinterpret_cast<RT*>(smem_raw + stage_coef_offset<ND, NF, WO, RT, TX, TY, NT, GATE, VISC, TMA>());
-  // split: FP32 y coefficients [TY+2][kCoefRec]; FP64: [kNumCoef][TY+2]
-  RT* scy = scx + (Sh::NCOEF64 > 0 ? kNumCoef : kCoefRec) * Sh::NCX;
+  // FP64 WENO5: coefficients [kNumCoef][TX+2], then [kNumCoef][TY+2]
+  RT* scx = reinterpret_cast<RT*>(smem_raw + stage_coef_offset<ND, NF, WO, RT, TX, TY, VISC, TMA>());
+  RT* scy = scx + kNumCoef * Sh::NCX;
   // element of variable v in the primitive tile and in the x / y WENO values
-  constexpr bool kPair = Sh::PAIR;
-  constexpr int NCX_ = TX + 2, NCY_ = TY + 2;
-  auto qi = [](int v, int ly, int lx) {
-    return kPair ? (((v >> 1) * LY + ly) * LX + lx) * 2 + (v & 1) : (v * LY + ly) * LX + lx;
-  };
-  auto wxi = [](int v, int ty, int cx) {
-    return kPair ? (((v >> 1) * TYE + ty) * NCX_ + cx) * 2 + (v & 1) : (v * TYE + ty) * NCX_ + cx;
-  };
-  auto wyi = [](int v, int cy, int tx) {
-    return kPair ? (((v >> 1) * NCY_ + cy) * TX + tx) * 2 + (v & 1) : (v * NCY_ + cy) * TX + tx;
-  };
+  auto qi = [](int v, int ly, int lx) { return (v * LY + ly) * LX + lx; };
+  auto wxi = [](int v, int ty, int cx) { return (v * TYE + ty) * Sh::NCX + cx; };
+  auto wyi = [](int v, int cy, int tx) { return (v * Sh::NCY + cy) * TX + tx; };
+  (void)scy;
   (void)wyi;
   // row r of the flux of x face f (left of cell f) of row ty, and of y face f
   auto fxv = [&](int r, int ty, int f) -> RT& { return fl[(r * TYE + ty) * (TX + 1) + f]; };
@@ -320,35 +321,8 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
   N eps;
   if constexpr (kSplit) eps = P.weno_eps_f;
   else eps = num(P.weno_eps);
-  // split WENO5 on a uniform grid: every cell of a direction shares one
-  // coefficient record, read from the kernel parameters
-  const bool ux = Sh::NCOEF > 0 && U != nullptr && U->on[0];
-  const bool uy = Sh::NCOEF > 0 && ND > 1 && U != nullptr && U->on[1];
-  (void)ux;
-  (void)uy;
-
   // ---- phase 1: load + BCs + cons -> prim --------------------------------
-  if constexpr (Sh::NCOEF > 0) {
-    // the tile's coefficient records (constant tables: staged before the
-    // wait for the previous stage); global reads coalesced along the cells,
-    // records written per cell
-    for (int it = ux ? kCoefRec * Sh::NCX : tid; it < kCoefRec * Sh::NCX; it += NT) {
-      const int cx = it % Sh::NCX, k = it / Sh::NCX;
-      scx[cx * kCoefRec + k] =
-          k < kNumCoef ? d2f_bits(__ldg(P.coef[0] + k * P.cstride[0] + clamp_coef_index(x0 - 1 + cx, nx) + P.coff))
-                       : 0.f;
-    }
-    if constexpr (ND > 1) {
-      for (int it = uy ? kCoefRec * Sh::NCY : tid; it < kCoefRec * Sh::NCY; it += NT) {
-        const int cy = it % Sh::NCY, k = it / Sh::NCY;
-        scy[cy * kCoefRec + k] =
-            k < kNumCoef
-                ? d2f_bits(__ldg(P.coef[1] + k * P.cstride[1] + clamp_coef_index(y0 - 1 + cy, ny) + P.coff))
-                : 0.f;
-      }
-    }
-  }
-  if constexpr (Sh::NCOEF64 > 0 && !CHAR) {
+  if constexpr (Sh::NCOEF > 0 && !CHAR) {
     // FP64 WENO5: the tile's coefficients, [k][cell], before the wait
     for (int it = tid; it < kNumCoef * Sh::NCX; it += NT) {
       const int cx = it % Sh::NCX, k = it / Sh::NCX;
@@ -365,10 +339,9 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
   auto store_prim = [&](double (&q)[S], const int ly, const int lx) {
     if constexpr (kSplit) {
       float pr[S];
-      cons_to_prim_split<ND, NF>(q, P, pr);
+      cons_to_prim_split<ND, NF>(q, P, one, pr);
 #pragma unroll
       for (int v = 0; v < S; ++v) sq[qi(v, ly, lx)] = pr[v];
-      if constexpr (Sh::SP > S) sq[qi(S, ly, lx)] = 0.f;  // the padding lane
     } else {
       cons_to_prim<ND, NF>(q, P, u0);
 #pragma unroll
@@ -386,7 +359,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
   // TMA staging: a tile whose halo lies inside the domain (no boundary
   // condition, no processor halo) arrives in one bulk tensor copy of all
   // variables into the WENO and flux arrays, which are free until phase 2
-  // (the coefficient records sit past the staging area).
+  // (the coefficients sit past the staging area).
   bool use_tma = false;
   unsigned char* stg = nullptr;
   uint32_t bar = 0;
@@ -397,9 +370,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
     if (use_tma) {
       stg = tma_staging<ND, NF, WO, RT, TX, TY>(smem_raw);
       bar = smem_addr(stg + kStageBytes);
-      // one tile per block: a fresh barrier; a block walking many tiles
-      // (tma_parity given) initialised it once and alternates its phase
-      if (tid == 0 && tma_parity == nullptr) mbar_init(bar, 1);
+      if (tid == 0) mbar_init(bar, 1);
     }
   }
   griddep_wait();  // the state below is the previous stage's output
@@ -415,19 +386,12 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
     }
   }
   if (use_tma) {
-    const uint32_t par = tma_parity ? *tma_parity : 0u;
     volatile int* landed = reinterpret_cast<volatile int*>(stg + kStageBytes + 8);
     if (tid == 0) {
-      // a walking block: its reads of this memory for the previous tile come
-      // first, and its maps live in global memory
-      if (tma_parity) {
-        fence_proxy_async_smem();
-        tensormap_acquire(&T->map);
-      }
       mbar_arrive_expect_tx(bar, kStageBytes);
       tma_load_3d(smem_addr(stg), &T->map, x0 - Box::kLead, y0 - H, 0, bar);
-      const bool ok = mbar_wait_bounded(bar, par, 1000000000ull);  // 1 s
-      if (!ok) (void)mbar_wait_bounded(bar, par, 1000000000ull);    // the copy may still be in flight
+      const bool ok = mbar_wait_bounded(bar, 0, 1000000000ull);  // 1 s
+      if (!ok) (void)mbar_wait_bounded(bar, 0, 1000000000ull);    // the copy may still be in flight
       *landed = ok ? 1 : 0;
     }
     __syncthreads();
@@ -435,8 +399,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
       if (tid == 0 && P.status) atomicOr(P.status, MFC_FLAG_TIMEOUT);
       return;
     }
-    (void)mbar_try_wait(bar, par);  // completed: each thread acquires the copy's writes
-    if (tma_parity) *tma_parity ^= 1u;
+    (void)mbar_try_wait(bar, 0);  // completed: each thread acquires the copy's writes
     const double* sd = reinterpret_cast<const double*>(stg);
     for (int c = tid; c < LX * LY; c += NT) {
       const int lx = c % LX, ly = c / LX;
@@ -450,37 +413,9 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
     for (int c = tid; c < LX * LY; c += NT) {
       const int lx = c % LX, ly = c / LX;
       if (unused_corner(lx, ly)) continue;
-      bool fx = false, fy = false;
-      const int rx = x0 - H + lx, ry = (ND > 1) ? y0 - H + ly : 0;
-      // processor boundaries: ghost cells come from the neighbour's halo buffer
-      const int px = rx < 0 ? (P.bc_beg[0] >= 0 ? 0 : -1) : (rx >= nx && P.bc_end[0] >= 0 ? 1 : -1);
-      const int py = (ND > 1) ? (ry < 0 ? (P.bc_beg[1] >= 0 ? 0 : -1) : (ry >= ny && P.bc_end[1] >= 0 ? 1 : -1)) : -1;
-      const double* src;
-      int64_t vs = P.sv;
-      // cells of partial edge tiles beyond the first H ghosts are never stored:
-      // their depth is clamped.  y strips are nx + 2 wide (the x ghost cells
-      // -1 and nx of the neighbour's rows come first and last).
-      if (px >= 0 && py >= 0) {
-        // between two processor boundaries (the viscous corner cells): the
-        // diagonal neighbour's cell, forwarded by the y neighbour
-        const int d = min(py == 0 ? -1 - ry : ry - ny, H - 1);
-        src = P.halo[2 + py] + (int64_t)d * (nx + 2) + (px == 0 ? 0 : nx + 1);
-        vs = (int64_t)H * (nx + 2);
-      } else if (px >= 0) {
-        const int d = min(px == 0 ? -1 - rx : rx - nx, H - 1);
-        const int yy = (ND > 1) ? map_cell(ry, ny, P.bc_beg[1], P.bc_end[1], &fy) : 0;
-        src = P.halo[px] + (int64_t)yy * H + d;
-        vs = (int64_t)ny * H;
-      } else if (py >= 0) {
-        const int d = min(py == 0 ? -1 - ry : ry - ny, H - 1);
-        const int xx = map_cell(rx, nx, P.bc_beg[0], P.bc_end[0], &fx);
-        src = P.halo[2 + py] + (int64_t)d * (nx + 2) + xx + 1;
-        vs = (int64_t)H * (nx + 2);
-      } else {
-        const int gx = map_cell(rx, nx, P.bc_beg[0], P.bc_end[0], &fx);
-        const int gy = (ND > 1) ? map_cell(ry, ny, P.bc_beg[1], P.bc_end[1], &fy) : 0;
-        src = qin + gy * P.sy + gx;
-      }
+      bool fx, fy;
+      int64_t vs;
+      const double* src = tile_cell<ND, H>(P, qin, x0 - H + lx, ND > 1 ? y0 - H + ly : 0, vs, fx, fy);
       double q[S];
 #pragma unroll
       for (int v = 0; v < S; ++v) q[v] = __ldg(src + v * vs);
@@ -490,101 +425,6 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
     }
   }
   __syncthreads();
-
-  // ---- learned gate: one flag per (cell, direction), tensor-core MLP -------
-  // The first stage of a time step (and an RHS evaluation) runs the network
-  // on every reconstructed position of the tile; with P.gate_flags it also
-  // stores the decisions, and the step's later stages read them back instead
-  // of running the network again: the gate judges each cell once per time
-  // step, on the state at t^n.  Every stored position (including the ghost
-  // positions x = -1, nx and y = -1, ny next to the domain) is written by
-  // exactly one tile.
-  const uint8_t* gflag = nullptr;
-  if constexpr (GATE) {
-    using G = GateShape<ND, TX, TY, NT>;
-    constexpr int NG = G::NGX + G::NGY;
-    uint8_t* flags = smem_raw + Sh::kMainBytes;
-    // position p of the tile: its slot in the stored planes (false: beyond
-    // the planes, a cell of a partial edge tile whose results are not kept)
-    // and whether this tile is the one that stores it
-    auto flag_slot = [&](const int p, int64_t& slot, bool& owner) {
-      if (p < G::NGX) {
-        const int cx = p % (TX + 2), ty = p / (TX + 2);
-        const int gx = x0 - 1 + cx, gy = y0 + ty;
-        slot = (int64_t)gy * (nx + 2) + (gx + 1);
-        owner = (cx >= 1 && cx <= TX) || gx == -1 || gx == nx;
-        return gx >= -1 && gx <= nx && gy < ny;
-      }
-      const int p2 = p - G::NGX, tx = p2 % TX, cy = p2 / TX;
-      const int gx = x0 + tx, gy = y0 - 1 + cy;
-      slot = (int64_t)ny * (nx + 2) + (int64_t)(gy + 1) * nx + gx;
-      owner = (cy >= 1 && cy <= TY) || gy == -1 || gy == ny;
-      return gx < nx && gy >= -1 && gy <= ny;
-    };
-    if (P.gate_flags != nullptr && kind != kRkEuler && kind != kRhsOnly) {
-      // a later stage of the step: the first stage's decisions
-      for (int p = tid; p < NG; p += NT) {
-        int64_t slot;
-        bool owner;
-        flags[p] = flag_slot(p, slot, owner) ? __ldg(P.gate_flags + slot) : uint8_t(1);
-      }
-    } else {
-      static_assert(G::kScratchBytes <= 2 * sizeof(RT) * size_t(Sh::align16(Sh::NW)),
-                    "the gate's scratch must fit the WENO value arrays");
-      unsigned char* scratch = reinterpret_cast<unsigned char*>(wl);
-      __half* gin = reinterpret_cast<__half*>(scratch);
-      uint32_t* frag = reinterpret_cast<uint32_t*>(scratch + G::kFragOff);
-      const int warp = tid >> 5, lane = tid & 31;
-      const uint32_t* gsrc =
-          reinterpret_cast<const uint32_t*>(static_cast<const unsigned char*>(P.gate_w) + kGateFragOffset);
-      for (int i = tid; i < kGateFragWords * 8; i += NT)
-        reinterpret_cast<uint4*>(frag)[i] = __ldg(reinterpret_cast<const uint4*>(gsrc) + i);
-      __syncthreads();
-      const GateFragsSmem F{frag + 4 * lane};
-      __half* my = gin + warp * 256;
-      constexpr int NCH = (NG + 15) / 16;
-      for (int ch = warp; ch < NCH; ch += NT / 32) {
-        const int cell = ch * 16 + (lane & 15);
-        const int var = lane < 16 ? Q::ADV : Q::E;  // alpha_1 | pressure
-        float s[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-        if (cell < G::NGX) {
-          const int cx = cell % (TX + 2), ty = cell / (TX + 2);
-#pragma unroll
-          for (int k = 0; k < 5; ++k) s[k] = sq[qi(var, (ND > 1) ? ty + H : 0, cx + H - 1 + k - 2)];
-        } else if (cell < NG) {
-          const int c2 = cell - G::NGX, tx = c2 % TX, cy = c2 / TX;
-#pragma unroll
-          for (int k = 0; k < 5; ++k) s[k] = sq[qi(var, cy + H - 1 + k - 2, tx + H)];
-        }
-        float xf[5];
-        gate_norm5_var(s, xf, lane < 16 ? 0 : 1);
-        // columns 0..7 (alpha_1) or 8..15 (pressure) of the cell's row: five
-        // features and three zeros, one 16-byte store
-        const uint4 half8 = make_uint4(pack_h2(xf[0], xf[1]), pack_h2(xf[2], xf[3]), pack_h2(xf[4], 0.f), 0u);
-        reinterpret_cast<uint4*>(my + (lane & 15) * 16)[lane >> 4] = half8;
-        __syncwarp();
-        float lo, hi;
-        gate_mlp16(my, F, lo, hi);
-        if ((lane & 3) == 0) {
-          const int c_lo = ch * 16 + (lane >> 2), c_hi = c_lo + 8;
-          if (c_lo < NG) flags[c_lo] = lo > 0.f;
-          if (c_hi < NG) flags[c_hi] = hi > 0.f;
-        }
-        __syncwarp();
-      }
-      __syncthreads();
-      if (P.gate_flags != nullptr && kind == kRkEuler) {
-        // the first stage stores the decisions of the positions it owns
-        for (int p = tid; p < NG; p += NT) {
-          int64_t slot;
-          bool owner;
-          if (flag_slot(p, slot, owner) && owner) P.gate_flags[slot] = flags[p];
-        }
-      }
-    }
-    gflag = flags;
-    __syncthreads();
-  }
 
   // ---- phase 2: x WENO over cells x0-1 .. x0+TX of the interior rows -------
   {
@@ -603,55 +443,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
       wl[wxi(v, ty, cx)] = low(vl);
       wr[wxi(v, ty, cx)] = low(vr);
     };
-    if constexpr (kPair) {
-      constexpr int NPR = Sh::SP / 2;  // variable pairs
-      const f32x2 eps2 = f2_pack(eps, eps);
-      // variable pair pr of the cell at (cx, ty); C(k): coefficient k as a (c, c) pair
-      auto x_pair = [&](const auto& C, const int cx, const int ty, const int pr, const bool nonlin) {
-        const f32x2* row = reinterpret_cast<const f32x2*>(sq) + (pr * LY + ((ND > 1) ? ty + H : 0)) * LX + cx + H - 1;
-        f32x2 st[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) st[k] = row[k - 2];
-        f32x2 vl, vr;
-        if constexpr (GATE) {
-          if (nonlin) weno5_pair_fast(C, st, eps2, vl, vr);
-          else weno5_pair_linear(C, st, vl, vr);
-        } else {
-          weno5_pair_fast(C, st, eps2, vl, vr);
-        }
-        reinterpret_cast<f32x2*>(wl)[(pr * TYE + ty) * NCX + cx] = vl;
-        reinterpret_cast<f32x2*>(wr)[(pr * TYE + ty) * NCX + cx] = vr;
-      };
-      // UNI: the shared record of a uniform grid, else the cell's staged
-      // record (reloaded per pair: keeping it live across them costs
-      // registers); chosen once per block
-      auto x_positions = [&](auto uni) {
-        constexpr bool UNI = decltype(uni)::value;
-        deal_positions<TYE * NCX, NPR, NT>(tid, [&](const int p, const int v, const bool all) {
-          const int cx = p % NCX, ty = p / NCX;
-          bool nonlin = true;
-          if constexpr (GATE) nonlin = gflag[p] != 0;
-          auto one = [&](const int w) {
-            if constexpr (UNI) {
-              const f32x2* rec = U->rec[0];
-              x_pair([&](int k) { return rec[k]; }, cx, ty, w, nonlin);
-            } else {
-              RT c[kCoefRec];
-              load_coef_record(scx + cx * kCoefRec, c);
-              x_pair([&](int k) { return f2_pack(c[k], c[k]); }, cx, ty, w, nonlin);
-            }
-          };
-          if (all) {
-#pragma unroll 1
-            for (int w = 0; w < NPR; ++w) one(w);
-          } else {
-            one(v);
-          }
-        });
-      };
-      if (ux) x_positions(FlagC<true>{});
-      else x_positions(FlagC<false>{});
-    } else if constexpr (CHAR) {
+    if constexpr (CHAR) {
       // characteristic fields: one thread per position, all variables
       const double* cf = P.coef[0];
       const int cs = P.cstride[0];
@@ -676,7 +468,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
       const double* cf = P.coef[0];
       const int cs = P.cstride[0];
       auto coef = [&](const int cx, RT (&c)[kCoefRec]) {
-        if constexpr (Sh::NCOEF64 > 0) {
+        if constexpr (Sh::NCOEF > 0) {
 #pragma unroll
           for (int k = 0; k < kNumCoef; ++k) c[k] = scx[k * Sh::NCX + cx];
         } else {
@@ -708,7 +500,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
         else wr[wxi(v, ty, cx)] = low(weno_cell_side<WO, 1, N>(NumCoef<N>{c, u0}, st, eps));
       }
     } else {
-      // split WENO1/3 (and FP64 WENO1): coefficients per reconstruction from global memory
+      // split WENO1/3 and FP64 WENO1: coefficients per reconstruction from global memory
       const double* cf = P.coef[0];
       const int cs = P.cstride[0];
       for (int it = tid; it < S * TYE * NCX; it += NT) {
@@ -836,51 +628,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
       wl[wyi(v, cy, tx)] = low(vl);
       wr[wyi(v, cy, tx)] = low(vr);
     };
-    if constexpr (kPair) {
-      constexpr int NPR = Sh::SP / 2;
-      const f32x2 eps2 = f2_pack(eps, eps);
-      auto y_pair = [&](const auto& C, const int tx, const int cy, const int pr, const bool nonlin) {
-        const f32x2* col = reinterpret_cast<const f32x2*>(sq) + (pr * LY + cy + H - 1) * LX + tx + H;
-        f32x2 st[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) st[k] = col[(k - 2) * LX];
-        f32x2 vl, vr;
-        if constexpr (GATE) {
-          if (nonlin) weno5_pair_fast(C, st, eps2, vl, vr);
-          else weno5_pair_linear(C, st, vl, vr);
-        } else {
-          weno5_pair_fast(C, st, eps2, vl, vr);
-        }
-        reinterpret_cast<f32x2*>(wl)[(pr * NCY + cy) * TX + tx] = vl;
-        reinterpret_cast<f32x2*>(wr)[(pr * NCY + cy) * TX + tx] = vr;
-      };
-      auto y_positions = [&](auto uni) {
-        constexpr bool UNI = decltype(uni)::value;
-        deal_positions<NCY * TX, NPR, NT>(tid, [&](const int p, const int v, const bool all) {
-          const int tx = p % TX, cy = p / TX;
-          bool nonlin = true;
-          if constexpr (GATE) nonlin = gflag[GateShape<ND, TX, TY, NT>::NGX + p] != 0;
-          auto one = [&](const int w) {
-            if constexpr (UNI) {
-              const f32x2* rec = U->rec[1];
-              y_pair([&](int k) { return rec[k]; }, tx, cy, w, nonlin);
-            } else {
-              RT c[kCoefRec];
-              load_coef_record(scy + cy * kCoefRec, c);
-              y_pair([&](int k) { return f2_pack(c[k], c[k]); }, tx, cy, w, nonlin);
-            }
-          };
-          if (all) {
-#pragma unroll 1
-            for (int w = 0; w < NPR; ++w) one(w);
-          } else {
-            one(v);
-          }
-        });
-      };
-      if (uy) y_positions(FlagC<true>{});
-      else y_positions(FlagC<false>{});
-    } else if constexpr (CHAR) {
+    if constexpr (CHAR) {
       const double* cf = P.coef[1];
       const int cs = P.cstride[1];
       for (int it = tid; it < NCY * TX; it += NT) {
@@ -900,7 +648,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
       const double* cf = P.coef[1];
       const int cs = P.cstride[1];
       auto coef = [&](const int cy, RT (&c)[kCoefRec]) {
-        if constexpr (Sh::NCOEF64 > 0) {
+        if constexpr (Sh::NCOEF > 0) {
 #pragma unroll
           for (int k = 0; k < kNumCoef; ++k) c[k] = scy[k * Sh::NCY + cy];
         } else {
@@ -1062,7 +810,7 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
           const double b = __ldg(qbase + o + v * P.sv);
           double in = b;
           if constexpr (KIND != kRkEuler) in = __ldg(qin + o + v * P.sv);
-          if constexpr (kSplit) out = rk_combine_split(KIND, b, in, dtf, rhs[k][v]);
+          if constexpr (kSplit) out = rk_combine_split(KIND, b, in, dtf, rhs[k][v], one);
           else out = rk_combine(KIND, num(b), num(in), num(dt), num(rhs[k][v]));
         }
         bad |= not_finite(out);
@@ -1108,53 +856,25 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
 // FMA tags the instantiations of the translation unit compiled with
 // multiply-add contraction (-fmad=true), so that their host-side symbols
 // differ from the bit-faithful ones; the kernel body does not use it.
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE = false, bool VISC = false,
-          bool FMA = false, bool CHAR = false>
-__global__ void __launch_bounds__(NT) stage_kernel(const DevParams P, const __grid_constant__ UniformCoef U,
-                                                   const double* __restrict__ qin, const double* __restrict__ qbase,
-                                                   double* __restrict__ qout, const double dt, const int kind) {
+template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool FMA = false, bool CHAR = false>
+__global__ void __launch_bounds__(NT) stage_kernel(const DevParams P, const double* __restrict__ qin,
+                                                   const double* __restrict__ qbase, double* __restrict__ qout,
+                                                   const double dt, const int kind) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  stage_tile<ND, NF, WO, RT, TX, TY, NT, GATE, VISC, UniformCoef, false, CHAR>(P, qin, qbase, qout, dt, kind,
-                                                                               blockIdx.x * TX,
-                                                     (ND > 1) ? blockIdx.y * TY : 0, smem_raw, &U);
-}
-
-// The same kernel with its registers capped so that MINB blocks fit on an SM.
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, int MINB, bool FMA = false,
-          bool VISC = false>
-__global__ void __launch_bounds__(NT, MINB) stage_kernel_mb(const DevParams P, const __grid_constant__ UniformCoef U,
-                                                            const double* __restrict__ qin,
-                                                            const double* __restrict__ qbase,
-                                                            double* __restrict__ qout, const double dt,
-                                                            const int kind) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  stage_tile<ND, NF, WO, RT, TX, TY, NT, GATE, VISC>(P, qin, qbase, qout, dt, kind, blockIdx.x * TX,
-                                                     (ND > 1) ? blockIdx.y * TY : 0, smem_raw, &U);
+  stage_tile<ND, NF, WO, RT, TX, TY, NT, false, false, CHAR>(P, qin, qbase, qout, dt, kind, blockIdx.x * TX,
+                                                             (ND > 1) ? blockIdx.y * TY : 0, smem_raw);
 }
 
 // The kernel with TMA staging of interior tiles (2-D, inviscid); T maps the
-// stage input qin.  MINB > 1 caps the registers as stage_kernel_mb does.
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, bool FMA = false>
-__global__ void __launch_bounds__(NT) stage_kernel_tma(const DevParams P, const __grid_constant__ UniformCoef U,
-                                                       const __grid_constant__ TileMap T,
+// stage input qin.
+template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool FMA = false>
+__global__ void __launch_bounds__(NT) stage_kernel_tma(const DevParams P, const __grid_constant__ TileMap T,
                                                        const double* __restrict__ qin,
                                                        const double* __restrict__ qbase, double* __restrict__ qout,
                                                        const double dt, const int kind) {
   extern __shared__ __align__(128) unsigned char smem_tma[];
-  stage_tile<ND, NF, WO, RT, TX, TY, NT, GATE, false, UniformCoef, true>(
-      P, qin, qbase, qout, dt, kind, blockIdx.x * TX, (ND > 1) ? blockIdx.y * TY : 0, smem_tma, &U, &T);
-}
-
-template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool GATE, int MINB, bool FMA = false>
-__global__ void __launch_bounds__(NT, MINB) stage_kernel_tma_mb(const DevParams P, const __grid_constant__ UniformCoef U,
-                                                                const __grid_constant__ TileMap T,
-                                                                const double* __restrict__ qin,
-                                                                const double* __restrict__ qbase,
-                                                                double* __restrict__ qout, const double dt,
-                                                                const int kind) {
-  extern __shared__ __align__(128) unsigned char smem_tma[];
-  stage_tile<ND, NF, WO, RT, TX, TY, NT, GATE, false, UniformCoef, true>(
-      P, qin, qbase, qout, dt, kind, blockIdx.x * TX, (ND > 1) ? blockIdx.y * TY : 0, smem_tma, &U, &T);
+  stage_tile<ND, NF, WO, RT, TX, TY, NT, false, true>(P, qin, qbase, qout, dt, kind, blockIdx.x * TX,
+                                                      (ND > 1) ? blockIdx.y * TY : 0, smem_tma, &T);
 }
 
 }  // namespace mfc

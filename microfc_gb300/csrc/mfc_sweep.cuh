@@ -91,8 +91,10 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
   using N = std::conditional_t<kSplit, float, Num64>;
   N u0;
   if constexpr (kSplit) u0 = 0.f;
-  else u0 = num64_unit(P.weno_eps);
+  else u0 = num64_unit(P.inv_d[0]);
   auto num = [&](RT x) { return lift(x, u0); };
+  const double one = kSplit ? fma64_unit(P.inv_d[0]).one : 1.0;  // split: the FP64 sums' register operand
+  (void)one;
   constexpr int OA = DIR, OB = DIR == 0 ? 1 : 0, OC = DIR == 2 ? 1 : 2;  // axis index of a, b, c
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -160,7 +162,7 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
   auto store_prim = [&](double (&q)[S], const int p, const int la, const int64_t own) {
     RT pr[S];
     if constexpr (kSplit) {
-      cons_to_prim_split<3, NF>(q, P, pr);
+      cons_to_prim_split<3, NF>(q, P, one, pr);
     } else {
       cons_to_prim<3, NF>(q, P, u0);
 #pragma unroll
@@ -462,7 +464,7 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
           const double b = __ldg(qbase + o + v * P.sv);
           double in = b;
           if constexpr (KIND != kRkEuler) in = __ldg(qin + o + v * P.sv);
-          if constexpr (kSplit) out = rk_combine_split(KIND, b, in, dtf, r[v]);
+          if constexpr (kSplit) out = rk_combine_split(KIND, b, in, dtf, r[v], one);
           else out = rk_combine(KIND, num(b), num(in), num(dt), r[v]);
         }
         bad |= not_finite(out);

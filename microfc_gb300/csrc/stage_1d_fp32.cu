@@ -4,10 +4,13 @@
 namespace mfc {
 
 void register_stage_1d_fp32(std::vector<StageEntry>& r) {
-#define MFC_1D(NF, WO) r.push_back(stage_entry<1, NF, WO, float, 128, 1, 128>());
-  MFC_1D(1, 1) MFC_1D(1, 3) MFC_1D(1, 5)
-  MFC_1D(2, 1) MFC_1D(2, 3) MFC_1D(2, 5)
-#undef MFC_1D
+  r.push_back(stage_entry<1, 1, 1, float, 128, 1, 128>());
+  r.push_back(stage_entry<1, 1, 3, float, 128, 1, 128>());
+  r.push_back(stage_entry<1, 2, 1, float, 128, 1, 128>());
+  r.push_back(stage_entry<1, 2, 3, float, 128, 1, 128>());
+  // 62 cells: 64 positions, a run of two of one of three pairs for each of 96 threads
+  r.push_back(pair_entry<1, 1, 62, 1, 96, 10, 2, 1>());
+  r.push_back(pair_entry<1, 2, 62, 1, 96, 10, 2, 1>());
 }
 
 }  // namespace mfc

@@ -4,35 +4,33 @@
 
 namespace mfc {
 
+// T x T tiles, interior ones loaded by TMA: 16x16 with 256 threads, four
+// blocks per SM; 8x8 with 160, six blocks.
+template <int NF, int T, bool GATE>
+struct Pair2D {
+  static StageEntry entry() {
+    if constexpr (T == 16) return pair_entry<2, NF, 16, 16, 256, 4, 9, 9, GATE, false, true>();
+    else return pair_entry<2, NF, 8, 8, 160, 6, 2, 2, GATE, false, true>();
+  }
+};
+
 void register_stage_2d_fp32(std::vector<StageEntry>& r) {
-  // the first entry is the default: the autotuner's usual choice on GB300,
-  // interior tiles staged by one TMA bulk tensor copy
-  r.push_back(stage_entry<2, 2, 5, float, 16, 16, 256, false, 5, false, true>());
-  r.push_back(stage_entry<2, 2, 5, float, 16, 16, 256, false, 5>());
-  r.push_back(stage_entry<2, 2, 5, float, 32, 16, 256>());
-  r.push_back(stage_entry<2, 2, 5, float, 32, 32, 512>());
-  r.push_back(stage_entry<2, 2, 5, float, 32, 8, 256>());
-  r.push_back(stage_entry<2, 2, 5, float, 16, 16, 256>());
-  r.push_back(stage_entry<2, 2, 5, float, 64, 8, 512>());
-  r.push_back(stage_entry<2, 2, 5, float, 16, 16, 256, false, 6>());
-  r.push_back(stage_entry<2, 2, 5, float, 16, 8, 128>());
-  r.push_back(stage_entry<2, 2, 5, float, 16, 16, 128>());
-  r.push_back(stage_entry<2, 2, 5, float, 32, 16, 256, false, 1, false, true>());
-  r.push_back(stage_entry<2, 1, 5, float, 32, 16, 256>());
+  // the default; the autotuner may take either size alone
+  r.push_back(sized_entry(Pair2D<2, 8, false>{}, Pair2D<2, 16, false>{}));
+  r.push_back(Pair2D<2, 16, false>::entry());
+  r.push_back(Pair2D<2, 8, false>::entry());
+  r.push_back(pair_entry<2, 2, 16, 16, 256, 4, 9, 9>());
+  r.push_back(sized_entry(Pair2D<1, 8, false>{}, Pair2D<1, 16, false>{}));
   r.push_back(stage_entry<2, 2, 3, float, 32, 16, 256>());
   r.push_back(stage_entry<2, 2, 1, float, 32, 16, 256>());
   r.push_back(stage_entry<2, 1, 3, float, 32, 16, 256>());
   r.push_back(stage_entry<2, 1, 1, float, 32, 16, 256>());
   // split precision with the learned WENO gate
-  r.push_back(stage_entry<2, 2, 5, float, 16, 16, 256, true, 5, false, true>());
-  r.push_back(stage_entry<2, 2, 5, float, 16, 16, 256, true, 5>());
-  r.push_back(stage_entry<2, 2, 5, float, 32, 16, 256, true>());
-  r.push_back(stage_entry<2, 2, 5, float, 16, 16, 256, true>());
-  r.push_back(stage_entry<2, 2, 5, float, 32, 32, 512, true>());
-  r.push_back(stage_entry<2, 2, 5, float, 32, 8, 256, true>());
-  r.push_back(stage_entry<2, 2, 5, float, 16, 16, 256, true, 4>());
-  r.push_back(stage_entry<2, 2, 5, float, 16, 8, 128, true, 8>());
-  r.push_back(stage_entry<2, 1, 5, float, 32, 16, 256, true>());
+  r.push_back(sized_entry(Pair2D<2, 8, true>{}, Pair2D<2, 16, true>{}));
+  r.push_back(Pair2D<2, 16, true>::entry());
+  r.push_back(Pair2D<2, 8, true>::entry());
+  r.push_back(pair_entry<2, 2, 16, 16, 256, 4, 9, 9, true>());
+  r.push_back(Pair2D<1, 16, true>::entry());
 }
 
 }  // namespace mfc

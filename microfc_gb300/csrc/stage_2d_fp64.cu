@@ -10,7 +10,7 @@ void register_stage_2d_fp64(std::vector<StageEntry>& r) {
   // 32x16, interior tiles staged by one TMA bulk tensor copy: 1 % faster than
   // the sized tiles on the largest grids (15585 against 15761 us a step at
   // 2048x1024), 1 % slower at 1024x512
-  r.push_back(stage_entry<2, 2, 5, double, 32, 16, 640, false, 1, false, true>());
+  r.push_back(stage_entry<2, 2, 5, double, 32, 16, 640, true>());
   r.push_back(flex_entry<2, 1, 5, 640>());
   r.push_back(flex_entry<2, 2, 3, 512>());
   r.push_back(flex_entry<2, 2, 1, 512>());

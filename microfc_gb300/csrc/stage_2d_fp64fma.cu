@@ -12,13 +12,13 @@ namespace mfc {
 
 void register_stage_2d_fp64fma(std::vector<StageEntry>& r) {
 #define MFC_2D_FMA(NF)                                                           \
-  r.push_back(stage_entry<2, NF, 5, double, 32, 16, 544, false, 1, false, false, true>()); \
-  r.push_back(stage_entry<2, NF, 5, double, 32, 16, 512, false, 1, false, false, true>()); \
-  r.push_back(stage_entry<2, NF, 5, double, 16, 16, 256, false, 1, false, false, true>());
+  r.push_back(stage_entry<2, NF, 5, double, 32, 16, 544, false, true>()); \
+  r.push_back(stage_entry<2, NF, 5, double, 32, 16, 512, false, true>()); \
+  r.push_back(stage_entry<2, NF, 5, double, 16, 16, 256, false, true>());
   MFC_2D_FMA(2)
   MFC_2D_FMA(1)
 #undef MFC_2D_FMA
-  r.push_back(stage_entry<2, 2, 5, double, 32, 16, 640, false, 1, false, false, true>());
+  r.push_back(stage_entry<2, 2, 5, double, 32, 16, 640, false, true>());
 }
 
 }  // namespace mfc

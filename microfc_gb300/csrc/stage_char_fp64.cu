@@ -9,7 +9,7 @@ namespace mfc {
 
 void register_stage_char_fp64(std::vector<StageEntry>& r) {
 #define MFC_CHAR(ND, NF, WO, TX, TY, NT) \
-  r.push_back(stage_entry<ND, NF, WO, double, TX, TY, NT, false, 1, false, false, false, true>());
+  r.push_back(stage_entry<ND, NF, WO, double, TX, TY, NT, false, false, true>());
   MFC_CHAR(2, 2, 5, 32, 16, 512)
   MFC_CHAR(2, 2, 5, 16, 16, 256)
   MFC_CHAR(2, 1, 5, 32, 16, 512)
