@@ -261,7 +261,7 @@ int launch_stage(mfc_gpu_ctx* c, const double* qin, const double* qbase, double*
     const bool fp32 = c->prm.precision != MFC_PREC_FP64;  // split or gated (contracted FP64 is refused)
     const cudaError_t g = mfc::visc_gradients_launch(c->nd, c->prm.num_fluids, fp32, c->dev, c->vg, qin, c->stream);
     if (g != cudaSuccess) return fail(MFC_ERR_CUDA, std::string("viscous gradients: ") + cudaGetErrorString(g));
-    c->launches += c->nd == 1 ? 3 : 4;
+    c->launches += mfc::visc_gradients_launches(c->nd, fp32);
   }
   cudaError_t e;
   if (c->prim[0] != nullptr && c->stage->launch_prims != nullptr) {
@@ -741,6 +741,7 @@ int mfc_gpu_set_viscosity(mfc_gpu_ctx* c, const double* re_shear, const double* 
   for (int f = 0; f < nf; ++f) {
     V.res[0][f] = re_shear ? re_shear[f] : 0.0;
     V.res[1][f] = re_bulk ? re_bulk[f] : 0.0;
+    for (int r = 0; r < 2; ++r) V.res_f[r][f] = (float)V.res[r][f];
   }
   for (int r = 0; r < 2; ++r)
     for (int f = 0; f < nf; ++f)
@@ -862,6 +863,20 @@ int mfc_gpu_set_viscous_gradients(mfc_gpu_ctx* c, int weno_re_flux) {
   for (int d = 0; d < nd; ++d) {
     MFC_CUDA(cudaMemcpy(c->vg.w[d], w[d].data(), sizeof(double) * w[d].size(), cudaMemcpyHostToDevice));
     if (fp32) MFC_CUDA(cudaMemcpy(c->vg.cf[d], cf[d].data(), sizeof(float) * cf[d].size(), cudaMemcpyHostToDevice));
+  }
+  if (fp32 && nd == 2) {
+    c->vg.uniform.on = 1;
+    for (int d = 0; d < 2; ++d) {
+      const size_t stride = w[d].size();
+      for (int kk = 0; kk <= mfc::kNumCoef; ++kk) {
+        const float* row = cf[d].data() + (size_t)kk * stride;
+        uint32_t b0;
+        std::memcpy(&b0, row, 4);
+        for (size_t j = 1; j < stride; ++j)
+          if (std::memcmp(row + j, row, 4) != 0) c->vg.uniform.on = 0;
+        c->vg.uniform.rec[d][kk] = (unsigned long long)b0 << 32 | b0;
+      }
+    }
   }
   c->visc_host.fg[0] = c->vg.fg[0];
   c->visc_host.fg[1] = c->vg.fg[1];

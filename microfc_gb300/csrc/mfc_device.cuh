@@ -96,6 +96,7 @@ using UniformCoef = UniformCoefT<3>;
 // s_populate_grid_variables_buffers).
 struct ViscParams {
   double res[2][kMaxFluids];
+  float res_f[2][kMaxFluids];  // rounded to FP32 (a conversion per face would occupy the FP64 unit)
   int re_size[2];
   int re_idx[2][kMaxFluids];
   const double* dcc[3];
@@ -103,6 +104,8 @@ struct ViscParams {
   // visc_gradients_launch (mfc_visc_grad.cu), read instead of the finite
   // differences.  fg[0]: x faces [c*ND+d][ny][nx+1] (face i+1/2 at i+1),
   // fg[1]: y faces [c*ND+d][ny+1][nx] (face j+1/2 at j+1); d u_c / d x_d.
+  // 2-D split and gated kernels read FP32 pairs of the two components instead:
+  // (d u/d x_d, d v/d x_d), [d][ny][nx+1] and [d][ny+1][nx].
   // NULL: the finite differences of weno_Re_flux = F.
   const double* fg[2];
 };
@@ -750,8 +753,9 @@ __device__ __forceinline__ void hllc_face(const RT (&qL)[Eqs<ND, NF>::S], const 
     const RT sM = num_min(zero, sL), sP = num_max(zero, sR);
     const RT xiL = div_rn(sL - uL, divisor(sL - sS));
     const RT xiR = div_rn(sR - uR, divisor(sR - sS));
-    const RT xiM = lift(0.5 + copysign(0.5, double(low(sS))), u0);
-    const RT xiP = lift(0.5 - copysign(0.5, double(low(sS))), u0);
+    // 0.5 +- sign(0.5, s_S) of the reference: exactly one or zero
+    const bool right = signbit(low(sS));
+    const RT xiM = right ? zero : none, xiP = right ? none : zero;
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
       const RT flg = d == DIR ? none : zero;
@@ -861,6 +865,13 @@ __device__ __forceinline__ void hllc_face_fast(const float (&qL)[Eqs<ND, NF>::S]
   ustar = w;
 }
 
+// Reynolds number r of fluid f in a number type.
+__device__ __forceinline__ float reynolds(const ViscParams& V, int r, int f, float) { return V.res_f[r][f]; }
+template <class N>
+__device__ __forceinline__ N reynolds(const ViscParams& V, int r, int f, const N& u0) {
+  return lift(V.res[r][f], u0);
+}
+
 // Viscous source flux of one face, s_compute_viscous_source_flux
 // (m_riemann_solvers.fpp:683-902), from the face's left/right states (for the
 // mixture Reynolds numbers, :169-230), vel_src vs and the face velocity
@@ -880,7 +891,7 @@ __device__ __forceinline__ void viscous_face_flux(const RT (&qL)[Eqs<ND, NF>::S]
     if (V.re_size[r] > 0) reL = reR = zero;
     for (int q = 0; q < V.re_size[r]; ++q) {
       const int f = V.re_idx[r][q];
-      const auto D = divisor(lift(V.res[r][f], u0));
+      const auto D = divisor(reynolds(V, r, f, u0));
       reL = div_rn(qL[Q::ADV + f], D) + reL;
       reR = div_rn(qR[Q::ADV + f], D) + reR;
     }

@@ -465,6 +465,7 @@ int mfc_gpu_ensemble_set_viscosity(mfc_gpu_ensemble* e, const double* re_shear, 
     for (int f = 0; f < nf; ++f) {
       v.res[0][f] = re_shear ? re_shear[(size_t)i * nf + f] : 0.0;
       v.res[1][f] = re_bulk ? re_bulk[(size_t)i * nf + f] : 0.0;
+      for (int r = 0; r < 2; ++r) v.res_f[r][f] = (float)v.res[r][f];
     }
     for (int r = 0; r < 2; ++r)
       for (int f = 0; f < nf; ++f)

@@ -465,15 +465,25 @@ cudaError_t ctx_scratch(mfc_gpu_ctx* c, size_t bytes, void** out);
 // direction for cells -kCoefPad .. n-1+kCoefPad and, for the split and gated
 // precisions, an FP32 table per direction: the WENO coefficients of those
 // cells ([kNumCoef][n + 2 kCoefPad]) followed by their inverse widths.
+// In 2-D those precisions hold the velocities and the face gradients as FP32
+// pairs of the two components in the same buffers (fg[0]: [d][ny][nx + 1]).
+// uniform: their coefficients, then the inverse width, as (c, c) pairs, when
+// every cell of each direction has the same.
+struct GradCoef {
+  int on = 0;
+  unsigned long long rec[2][kCoefRec] = {};
+};
 struct ViscGradBuffers {
+  GradCoef uniform;
   double* vel = nullptr;
   double* g = nullptr;
   double* fg[2] = {nullptr, nullptr};
   double* w[2] = {nullptr, nullptr};
   float* cf[2] = {nullptr, nullptr};
 };
-// Prepares the face gradients of the stage input q on stream st (3 launches
-// in 1-D, 4 in 2-D), reconstructing in FP32 when fp32 is set (split and
+// Launches of one preparation: 3 in 1-D, 4 in 2-D, 2 in 2-D with fp32.
+inline int visc_gradients_launches(int nd, bool fp32) { return nd == 1 ? 3 : fp32 ? 2 : 4; }
+// Prepares the face gradients of the stage input q on stream st, reconstructing in FP32 when fp32 is set (split and
 // gated contexts), else in FP64.
 cudaError_t visc_gradients_launch(int nd, int nf, bool fp32, const DevParams& P, const ViscGradBuffers& B,
                                   const double* q, cudaStream_t st);

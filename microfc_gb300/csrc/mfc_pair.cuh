@@ -514,11 +514,13 @@ __device__ __forceinline__ void pair_tile(const DevParams& P, const double* __re
             // for the rows and faces of partial tiles, whose results are dropped)
             const int gy = ND > 1 ? min(y0 + ty, ny - 1) : 0;
             const int64_t plane = (int64_t)(ND > 1 ? ny : 1) * (nx + 1);
-            const double* g = V.fg[0] + (int64_t)gy * (nx + 1) + (min(max(gface, -1), nx - 1) + 1);
-#pragma unroll
-            for (int c = 0; c < ND; ++c) {
-              dxv[c] = d2f_bits(__ldg(g + (c * ND) * plane));
-              if constexpr (ND > 1) dyv[c] = d2f_bits(__ldg(g + (c * ND + 1) * plane));
+            const int64_t o = (int64_t)gy * (nx + 1) + (min(max(gface, -1), nx - 1) + 1);
+            if constexpr (ND > 1) {  // pairs of the two components
+              const f32x2* g = reinterpret_cast<const f32x2*>(V.fg[0]) + o;
+              f2_unpack(__ldg(g), dxv[0], dxv[1]);
+              f2_unpack(__ldg(g + plane), dyv[0], dyv[1]);
+            } else {
+              dxv[0] = d2f_bits(__ldg(V.fg[0] + o));
             }
           } else {
             const int ly = ty + HY, lx = f + H - 1;  // the face's left cell
@@ -563,13 +565,10 @@ __device__ __forceinline__ void pair_tile(const DevParams& P, const double* __re
           const int gx = min(x0 + tx, nx - 1);
           if (V.fg[1] != nullptr) {
             // weno_Re_flux = T: the prepared face gradients
-            const int64_t plane = (int64_t)(ny + 1) * nx;
-            const double* g = V.fg[1] + (int64_t)(min(max(gface, -1), ny - 1) + 1) * nx + gx;
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              dxv[c] = d2f_bits(__ldg(g + (c * 2) * plane));
-              dyv[c] = d2f_bits(__ldg(g + (c * 2 + 1) * plane));
-            }
+            const f32x2* g = reinterpret_cast<const f32x2*>(V.fg[1]) +
+                             (int64_t)(min(max(gface, -1), ny - 1) + 1) * nx + gx;
+            f2_unpack(__ldg(g), dxv[0], dxv[1]);
+            f2_unpack(__ldg(g + (int64_t)(ny + 1) * nx), dyv[0], dyv[1]);
           } else {
             const int ly = f + H - 1, lx = tx + H;  // the face's lower cell
             const auto Dy = divisor(d2f_bits(__ldg(V.dcc[1] + min(y0 + f, ny))));  // y_cc(k+1) - y_cc(k)

@@ -16,7 +16,8 @@
 // the plain path (the arithmetic and operation order of the oracle, so the
 // result is bit-identical to it), FP32 for the split and gated paths, whose
 // stage kernels take the gradients in FP32 anyway.  The buffers stay FP64
-// (an FP32 value widened, so the stage kernel narrows it back exactly).
+// (an FP32 value widened, so the stage kernel narrows it back exactly), but in
+// 2-D the split and gated paths take one tiled kernel and FP32 pairs (below).
 // Cells outside the domain take the boundary conditions by index mapping,
 // as everywhere else.
 //
@@ -99,6 +100,14 @@ __device__ __forceinline__ RT inverse_width(const DevParams& P, const double* __
   else return div_rn(1.0, divisor(__ldg(w + gi)));
 }
 
+// weno_cell on a record of RT coefficients, in the number type N.
+template <class RT, class N>
+__device__ __forceinline__ void grad_cell(const RT (&c)[kCoefRec], const N (&v)[5], const N& eps, const N& u0, N& vl,
+                                          N& vr) {
+  if constexpr (sizeof(RT) == 8) weno_cell<5, N>(NumCoef<N>{c, u0}, v, eps, vl, vr);
+  else weno_cell<5, N>(c, v, eps, vl, vr);
+}
+
 // Step 1 on the ncol x nrow cells from (ib, jb): out[c*ND+d][row][col].
 // B.w[d]: the cell widths ds of direction d for cells -kCoefPad ..
 // n-1+kCoefPad; B.cf[d]: the FP32 table of the direction.
@@ -109,7 +118,11 @@ __global__ void __launch_bounds__(256) visc_cell_gradients(const DevParams P, co
   const double* __restrict__ vel = B.vel;
   const int64_t cells = (int64_t)ncol * nrow;
   const int64_t vplane = (int64_t)vcol * vrow;
-  const RT eps = narrow<RT>(P.weno_eps);
+  using N = std::conditional_t<sizeof(RT) == 8, Num64, RT>;
+  N u0;
+  if constexpr (sizeof(RT) == 8) u0 = num64_unit(P.inv_d[0]);
+  else u0 = RT(0);
+  const N eps = lift(narrow<RT>(P.weno_eps), u0);
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < cells; t += (int64_t)gridDim.x * blockDim.x) {
     const int col = (int)(t % ncol), row = (int)(t / ncol);
     const int i = ib + col, j = jb + row;
@@ -121,15 +134,15 @@ __global__ void __launch_bounds__(256) visc_cell_gradients(const DevParams P, co
       const RT inv = inverse_width<RT>(P, B.w[d], B.cf[d], d, cell);
 #pragma unroll
       for (int c = 0; c < ND; ++c) {
-        RT st[5];
+        N st[5];
 #pragma unroll
         for (int o = 0; o < 5; ++o) {
           const int vi = i + (d == 0 ? o - 2 : 0) + 5, vj = ND > 1 ? j + (d == 1 ? o - 2 : 0) + 5 : 0;
-          st[o] = narrow<RT>(__ldg(vel + c * vplane + (int64_t)vj * vcol + vi));
+          st[o] = lift(narrow<RT>(__ldg(vel + c * vplane + (int64_t)vj * vcol + vi)), u0);
         }
-        RT vl, vr;
-        weno_cell<5, RT>(cf, st, eps, vl, vr);
-        out[((int64_t)(c * ND + d) * nrow + row) * ncol + col] = widen(inv * (vr - vl));
+        N vl, vr;
+        grad_cell(cf, st, eps, u0, vl, vr);
+        out[((int64_t)(c * ND + d) * nrow + row) * ncol + col] = widen(low(lift(inv, u0) * (vr - vl)));
       }
     }
   }
@@ -158,7 +171,11 @@ __global__ void __launch_bounds__(256) visc_face_gradients_x(const DevParams P, 
   const int64_t warps = (int64_t)chunks * nl;
   const int64_t plane_out = (int64_t)nf * nl;
   const int lane = threadIdx.x & 31;
-  const RT eps = narrow<RT>(P.weno_eps);
+  using N = std::conditional_t<sizeof(RT) == 8, Num64, RT>;
+  N u0;
+  if constexpr (sizeof(RT) == 8) u0 = num64_unit(P.inv_d[0]);
+  else u0 = RT(0);
+  const N eps = lift(narrow<RT>(P.weno_eps), u0);
   const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < warps; w += stride) {
     const int l = (int)(w / chunks), base = (int)(w % chunks) * 31;
@@ -169,13 +186,13 @@ __global__ void __launch_bounds__(256) visc_face_gradients_x(const DevParams P, 
     const double* row = G + (int64_t)(l - gjb) * gncol + (cell - gib);
 #pragma unroll
     for (int k = 0; k < ND * ND; ++k) {
-      RT st[5];
+      N st[5];
 #pragma unroll
-      for (int o = 0; o < 5; ++o) st[o] = narrow<RT>(__ldg(row + (int64_t)k * gnrow * gncol + (o - 2)));
-      RT vl, vr;
-      weno_cell<5, RT>(cf, st, eps, vl, vr);
-      const RT right = __shfl_up_sync(0xffffffffu, vr, 1);  // face value of the cell before
-      if (lane >= 1 && F < nf) out[k * plane_out + (int64_t)l * nf + F] = widen(RT(0.5) * (right + vl));
+      for (int o = 0; o < 5; ++o) st[o] = lift(narrow<RT>(__ldg(row + (int64_t)k * gnrow * gncol + (o - 2))), u0);
+      N vl, vr;
+      grad_cell(cf, st, eps, u0, vl, vr);
+      const RT right = __shfl_up_sync(0xffffffffu, low(vr), 1);  // face value of the cell before
+      if (lane >= 1 && F < nf) out[k * plane_out + (int64_t)l * nf + F] = widen(low(lift(RT(0.5), u0) * (lift(right, u0) + vl)));
     }
   }
 }
@@ -191,10 +208,14 @@ __global__ void __launch_bounds__(256) visc_face_gradients_y(const DevParams P, 
   const int runs = (nf + R - 1) / R;
   const int64_t items = (int64_t)nx * runs;
   const int64_t plane_out = (int64_t)nf * nx;
-  const RT eps = narrow<RT>(P.weno_eps);
+  using N = std::conditional_t<sizeof(RT) == 8, Num64, RT>;
+  N u0;
+  if constexpr (sizeof(RT) == 8) u0 = num64_unit(P.inv_d[0]);
+  else u0 = RT(0);
+  const N eps = lift(narrow<RT>(P.weno_eps), u0);
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < items; t += (int64_t)gridDim.x * blockDim.x) {
     const int l = (int)(t % nx), f0 = (int)(t / nx) * R;
-    RT prev[ND * ND];
+    N prev[ND * ND];
 #pragma unroll 1
     for (int j = -1; j < R; ++j) {
       const int cell = f0 + j;  // -1 .. ny
@@ -204,16 +225,229 @@ __global__ void __launch_bounds__(256) visc_face_gradients_y(const DevParams P, 
       const double* col = G + (int64_t)(cell - gjb) * gncol + (l - gib);
 #pragma unroll
       for (int k = 0; k < ND * ND; ++k) {
-        RT st[5];
+        N st[5];
 #pragma unroll
-        for (int o = 0; o < 5; ++o) st[o] = narrow<RT>(__ldg(col + ((int64_t)k * gnrow + (o - 2)) * gncol));
-        RT vl, vr;
-        weno_cell<5, RT>(cf, st, eps, vl, vr);
-        if (j >= 0) out[k * plane_out + (int64_t)cell * nx + l] = widen(RT(0.5) * (prev[k] + vl));
+        for (int o = 0; o < 5; ++o) st[o] = lift(narrow<RT>(__ldg(col + ((int64_t)k * gnrow + (o - 2)) * gncol)), u0);
+        N vl, vr;
+        grad_cell(cf, st, eps, u0, vl, vr);
+        if (j >= 0) out[k * plane_out + (int64_t)cell * nx + l] = widen(low(lift(RT(0.5), u0) * (prev[k] + vl)));
         prev[k] = vr;
       }
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// 2-D split and gated contexts: one tiled kernel in place of the cell- and
+// face-gradient kernels, on pairs (d u/d x_d, d v/d x_d).
+//
+// The unfused FP32 kernels were bound by issue: 12 scalar reconstructions a
+// cell with 12 IEEE divisions each, 27 coefficient loads per cell and
+// direction, intermediates widened to FP64 through L2 (130 us a stage at
+// 1024x512).  Here a block takes 32x16 faces of each direction: velocities
+// with a halo of 5, both cell gradients with a halo of 3 and the face values
+// live in shared memory, both components are reconstructed by packed FP32
+// operations, and a
+// uniform grid's coefficients come from the parameters.  Measured at 1024x512:
+// 130 -> 30 us a stage with the velocities; a split weno_Re_flux step 621 ->
+// 288 us.
+constexpr int kGX = 32, kGY = 16, kGT = 256;
+struct GradShape {
+  static constexpr int UX = kGX + 9, UY = kGY + 9;    // velocities: x0-5 .. x0+kGX+3
+  static constexpr int GX = kGX + 5, GY = kGY + 5;    // cell gradients: x0-3 .. x0+kGX+1
+  static constexpr int PX = kGX + 1, PY = kGY + 1;    // reconstructed cells: x0-1 .. x0+kGX-1
+  static constexpr int NU = UX * UY, NG = GX * GY, NX = PX * kGY, NY = PY * kGX;
+  static constexpr size_t kBytes = sizeof(f32x2) * size_t(NU + 2 * NG + 4 * (NX > NY ? NX : NY));
+};
+
+// One pair's reconstruction from its stencil: weno5_pair_diffs (mfc_device.cuh)
+// with two changes.  The weights act on the candidates' increments over the
+// cell's value, v + sum w_k (p_k - v), so that their rounding does not reach
+// the value itself: against FP64 (2^20 stencils each: smooth, noisy, jumps,
+// random) its errors are below those of the scalar form with IEEE divisions
+// that the unfused kernels used.  And 1 / b_k is squared after scaling by the
+// smallest b (only ratios enter the weights): b_k^2 would leave FP32 at
+// gradient jumps of 2^31, which small cells reach.
+template <class Coef>
+__device__ __forceinline__ void grad_weno(const Coef& C, const f32x2 (&v)[5], const f32x2 eps, f32x2& vL, f32x2& vR) {
+  const f32x2 d1 = f2_sub(v[4], v[3]), d0 = f2_sub(v[3], v[2]), dm1 = f2_sub(v[2], v[1]), dm2 = f2_sub(v[1], v[0]);
+  const f32x2 b0 = f2_fma(d1, f2_fma(C(kBeta + 0), d1, f2_mul(C(kBeta + 1), d0)), f2_fma(f2_mul(C(kBeta + 2), d0), d0, eps));
+  const f32x2 b1 = f2_fma(d0, f2_fma(C(kBeta + 3), d0, f2_mul(C(kBeta + 4), dm1)), f2_fma(f2_mul(C(kBeta + 5), dm1), dm1, eps));
+  const f32x2 b2 = f2_fma(dm1, f2_fma(C(kBeta + 6), dm1, f2_mul(C(kBeta + 7), dm2)), f2_fma(f2_mul(C(kBeta + 8), dm2), dm2, eps));
+  float x0, x1, x2, y0, y1, y2;
+  f2_unpack(b0, x0, y0);
+  f2_unpack(b1, x1, y1);
+  f2_unpack(b2, x2, y2);
+  const f32x2 m = f2_pack(fminf(x0, fminf(x1, x2)), fminf(y0, fminf(y1, y2)));
+  const f32x2 t0 = f2_mul(m, f2_rcp(b0)), t1 = f2_mul(m, f2_rcp(b1)), t2 = f2_mul(m, f2_rcp(b2));
+  const f32x2 r0 = f2_mul(t0, t0), r1 = f2_mul(t1, t1), r2 = f2_mul(t2, t2);
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    const int kP = side ? kPR : kPL, kD = side ? kDR : kDL;
+    const f32x2 p0 = f2_fma(C(kP + 1), d0, f2_mul(C(kP + 0), d1));
+    const f32x2 p1 = f2_fma(C(kP + 3), dm1, f2_mul(C(kP + 2), d0));
+    const f32x2 p2 = f2_fma(C(kP + 5), dm2, f2_mul(C(kP + 4), dm1));
+    const f32x2 a0 = f2_mul(C(kD + 0), r0), a1 = f2_mul(C(kD + 1), r1), a2 = f2_mul(C(kD + 2), r2);
+    const f32x2 is = f2_rcp(f2_add(f2_add(a0, a1), a2));
+    const f32x2 val = f2_fma(f2_mul(a2, is), p2, f2_fma(f2_mul(a1, is), p1, f2_fma(f2_mul(a0, is), p0, v[2])));
+    if (side) vR = val;
+    else vL = val;
+  }
+}
+
+// vel: the velocities as (u, v) pairs, [ny + 10][nx + 10] from x = y = -5.
+// fx, fy: the face gradients, pairs of components: [d][ny][nx + 1] and
+// [d][ny + 1][nx] (face F between cells F - 1 and F).
+// UNI: the shared coefficients U of a uniform grid, else per-cell ones (two
+// kernels: together their code missed the instruction cache).
+template <bool UNI>
+__global__ void __launch_bounds__(kGT) visc_gradients_tiled(const DevParams P, const __grid_constant__ GradCoef U,
+                                                           const float* __restrict__ cfx,
+                                                           const float* __restrict__ cfy,
+                                                           const f32x2* __restrict__ vel, f32x2* __restrict__ fx,
+                                                           f32x2* __restrict__ fy) {
+  using Sh = GradShape;
+  extern __shared__ __align__(16) f32x2 grad_smem[];
+  f32x2* const su = grad_smem;          // [UY][UX]
+  f32x2* const sg = su + Sh::NU;        // [d][GY][GX]
+  f32x2* const sl = sg + 2 * Sh::NG;    // [d][..] left values
+  f32x2* const sr = sl + 2 * (Sh::NX > Sh::NY ? Sh::NX : Sh::NY);
+  const int tid = threadIdx.x, nx = P.n[0], ny = P.n[1];
+  const int x0 = blockIdx.x * kGX, y0 = blockIdx.y * kGY;
+  const f32x2 eps2 = f2_pack(P.weno_eps_f, P.weno_eps_f);
+  const f32x2 half = f2_pack(0.5f, 0.5f);
+  griddep_wait();
+  for (int it = tid; it < Sh::NU; it += kGT) {
+    const int r = it / Sh::UX, c = it - r * Sh::UX;
+    // cells past the buffer (partial tiles) are never used
+    su[it] = __ldg(vel + (int64_t)min(y0 + r, ny + 9) * (nx + 10) + min(x0 + c, nx + 9));
+  }
+  __syncthreads();
+  // with the coefficients of cell `cell` along direction d
+  auto with_coef = [&](auto dir, const int cell, auto&& use) {
+    constexpr int D = decltype(dir)::value;
+    if constexpr (UNI) {
+      use([&](int k) { return f32x2(U.rec[D][k]); }, f32x2(U.rec[D][kNumCoef]));
+    } else {
+      float c[kCoefRec];
+      const float* cf = D == 0 ? cfx : cfy;
+      coef_of<float>(P, cf, D, cell, c);
+      const float inv = inverse_width<float>(P, nullptr, cf, D, cell);
+      use([&](int k) { return f2_pack(c[k], c[k]); }, f2_pack(inv, inv));
+    }
+  };
+  // step 1: the cell gradients that a face of the tile needs: the tile's rows
+  // with all columns, then the other rows of the tile's columns
+  constexpr int kA = kGY * Sh::GX, kB = (Sh::GY - kGY) * kGX;
+  for (int it = tid; it < 2 * (kA + kB); it += kGT) {
+    const int d = it >= kA + kB, i = d ? it - (kA + kB) : it;
+    int gx, gy;
+    if (i < kA) {
+      gy = 3 + i / Sh::GX;
+      gx = i % Sh::GX;
+    } else {
+      const int r = (i - kA) / kGX;
+      gy = r < 3 ? r : kGY + r;
+      gx = 3 + (i - kA) % kGX;
+    }
+    const f32x2* at = su + (gy + 2) * Sh::UX + gx + 2;  // the cell: x0 - 3 + gx
+    f32x2 v[5], vl, vr;
+    auto recon = [&](const auto& C, const f32x2 inv) {
+      grad_weno(C, v, eps2, vl, vr);
+      sg[d * Sh::NG + gy * Sh::GX + gx] = f2_mul(inv, f2_sub(vr, vl));
+    };
+    if (d == 0) {
+#pragma unroll
+      for (int k = 0; k < 5; ++k) v[k] = at[k - 2];
+      with_coef(KindC<0>{}, min(x0 - 3 + gx, nx + 2), recon);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 5; ++k) v[k] = at[(k - 2) * Sh::UX];
+      with_coef(KindC<1>{}, min(y0 - 3 + gy, ny + 2), recon);
+    }
+  }
+  __syncthreads();
+  // step 2, x faces: both gradient pairs along the rows
+  for (int it = tid; it < 2 * Sh::NX; it += kGT) {
+    const int d = it >= Sh::NX, i = d ? it - Sh::NX : it, r = i / Sh::PX, c = i - r * Sh::PX;  // cell x0 - 1 + c
+    const f32x2* at = sg + d * Sh::NG + (r + 3) * Sh::GX + c + 2;
+    f32x2 v[5], vl, vr;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) v[k] = at[k - 2];
+    with_coef(KindC<0>{}, min(x0 - 1 + c, nx), [&](const auto& C, f32x2) { grad_weno(C, v, eps2, vl, vr); });
+    sl[d * Sh::NX + i] = vl;
+    sr[d * Sh::NX + i] = vr;
+  }
+  __syncthreads();
+  for (int it = tid; it < 2 * kGX * kGY; it += kGT) {
+    const int d = it / (kGX * kGY), i = it % (kGX * kGY), r = i / kGX, f = i % kGX;
+    const int F = x0 + f, y = y0 + r;
+    if (F > nx || y >= ny) continue;
+    const int o = d * Sh::NX + r * Sh::PX + f;
+    fx[((int64_t)d * ny + y) * (nx + 1) + F] = f2_mul(half, f2_add(sr[o], sl[o + 1]));
+  }
+  __syncthreads();
+  // y faces: along the columns
+  for (int it = tid; it < 2 * Sh::NY; it += kGT) {
+    const int d = it >= Sh::NY, i = d ? it - Sh::NY : it, r = i / kGX, c = i - r * kGX;  // cell y0 - 1 + r
+    const f32x2* at = sg + d * Sh::NG + (r + 2) * Sh::GX + c + 3;
+    f32x2 v[5], vl, vr;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) v[k] = at[(k - 2) * Sh::GX];
+    with_coef(KindC<1>{}, min(y0 - 1 + r, ny), [&](const auto& C, f32x2) { grad_weno(C, v, eps2, vl, vr); });
+    sl[d * Sh::NY + i] = vl;
+    sr[d * Sh::NY + i] = vr;
+  }
+  __syncthreads();
+  for (int it = tid; it < 2 * kGX * kGY; it += kGT) {
+    const int d = it / (kGX * kGY), i = it % (kGX * kGY), r = i / kGX, c = i % kGX;
+    const int F = y0 + r, x = x0 + c;
+    if (F > ny || x >= nx) continue;
+    const int o = d * Sh::NY + r * kGX + c;
+    fy[((int64_t)d * (ny + 1) + F) * nx + x] = f2_mul(half, f2_add(sr[o], sl[o + kGX]));
+  }
+}
+
+// The velocities of visc_velocities as FP32 (u, v) pairs.
+template <int NF>
+__global__ void __launch_bounds__(256) visc_velocity_pairs(const DevParams P, const double* __restrict__ q,
+                                                          const int ncol, const int nrow, f32x2* __restrict__ vel) {
+  const int64_t cells = (int64_t)ncol * nrow;
+  const double one = fma64_unit(P.inv_d[0]).one;
+  griddep_wait();
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < cells; t += (int64_t)gridDim.x * blockDim.x) {
+    const int col = (int)(t % ncol), row = (int)(t / ncol);
+    bool fx = false, fy = false;
+    const int gx = map_cell(col - 5, P.n[0], P.bc_beg[0], P.bc_end[0], &fx);
+    const int gy = map_cell(row - 5, P.n[1], P.bc_beg[1], P.bc_end[1], &fy);
+    const double* c = q + (int64_t)gy * P.sy + gx;
+    double rho = __ldg(c);
+#pragma unroll
+    for (int f = 1; f < NF; ++f) rho = __fma_rn(rho, one, __ldg(c + f * P.sv));
+    // fmax(rho, 1e-16) on the bits, which order like the values of positive
+    // numbers (a comparison would occupy the FP64 unit); NaN gives 1e-16 too
+    const long long b = __double_as_longlong(rho);
+    if (b < __double_as_longlong(1e-16) || b > 0x7ff0000000000000ll) rho = 1e-16;
+    const DivisorF64 R = divisor(rho);
+    const double mu = __ldg(c + NF * P.sv), mv = __ldg(c + (NF + 1) * P.sv);
+    vel[t] = f2_pack(d2f_bits(div_rn(fx ? -mu : mu, R)), d2f_bits(div_rn(fy ? -mv : mv, R)));
+  }
+}
+
+template <int NF>
+cudaError_t launch_tiled(const DevParams& P, const ViscGradBuffers& B, const double* q, cudaStream_t st) {
+  const int nx = P.n[0], ny = P.n[1], vcol = nx + 10, vrow = ny + 10;
+  const int64_t cells = (int64_t)vcol * vrow;
+  cudaError_t e = launch_dependent(&visc_velocity_pairs<NF>, dim3((unsigned)std::min<int64_t>((cells + 255) / 256, 152 * 16)),
+                                   dim3(256), 0, st, P, q, vcol, vrow, reinterpret_cast<f32x2*>(B.vel));
+  if (e != cudaSuccess) return e;
+  const auto kernel = B.uniform.on ? visc_gradients_tiled<true> : visc_gradients_tiled<false>;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GradShape::kBytes);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((unsigned)(nx / kGX + 1), (unsigned)(ny / kGY + 1));  // nx + 1 and ny + 1 faces
+  return launch_dependent(kernel, grid, dim3(kGT), GradShape::kBytes, st, P, B.uniform, B.cf[0], B.cf[1],
+                          reinterpret_cast<const f32x2*>(B.vel), reinterpret_cast<f32x2*>(B.fg[0]),
+                          reinterpret_cast<f32x2*>(B.fg[1]));
 }
 
 template <int ND, int NF, class RT>
@@ -233,7 +467,7 @@ cudaError_t launch_all(const DevParams& P, const ViscGradBuffers& B, const doubl
   visc_face_gradients_x<ND, RT><<<grid(32 * xwarps), 256, 0, st>>>(P, B.cf[0], B.g, -3, gjb, gcol, grow, B.fg[0]);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if constexpr (ND > 1) {
-    constexpr int R = sizeof(RT) == 8 ? 8 : 4;  // faces per thread (FP32 wants more threads)
+    constexpr int R = 8;  // faces per thread
     visc_face_gradients_y<ND, RT, R><<<grid((int64_t)nx * ((ny + 1 + R - 1) / R)), 256, 0, st>>>(
         P, B.cf[1], B.g, -3, gjb, gcol, grow, B.fg[1]);
     e = cudaGetLastError();
@@ -249,8 +483,8 @@ cudaError_t visc_gradients_launch(int nd, int nf, bool fp32, const DevParams& P,
     if (B.cf[0] == nullptr || (nd > 1 && B.cf[1] == nullptr)) return cudaErrorInvalidValue;
     if (nd == 1 && nf == 1) return launch_all<1, 1, float>(P, B, q, st);
     if (nd == 1 && nf == 2) return launch_all<1, 2, float>(P, B, q, st);
-    if (nd == 2 && nf == 1) return launch_all<2, 1, float>(P, B, q, st);
-    if (nd == 2 && nf == 2) return launch_all<2, 2, float>(P, B, q, st);
+    if (nd == 2 && nf == 1) return launch_tiled<1>(P, B, q, st);
+    if (nd == 2 && nf == 2) return launch_tiled<2>(P, B, q, st);
   } else {
     if (nd == 1 && nf == 1) return launch_all<1, 1, double>(P, B, q, st);
     if (nd == 1 && nf == 2) return launch_all<1, 2, double>(P, B, q, st);
