@@ -14,7 +14,7 @@
 
 namespace mfc {
 
-constexpr int kMaxFluids = 4;
+constexpr int kMaxFluids = 2;  // what the kernels are compiled for (validate_params refuses more)
 constexpr int kNumCoef = 27;  // per cell: polyL[3][2], polyR[3][2], dL[3], dR[3], beta[3][3]
 // offsets inside one coefficient record
 constexpr int kPL = 0, kPR = 6, kDL = 12, kDR = 15, kBeta = 18;

@@ -53,6 +53,7 @@ struct mfc_gpu_ensemble {
   std::vector<double> dt;
   double* state = nullptr;
   double* tables = nullptr;
+  mfc::f32x2* prim = nullptr;  // split and gated: every case's primitive pairs, two buffers each
   uint32_t* status = nullptr;
   void* gate_w = nullptr;  // MFC_PREC_GATED: FP16 gate parameters
   uint8_t* gate_flags = nullptr;  // MFC_PREC_GATED: every case's first-stage gate decisions
@@ -76,9 +77,8 @@ int configure(mfc_gpu_ensemble* e, const mfc::EnsembleEntry* en) {
   cudaError_t err = cudaFuncSetAttribute(en->func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)en->smem);
   if (err != cudaSuccess) return mfc::report_error(MFC_ERR_CUDA, cudaGetErrorString(err));
   const size_t smem = (e->U.on[0] && e->U.on[1]) ? en->smem_shared_coef : en->smem;
-  int bps = 0, sms = 0;
+  int bps = 0;
   err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, en->func, en->nt, smem);
-  if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
   if (err != cudaSuccess) return mfc::report_error(MFC_ERR_CUDA, cudaGetErrorString(err));
   if (bps < 1) return mfc::report_error(MFC_ERR_INVALID, "ensemble tile variant does not fit on an SM");
   int base = 0;
@@ -89,19 +89,21 @@ int configure(mfc_gpu_ensemble* e, const mfc::EnsembleEntry* en) {
     base += tx * ty;
   }
   e->total_tiles = base;
-  e->grid = std::min(base, bps * sms);
+  e->grid = base;
   e->smem = smem;
   e->entry = en;
   if (en->tma && e->maps) {
     // the maps of this variant's box, in stream order after any launch of
     // the previous variant that reads them
     std::vector<mfc::TileMap> maps(3 * (size_t)e->num);
-    for (int r = 0; r < 3; ++r)
-      for (int i = 0; i < e->num; ++i) {
-        const mfc::EnsCase& C = e->cases[i];
-        mfc::encode_tile_map(maps[(size_t)r * e->num + i], C.reg[r], e->nx[i], e->ny[i], 2 * e->nf + 3, C.P.sy,
-                             C.P.sv, en->box_w, en->box_h);
-      }
+    for (int i = 0; i < e->num; ++i) {
+      const mfc::EnsCase& C = e->cases[i];
+      mfc::encode_tile_map(maps[i], C.reg[0], e->nx[i], e->ny[i], 2 * e->nf + 3, C.P.sy, C.P.sv, en->box_w, en->box_h);
+      const int64_t pitch = mfc::prim_pitch(e->nx[i]);
+      for (int k = 0; k < 2; ++k)
+        mfc::encode_tile_map(maps[(size_t)(k + 1) * e->num + i], reinterpret_cast<const double*>(C.prim[k]), (int)pitch,
+                             e->ny[i], e->nf + 2, pitch, pitch * e->ny[i], en->tx + 6, en->ty + 6);
+    }
     err = cudaMemcpyAsync(e->maps, maps.data(), sizeof(mfc::TileMap) * maps.size(), cudaMemcpyHostToDevice,
                           e->stream);
     if (err != cudaSuccess) return mfc::report_error(MFC_ERR_CUDA, cudaGetErrorString(err));
@@ -187,9 +189,9 @@ int mfc_gpu_ensemble_init(const mfc_params* cases, const double* dts, int num_ca
   };
 
   // sizes, grid tables
-  std::vector<int64_t> reg_off(num_cases), tab_off(num_cases);
+  std::vector<int64_t> reg_off(num_cases), tab_off(num_cases), prim_off(num_cases);
   std::vector<mfc::GridTables> gts(num_cases);
-  int64_t state_elems = 0, table_elems = 0;
+  int64_t state_elems = 0, table_elems = 0, prim_elems = 0;
   const int b = (c0.weno_order - 1) / 2 + 2;
   for (int i = 0; i < num_cases; ++i) {
     const mfc_params& p = cases[i];
@@ -229,6 +231,8 @@ int mfc_gpu_ensemble_init(const mfc_params* cases, const double* dts, int num_ca
     const int S = 2 * p.num_fluids + 3;
     reg_off[i] = state_elems;
     state_elems += 3 * D.sv * S;
+    prim_off[i] = prim_elems;
+    prim_elems += 2 * (int64_t)(p.num_fluids + 2) * mfc::prim_pitch(n[0]) * n[1];
     tab_off[i] = table_elems;
     table_elems += (int64_t)gts[i].host.size();
   }
@@ -236,6 +240,8 @@ int mfc_gpu_ensemble_init(const mfc_params* cases, const double* dts, int num_ca
       (err = cudaMalloc(&e->state, sizeof(double) * state_elems)) != cudaSuccess ||
       (err = cudaMalloc(&e->tables, sizeof(double) * table_elems)) != cudaSuccess ||
       (err = cudaMalloc(&e->status, sizeof(uint32_t))) != cudaSuccess ||
+      (c0.precision != MFC_PREC_FP64 &&
+       (err = cudaMalloc(&e->prim, sizeof(mfc::f32x2) * prim_elems)) != cudaSuccess) ||
       (err = cudaMalloc(&e->maps, sizeof(mfc::TileMap) * 3 * (size_t)num_cases)) != cudaSuccess ||
       (c0.precision == MFC_PREC_GATED && (err = cudaMalloc(&e->gate_w, mfc::kGateBufferBytes)) != cudaSuccess))
     return cleanup(mfc::report_error(MFC_ERR_NOMEM, cudaGetErrorString(err)));
@@ -250,6 +256,8 @@ int mfc_gpu_ensemble_init(const mfc_params* cases, const double* dts, int num_ca
     mfc::EnsCase& C = e->cases[i];
     const int S = 2 * cases[i].num_fluids + 3;
     for (int r = 0; r < 3; ++r) C.reg[r] = e->state + reg_off[i] + r * C.P.sv * S;
+    for (int k = 0; k < 2 && e->prim; ++k)
+      C.prim[k] = e->prim + prim_off[i] + k * (int64_t)(cases[i].num_fluids + 2) * mfc::prim_pitch(e->nx[i]) * e->ny[i];
     double* tb = e->tables + tab_off[i];
     if ((err = cudaMemcpyAsync(tb, gts[i].host.data(), sizeof(double) * gts[i].host.size(), cudaMemcpyHostToDevice,
                                e->stream)) != cudaSuccess)
@@ -519,6 +527,7 @@ int mfc_gpu_ensemble_finalize(mfc_gpu_ensemble* e) {
   if (e->stream) cudaStreamSynchronize(e->stream);
   cudaFree(e->state);
   cudaFree(e->tables);
+  cudaFree(e->prim);
   cudaFree(e->status);
   cudaFree(e->gate_w);
   cudaFree(e->gate_flags);

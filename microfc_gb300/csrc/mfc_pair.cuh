@@ -117,18 +117,18 @@ struct PrimPairs {
   f32x2* out;
   int64_t pitch, plane;
 };
-inline int64_t prim_pitch(int nx) { return (nx + 2 + 15) / 16 * 16; }
+__host__ __device__ inline int64_t prim_pitch(int nx) { return (nx + 2 + 15) / 16 * 16; }
 
 // One tile of one RK stage; the tile's first cell is (x0, y0).  U: shared
 // coefficient records; T: the TMA map of B.in, or of the stage input where
-// that is null (TMA kernels); tma_parity: given by a block that walks many
-// tiles (the ensemble).
+// that is null (TMA kernels), in the kernel's parameters or, map_in_memory
+// (the ensemble's), in global memory.
 template <int ND, int NF, int TX, int TY, int NT, bool GATE, bool VISC, class UC, bool TMA, int RX, int RY>
 __device__ __forceinline__ void pair_tile(const DevParams& P, const double* __restrict__ qin,
                                           const double* __restrict__ qbase, double* __restrict__ qout,
                                           const double dt, const int kind, const int x0, const int y0,
                                           unsigned char* smem_raw, const UC* U, const PrimPairs& B,
-                                          const TileMap* T = nullptr, uint32_t* tma_parity = nullptr) {
+                                          const TileMap* T = nullptr, const bool map_in_memory = false) {
   using Sh = PairShape<ND, NF, TX, TY, VISC>;
   using Q = Eqs<ND, NF>;
   constexpr int S = Sh::S, H = Sh::H, NPR = Sh::NPR, LX = Sh::LX, LY = Sh::LY, TYE = Sh::TYE;
@@ -215,9 +215,7 @@ __device__ __forceinline__ void pair_tile(const DevParams& P, const double* __re
     if (use_tma) {
       stg = pair_staging<ND, NF, TX, TY, VISC>(smem_raw);  // B.in: only its barrier and flag are used
       bar = smem_addr(stg + Sh::kStageBytes);
-      // one tile per block: a fresh barrier; a block walking many tiles
-      // initialised it once and alternates its phase
-      if (tid == 0 && tma_parity == nullptr) mbar_init(bar, 1);
+      if (tid == 0) mbar_init(bar, 1);
     }
   }
   griddep_wait();  // the state below is the previous stage's output
@@ -268,15 +266,9 @@ __device__ __forceinline__ void pair_tile(const DevParams& P, const double* __re
     }
   }
   if (use_tma) {
-    const uint32_t par = tma_parity ? *tma_parity : 0u;
     volatile int* landed = reinterpret_cast<volatile int*>(stg + Sh::kStageBytes + 8);
     if (tid == 0) {
-      // a walking block: its reads of this memory for the previous tile come
-      // first, and its maps live in global memory
-      if (tma_parity) {
-        fence_proxy_async_smem();
-        tensormap_acquire(&T->map);
-      }
+      if (map_in_memory) tensormap_acquire(&T->map);
       if (B.in != nullptr) {
         mbar_arrive_expect_tx(bar, uint32_t(Sh::NQ * sizeof(f32x2)));
         tma_load_3d(smem_addr(sq), &T->map, x0 - H + 1, y0 - H, 0, bar);
@@ -284,8 +276,8 @@ __device__ __forceinline__ void pair_tile(const DevParams& P, const double* __re
         mbar_arrive_expect_tx(bar, Sh::kStageBytes);
         tma_load_3d(smem_addr(stg), &T->map, x0 - Box::kLead, y0 - H, 0, bar);
       }
-      const bool ok = mbar_wait_bounded(bar, par, 1000000000ull);  // 1 s
-      if (!ok) (void)mbar_wait_bounded(bar, par, 1000000000ull);    // the copy may still be in flight
+      const bool ok = mbar_wait_bounded(bar, 0, 1000000000ull);  // 1 s
+      if (!ok) (void)mbar_wait_bounded(bar, 0, 1000000000ull);    // the copy may still be in flight
       *landed = ok ? 1 : 0;
     }
     __syncthreads();
@@ -293,8 +285,7 @@ __device__ __forceinline__ void pair_tile(const DevParams& P, const double* __re
       if (tid == 0 && P.status) atomicOr(P.status, MFC_FLAG_TIMEOUT);
       return;
     }
-    (void)mbar_try_wait(bar, par);  // completed: each thread acquires the copy's writes
-    if (tma_parity) *tma_parity ^= 1u;
+    (void)mbar_try_wait(bar, 0);  // completed: each thread acquires the copy's writes
     const double* sd = reinterpret_cast<const double*>(stg);
     for (int c = B.in != nullptr ? WX * LY : tid; c < WX * LY; c += NT) {
       const int lx = c % WX, ly = c / WX;
