@@ -247,10 +247,9 @@ __global__ void __launch_bounds__(256) visc_face_gradients_y(const DevParams P, 
 // 1024x512).  Here a block takes 32x16 faces of each direction: velocities
 // with a halo of 5, both cell gradients with a halo of 3 and the face values
 // live in shared memory, both components are reconstructed by packed FP32
-// operations, and a
-// uniform grid's coefficients come from the parameters.  Measured at 1024x512:
-// 130 -> 30 us a stage with the velocities; a split weno_Re_flux step 621 ->
-// 288 us.
+// operations that round as weno_cell's do, and a uniform grid's coefficients
+// come from the parameters.  Measured at 1024x512: 130 -> 48 us a stage with
+// the velocities; a split weno_Re_flux step 604 -> 338 us.  Bound by FP32 issue.
 constexpr int kGX = 32, kGY = 16, kGT = 256;
 struct GradShape {
   static constexpr int UX = kGX + 9, UY = kGY + 9;    // velocities: x0-5 .. x0+kGX+3
@@ -260,36 +259,49 @@ struct GradShape {
   static constexpr size_t kBytes = sizeof(f32x2) * size_t(NU + 2 * NG + 4 * (NX > NY ? NX : NY));
 };
 
-// One pair's reconstruction from its stencil: weno5_pair_diffs (mfc_device.cuh)
-// with two changes.  The weights act on the candidates' increments over the
-// cell's value, v + sum w_k (p_k - v), so that their rounding does not reach
-// the value itself: against FP64 (2^20 stencils each: smooth, noisy, jumps,
-// random) its errors are below those of the scalar form with IEEE divisions
-// that the unfused kernels used.  And 1 / b_k is squared after scaling by the
-// smallest b (only ratios enter the weights): b_k^2 would leave FP32 at
-// gradient jumps of 2^31, which small cells reach.
+// One pair's reconstruction from its stencil: weno_cell's operations in their
+// order, rounded one by one, two variables at a time.  The quotients are
+// Markstein's (Handbook of Floating-Point Arithmetic, 2nd ed., ch. 4.7): the
+// reciprocal refined by a Newton step, the quotient corrected by its exact
+// remainder -- the IEEE quotient but for rare last bits, at a third of its
+// instructions, and the reciprocal of b_k^2 serves both faces, that of the
+// sum all three weights.  A product that a sum takes is fma(a, b, nz) with
+// nz = -0 in a register: ptxas contracts packed multiplies and adds whatever
+// their rounding modifiers say.  b_k is scaled by 2^-4 first, which leaves the
+// weights as they are and their divisors inside the reciprocal's range.
+__device__ __forceinline__ f32x2 f2_neg(f32x2 a) { return a ^ 0x8000000080000000ull; }
+__device__ __forceinline__ f32x2 f2_reciprocal(f32x2 a) {
+  const f32x2 r = f2_rcp(a);
+  return f2_fma(r, f2_fma(f2_neg(a), r, f2_pack(1.f, 1.f)), r);
+}
+__device__ __forceinline__ f32x2 f2_quotient(f32x2 n, f32x2 d, f32x2 r) {
+  const f32x2 q = f2_mul(n, r);
+  return f2_fma(f2_fma(f2_neg(d), q, n), r, q);
+}
 template <class Coef>
-__device__ __forceinline__ void grad_weno(const Coef& C, const f32x2 (&v)[5], const f32x2 eps, f32x2& vL, f32x2& vR) {
+__device__ __forceinline__ void grad_weno(const Coef& C, const f32x2 (&v)[5], const f32x2 eps, const f32x2 nz,
+                                          f32x2& vL, f32x2& vR) {
   const f32x2 d1 = f2_sub(v[4], v[3]), d0 = f2_sub(v[3], v[2]), dm1 = f2_sub(v[2], v[1]), dm2 = f2_sub(v[1], v[0]);
-  const f32x2 b0 = f2_fma(d1, f2_fma(C(kBeta + 0), d1, f2_mul(C(kBeta + 1), d0)), f2_fma(f2_mul(C(kBeta + 2), d0), d0, eps));
-  const f32x2 b1 = f2_fma(d0, f2_fma(C(kBeta + 3), d0, f2_mul(C(kBeta + 4), dm1)), f2_fma(f2_mul(C(kBeta + 5), dm1), dm1, eps));
-  const f32x2 b2 = f2_fma(dm1, f2_fma(C(kBeta + 6), dm1, f2_mul(C(kBeta + 7), dm2)), f2_fma(f2_mul(C(kBeta + 8), dm2), dm2, eps));
-  float x0, x1, x2, y0, y1, y2;
-  f2_unpack(b0, x0, y0);
-  f2_unpack(b1, x1, y1);
-  f2_unpack(b2, x2, y2);
-  const f32x2 m = f2_pack(fminf(x0, fminf(x1, x2)), fminf(y0, fminf(y1, y2)));
-  const f32x2 t0 = f2_mul(m, f2_rcp(b0)), t1 = f2_mul(m, f2_rcp(b1)), t2 = f2_mul(m, f2_rcp(b2));
-  const f32x2 r0 = f2_mul(t0, t0), r1 = f2_mul(t1, t1), r2 = f2_mul(t2, t2);
+  const f32x2 scale = f2_pack(0.0625f, 0.0625f);
+  auto indicator = [&](const int k, const f32x2 a, const f32x2 b) {  // (b_k 2^-4)^2
+    const f32x2 t0 = f2_fma(f2_mul(C(kBeta + 3 * k), a), a, nz), t1 = f2_fma(f2_mul(C(kBeta + 3 * k + 1), a), b, nz),
+                t2 = f2_fma(f2_mul(C(kBeta + 3 * k + 2), b), b, nz);
+    const f32x2 s = f2_mul(f2_add(f2_add(f2_add(t0, t1), t2), eps), scale);
+    return f2_mul(s, s);
+  };
+  const f32x2 D0 = indicator(0, d1, d0), D1 = indicator(1, d0, dm1), D2 = indicator(2, dm1, dm2);
+  const f32x2 r0 = f2_reciprocal(D0), r1 = f2_reciprocal(D1), r2 = f2_reciprocal(D2);
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
     const int kP = side ? kPR : kPL, kD = side ? kDR : kDL;
-    const f32x2 p0 = f2_fma(C(kP + 1), d0, f2_mul(C(kP + 0), d1));
-    const f32x2 p1 = f2_fma(C(kP + 3), dm1, f2_mul(C(kP + 2), d0));
-    const f32x2 p2 = f2_fma(C(kP + 5), dm2, f2_mul(C(kP + 4), dm1));
-    const f32x2 a0 = f2_mul(C(kD + 0), r0), a1 = f2_mul(C(kD + 1), r1), a2 = f2_mul(C(kD + 2), r2);
-    const f32x2 is = f2_rcp(f2_add(f2_add(a0, a1), a2));
-    const f32x2 val = f2_fma(f2_mul(a2, is), p2, f2_fma(f2_mul(a1, is), p1, f2_fma(f2_mul(a0, is), p0, v[2])));
+    const f32x2 p0 = f2_add(f2_add(v[2], f2_fma(C(kP + 0), d1, nz)), f2_fma(C(kP + 1), d0, nz));
+    const f32x2 p1 = f2_add(f2_add(v[2], f2_fma(C(kP + 2), d0, nz)), f2_fma(C(kP + 3), dm1, nz));
+    const f32x2 p2 = f2_add(f2_add(v[2], f2_fma(C(kP + 4), dm1, nz)), f2_fma(C(kP + 5), dm2, nz));
+    const f32x2 a0 = f2_quotient(C(kD + 0), D0, r0), a1 = f2_quotient(C(kD + 1), D1, r1),
+                a2 = f2_quotient(C(kD + 2), D2, r2);
+    const f32x2 s = f2_add(f2_add(a0, a1), a2), rs = f2_reciprocal(s);
+    const f32x2 val = f2_add(f2_add(f2_fma(f2_quotient(a0, s, rs), p0, nz), f2_fma(f2_quotient(a1, s, rs), p1, nz)),
+                             f2_fma(f2_quotient(a2, s, rs), p2, nz));
     if (side) vR = val;
     else vL = val;
   }
@@ -314,8 +326,12 @@ __global__ void __launch_bounds__(kGT) visc_gradients_tiled(const DevParams P, c
   f32x2* const sr = sl + 2 * (Sh::NX > Sh::NY ? Sh::NX : Sh::NY);
   const int tid = threadIdx.x, nx = P.n[0], ny = P.n[1];
   const int x0 = blockIdx.x * kGX, y0 = blockIdx.y * kGY;
-  const f32x2 eps2 = f2_pack(P.weno_eps_f, P.weno_eps_f);
+  const float eps = d2f_bits(P.weno_eps);  // cut like every value, where weno_eps_f is rounded
+  const f32x2 eps2 = f2_pack(eps, eps);
   const f32x2 half = f2_pack(0.5f, 0.5f);
+  // -0 in both lanes, opaque to the compiler as fma64_unit's constants are
+  const uint32_t sign = 0x80000000u | (uint32_t)(__double2hiint(__ldg(P.inv_d[0])) >> 31);
+  const f32x2 nz = (f32x2)sign << 32 | sign;
   griddep_wait();
   for (int it = tid; it < Sh::NU; it += kGT) {
     const int r = it / Sh::UX, c = it - r * Sh::UX;
@@ -353,7 +369,7 @@ __global__ void __launch_bounds__(kGT) visc_gradients_tiled(const DevParams P, c
     const f32x2* at = su + (gy + 2) * Sh::UX + gx + 2;  // the cell: x0 - 3 + gx
     f32x2 v[5], vl, vr;
     auto recon = [&](const auto& C, const f32x2 inv) {
-      grad_weno(C, v, eps2, vl, vr);
+      grad_weno(C, v, eps2, nz, vl, vr);
       sg[d * Sh::NG + gy * Sh::GX + gx] = f2_mul(inv, f2_sub(vr, vl));
     };
     if (d == 0) {
@@ -374,7 +390,7 @@ __global__ void __launch_bounds__(kGT) visc_gradients_tiled(const DevParams P, c
     f32x2 v[5], vl, vr;
 #pragma unroll
     for (int k = 0; k < 5; ++k) v[k] = at[k - 2];
-    with_coef(KindC<0>{}, min(x0 - 1 + c, nx), [&](const auto& C, f32x2) { grad_weno(C, v, eps2, vl, vr); });
+    with_coef(KindC<0>{}, min(x0 - 1 + c, nx), [&](const auto& C, f32x2) { grad_weno(C, v, eps2, nz, vl, vr); });
     sl[d * Sh::NX + i] = vl;
     sr[d * Sh::NX + i] = vr;
   }
@@ -394,7 +410,7 @@ __global__ void __launch_bounds__(kGT) visc_gradients_tiled(const DevParams P, c
     f32x2 v[5], vl, vr;
 #pragma unroll
     for (int k = 0; k < 5; ++k) v[k] = at[(k - 2) * Sh::GX];
-    with_coef(KindC<1>{}, min(y0 - 1 + r, ny), [&](const auto& C, f32x2) { grad_weno(C, v, eps2, vl, vr); });
+    with_coef(KindC<1>{}, min(y0 - 1 + r, ny), [&](const auto& C, f32x2) { grad_weno(C, v, eps2, nz, vl, vr); });
     sl[d * Sh::NY + i] = vl;
     sr[d * Sh::NY + i] = vr;
   }
