@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
   // primitive tile and the WENO values, reconstructed two at a time with
   // packed FP32 instructions (sys_size is even in 3-D)
   constexpr bool kPair = Sh::NCOEF > 0;
-  static_assert(!kPair || S % 2 == 0, "3-D pairs need an even number of variables");
+  static_assert(!kPair || (S % 2 == 0 && DIR == 0), "pairs: an even number of variables, the x sweep (y and z: mfc_pair_sweep.cuh)");
   auto qi = [](int v, int p, int la) {
     return kPair ? (((v >> 1) * NP + p) * LA + la) * 2 + (v & 1) : (v * NP + p) * LA + la;
   };
@@ -171,8 +171,14 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
 #pragma unroll
     for (int v = 0; v < S; ++v) sq[qi(v, p, la)] = pr[v];
     if (DIR == 0 && own >= 0) {
+      if constexpr (kPair) {  // as pairs, like the partial RHS
+        f32x2* const g = reinterpret_cast<f32x2*>(gprim) + own;
 #pragma unroll
-      for (int v = 0; v < S; ++v) gprim[own + v * P.sv] = pr[v];
+        for (int k = 0; k < S / 2; ++k) g[k * P.sv] = f2_pack(pr[2 * k], pr[2 * k + 1]);
+      } else {
+#pragma unroll
+        for (int v = 0; v < S; ++v) gprim[own + v * P.sv] = pr[v];
+      }
     }
   };
   // x sweep: the offset of tile cell (la, pb, pc) when the block owns it
@@ -450,25 +456,29 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
         const N a = num(sq[qi(Q::ADV + f, p, ta + H)]);
         r[Q::ADV + f] = mul_add(inv * a, du, r[Q::ADV + f]);
       }
-      if constexpr (DIR < 2) {
+      if constexpr (kPair) {
+        f32x2* const g = reinterpret_cast<f32x2*>(rhs_buf) + o;
+#pragma unroll
+        for (int k = 0; k < S / 2; ++k) g[k * P.sv] = f2_pack(r[2 * k], r[2 * k + 1]);
+      } else if constexpr (DIR < 2) {
 #pragma unroll
         for (int v = 0; v < S; ++v) rhs_buf[o + v * P.sv] = low(r[v]);
-        continue;
-      }
+      } else {
 #pragma unroll
-      for (int v = 0; v < S; ++v) {
-        double out;
-        if constexpr (KIND == kRhsOnly) {
-          out = widen(low(r[v]));
-        } else {
-          const double b = __ldg(qbase + o + v * P.sv);
-          double in = b;
-          if constexpr (KIND != kRkEuler) in = __ldg(qin + o + v * P.sv);
-          if constexpr (kSplit) out = rk_combine_split(KIND, b, in, dtf, r[v], one);
-          else out = rk_combine(KIND, num(b), num(in), num(dt), r[v]);
+        for (int v = 0; v < S; ++v) {
+          double out;
+          if constexpr (KIND == kRhsOnly) {
+            out = widen(low(r[v]));
+          } else {
+            const double b = __ldg(qbase + o + v * P.sv);
+            double in = b;
+            if constexpr (KIND != kRkEuler) in = __ldg(qin + o + v * P.sv);
+            if constexpr (kSplit) out = rk_combine_split(KIND, b, in, dtf, r[v], one);
+            else out = rk_combine(KIND, num(b), num(in), num(dt), r[v]);
+          }
+          bad |= not_finite(out);
+          qout[o + v * P.sv] = out;
         }
-        bad |= not_finite(out);
-        qout[o + v * P.sv] = out;
       }
     }
     // the stability monitor (the last stage of a monitored step) reads the
