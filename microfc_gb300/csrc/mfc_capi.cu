@@ -167,7 +167,7 @@ struct mfc_gpu_ctx {
   void* gate_w = nullptr;       // MFC_PREC_GATED: FP16 gate parameters
   uint8_t* gate_flags = nullptr;  // MFC_PREC_GATED: a step's first-stage gate decisions
   bool gate_ready = false;
-  // split and gated 2-D WENO5: the primitive pairs of the last stage's output
+  // split and gated 2-D and split 3-D WENO5: the primitive pairs of the last stage's output
   // (prim[prim_at]; of register prim_of, or of none), and the buffer that the
   // next stage writes them to
   mfc::f32x2* prim[2] = {nullptr, nullptr};
@@ -267,8 +267,11 @@ int launch_stage(mfc_gpu_ctx* c, const double* qin, const double* qbase, double*
   if (c->prim[0] != nullptr && c->stage->launch_prims != nullptr) {
     const bool keep = kind != mfc::kRhsOnly;  // an RHS evaluation makes no state
     const int64_t pitch = mfc::prim_pitch(c->n[0]);
-    const mfc::PrimPairs B{c->prim_of == qin ? c->prim[c->prim_at] : nullptr,
-                           keep ? c->prim[c->prim_at ^ 1] : nullptr, pitch, pitch * c->n[1]};
+    // 3-D stages always have the pairs of their input somewhere: an RHS
+    // evaluation's go where they spare the last stage's
+    const bool have = c->prim_of == qin;
+    const mfc::PrimPairs B{have ? c->prim[c->prim_at] : nullptr, keep ? c->prim[c->prim_at ^ 1] : nullptr, pitch,
+                           pitch * c->n[1], c->prim[have || keep ? c->prim_at : c->prim_at ^ 1]};
     e = c->stage->launch_prims(P, c->ucoef, qin, qbase, qout, dt, kind, B, c->stream);
     if (keep) {
       c->prim_at ^= 1;
@@ -444,9 +447,12 @@ int mfc_gpu_init(const mfc_params* p, mfc_gpu_ctx** out) {
         return cleanup(fail(MFC_ERR_NOMEM, cudaGetErrorString(e)));
   }
   // 3-D: the partial RHS, then the primitives the x sweep stores (S x sv
-  // values each, in the reconstruction type: FP64 at most)
+  // values each, in the reconstruction type: FP64 at most); split WENO5: three
+  // quarters of it, for the partial RHS and two buffers of primitive pairs
   if (c->nd == 3 && (e = cudaMalloc(&c->work, sizeof(double) * c->reg_elems * 2)) != cudaSuccess)
     return cleanup(fail(MFC_ERR_NOMEM, cudaGetErrorString(e)));
+  if (c->nd == 3 && p->weno_order == 5 && p->precision == MFC_PREC_SPLIT)
+    for (int k = 0; k < 2; ++k) c->prim[k] = reinterpret_cast<mfc::f32x2*>(c->work) + (k + 1) * (c->reg_elems / 2);
   if ((e = cudaMalloc(&c->monitor, sizeof(unsigned long long))) != cudaSuccess)
     return cleanup(fail(MFC_ERR_NOMEM, cudaGetErrorString(e)));
   cudaMemsetAsync(c->monitor, 0, sizeof(unsigned long long), c->stream);
@@ -1017,14 +1023,14 @@ int mfc_gpu_tune(mfc_gpu_ctx* c, int reps, int* variant_out, double* ms_out) {
     // first-stage launches read register 0 and write register 1 only; with
     // primitive pairs (of the same state, dt being 0) after the first
     const int64_t pitch = mfc::prim_pitch(c->n[0]);
-    mfc::PrimPairs B{nullptr, c->prim[0], pitch, pitch * c->n[1]};
+    mfc::PrimPairs B{nullptr, c->prim[0], pitch, pitch * c->n[1], c->prim[1]};
     auto once = [&] {
       if (c->prim[0] != nullptr && e.launch_prims != nullptr)
         return e.launch_prims(c->dev, c->ucoef, c->reg[0], c->reg[0], c->reg[1], 0.0, mfc::kRkEuler, B, c->stream);
       return e.launch(c->dev, c->ucoef, c->reg[0], c->reg[0], c->reg[1], 0.0, mfc::kRkEuler, c->stream);
     };
     if (once() != cudaSuccess) continue;
-    B.in = c->prim[0];
+    B.in = B.cur = c->prim[0];
     B.out = c->prim[1];
     cudaEventRecord(a, c->stream);
     for (int r = 0; r < reps; ++r) once();
@@ -1177,8 +1183,10 @@ int mfc_gpu_finalize(mfc_gpu_ctx* c) {
   cudaFree(c->tables);
   cudaFree(c->status);
   cudaFree(c->work);
-  cudaFree(c->prim[0]);
-  cudaFree(c->prim[1]);
+  if (c->nd < 3) {  // 3-D: parts of work
+    cudaFree(c->prim[0]);
+    cudaFree(c->prim[1]);
+  }
   cudaFree(c->scratch);
   cudaFree(c->vg.vel);
   cudaFree(c->vg.g);

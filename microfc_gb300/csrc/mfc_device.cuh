@@ -603,11 +603,6 @@ __device__ __forceinline__ void weno5_pair_diffs(const Coef& C, f32x2 v, f32x2 d
     else vL = val;
   }
 }
-template <class Coef>
-__device__ __forceinline__ void weno5_pair_fast(const Coef& C, const f32x2 (&v)[5], f32x2 eps, f32x2& vL,
-                                                f32x2& vR) {
-  weno5_pair_diffs(C, v[2], f2_sub(v[4], v[3]), f2_sub(v[3], v[2]), f2_sub(v[2], v[1]), f2_sub(v[1], v[0]), eps, vL, vR);
-}
 
 // WENO reconstruction of one cell from its stencil, m_weno.fpp:391-536.
 // c: the cell's kNumCoef coefficients; v[k] = value at offset k - 2.

@@ -387,29 +387,16 @@ struct Sweep3D {
   template <int DIR>
   using K = std::conditional_t<DIR == 0, SweepShape<NF, WO, RT, 0, TA0, TB0, TC0>,
                                SweepShape<NF, WO, RT, DIR, TA1, TB1, 1>>;
-  // split WENO5: the y and z sweeps on pairs
-  static constexpr bool kPair = sizeof(RT) == 4 && WO == 5;
-  static constexpr int kPairNT = 128, kPairRun = 9;
-  using KP = PairSweepShape<NF, TA1, TB1>;
-  template <int DIR>
-  static constexpr int threads() { return kPair && DIR > 0 ? kPairNT : NT; }
-  static size_t smem(int dir, const UniformCoef& U) {
-    if (dir == 0) return K<0>::kSmemBytes;
-    if constexpr (kPair) return KP::kCoefOffset + (U.on[dir] ? 0 : KP::kCoefBytes);
-    else return dir == 1 ? K<1>::kSmemBytes : K<2>::kSmemBytes;
-  }
   template <int DIR>
   static constexpr auto func() {
-    if constexpr (kPair && DIR > 0)
-      return &pair_sweep_kernel<NF, DIR, TA1, TB1, kPairNT, kPairRun, TMA, DIR == 2 ? MINB2 : MINB01>;
-    else if constexpr (DIR == 0) return &sweep_kernel<NF, WO, RT, 0, TA0, TB0, TC0, NT, TMA, kPair ? 0 : MINB01, CHAR>;
+    if constexpr (DIR == 0) return &sweep_kernel<NF, WO, RT, 0, TA0, TB0, TC0, NT, TMA, MINB01, CHAR>;
     else if constexpr (DIR == 2) return &sweep_kernel<NF, WO, RT, 2, TA1, TB1, 1, NT, TMA, MINB2, CHAR>;
     else return &sweep_kernel<NF, WO, RT, DIR, TA1, TB1, 1, NT, TMA, MINB01, CHAR>;
   }
 
   template <int DIR>
   static cudaError_t prep() {
-    return cudaFuncSetAttribute(func<DIR>(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(DIR, UniformCoef{}));
+    return cudaFuncSetAttribute(func<DIR>(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K<DIR>::kSmemBytes);
   }
   static cudaError_t prepare() {
     cudaError_t e = prep<0>();
@@ -423,12 +410,7 @@ struct Sweep3D {
   template <int DIR>
   static TileMap tile_map(const DevParams& P, const double* qin) {
     TileMap T{};
-    if constexpr (TMA && kPair && DIR > 0) {
-      // primitive pairs: 8-byte elements, a tile in its final layout
-      const void* base = static_cast<const f32x2*>(static_cast<const void*>(P.work)) + int64_t(KP::NPR) * P.sv;
-      encode_tile_map_3d(T, base, 8, P.n[0], P.n[1], P.n[2], KP::NPR, P.sy, P.sz, P.sv, TB1, DIR == 1 ? KP::LA : 1,
-                         DIR == 2 ? KP::LA : 1);
-    } else if constexpr (TMA && K<DIR>::kTmaFits) {
+    if constexpr (TMA && K<DIR>::kTmaFits) {
       constexpr int S = K<DIR>::S;
       const void* base = DIR == 0 ? static_cast<const void*>(qin)
                                   : static_cast<const void*>(static_cast<const RT*>(P.work) + int64_t(S) * P.sv);
@@ -445,18 +427,73 @@ struct Sweep3D {
     const dim3 g2((nx + TB1 - 1) / TB1, (nz + TA1 - 1) / TA1, ny);
     const TileMap T0 = tile_map<0>(P, qin), T1 = tile_map<1>(P, qin), T2 = tile_map<2>(P, qin);
     cudaError_t e =
-        launch_dependent(func<0>(), g0, dim3(threads<0>()), smem(0, U), st, P, U, T0, qin, qbase, qout, dt, kind);
+        launch_dependent(func<0>(), g0, dim3(NT), K<0>::kSmemBytes, st, P, T0, qin, qbase, qout, dt, kind);
     if (e == cudaSuccess)
-      e = launch_dependent(func<1>(), g1, dim3(threads<1>()), smem(1, U), st, P, U, T1, qin, qbase, qout, dt, kind);
+      e = launch_dependent(func<1>(), g1, dim3(NT), K<1>::kSmemBytes, st, P, T1, qin, qbase, qout, dt, kind);
     if (e == cudaSuccess)
-      e = launch_dependent(func<2>(), g2, dim3(threads<2>()), smem(2, U), st, P, U, T2, qin, qbase, qout, dt, kind);
+      e = launch_dependent(func<2>(), g2, dim3(NT), K<2>::kSmemBytes, st, P, T2, qin, qbase, qout, dt, kind);
     return e;
   }
   static StageEntry entry() {
     static_assert(!TMA || (K<0>::kTmaFits && K<1>::kTmaFits && K<2>::kTmaFits),
                   "the TMA box of every sweep must fit its WENO and flux arrays");
-    return StageEntry{3, NF, WO, sizeof(RT) == 8 ? 0 : 1, TA0, TB1, NT, smem(1, UniformCoef{}), 3, &prepare, &launch,
+    return StageEntry{3, NF, WO, sizeof(RT) == 8 ? 0 : 1, TA0, TB1, NT, K<1>::kSmemBytes, 3, &prepare, &launch,
                       false, TMA, CHAR};
+  }
+};
+
+// Split WENO5: the three sweeps on primitive pairs (mfc_pair_sweep.cuh), tiles
+// of TA cells along the sweep and 16 pencils.  TMA: interior tiles by one
+// bulk tensor copy.
+template <int NF, int TA, int NT, int R, bool TMA, int MINB>
+struct PairSweep3D {
+  static constexpr int TB = 16;
+  template <int DIR>
+  using K = PairSweepShape<NF, DIR, TA, TB>;
+  template <int DIR>
+  static constexpr auto func() {
+    return &pair_sweep_kernel<NF, DIR, TA, TB, NT, R, TMA, MINB>;
+  }
+  template <int DIR>
+  static cudaError_t prep() {
+    return cudaFuncSetAttribute(func<DIR>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(K<DIR>::kCoefOffset + K<DIR>::kCoefBytes));
+  }
+  static cudaError_t prepare() {
+    cudaError_t e = prep<0>();
+    if (e == cudaSuccess) e = prep<1>();
+    if (e == cudaSuccess) e = prep<2>();
+    return e;
+  }
+  template <int DIR>
+  static cudaError_t sweep(dim3 grid, const DevParams& P, const UniformCoef& U, const double* qin, const double* qbase,
+                           double* qout, double dt, int kind, const PrimPairs& B, cudaStream_t st) {
+    TileMap T{};
+    if constexpr (TMA)  // 8-byte elements, a tile in its final layout
+      encode_tile_map_3d(T, B.cur, 8, P.n[0], P.n[1], P.n[2], K<DIR>::NPR, P.sy, P.sz, P.sv,
+                         DIR == 0 ? K<DIR>::PLA : TB, DIR == 0 ? TB : DIR == 1 ? K<DIR>::LA : 1,
+                         DIR == 2 ? K<DIR>::LA : 1);
+    return launch_dependent(func<DIR>(), grid, dim3(NT), K<DIR>::kCoefOffset + (U.on[DIR] ? 0 : K<DIR>::kCoefBytes), st,
+                            P, U, T, qin, qbase, qout, dt, kind, B);
+  }
+  static cudaError_t launch_prims(const DevParams& P, const UniformCoef& U, const double* qin, const double* qbase,
+                                  double* qout, double dt, int kind, const PrimPairs& B, cudaStream_t st) {
+    const unsigned nx = P.n[0], ny = P.n[1], nz = P.n[2];
+    auto tiles = [](unsigned n, unsigned t) { return (n + t - 1) / t; };
+    cudaError_t e = sweep<0>(dim3(tiles(nx, TA), tiles(ny, TB), nz), P, U, qin, qbase, qout, dt, kind, B, st);
+    if (e == cudaSuccess) e = sweep<1>(dim3(tiles(nx, TB), tiles(ny, TA), nz), P, U, qin, qbase, qout, dt, kind, B, st);
+    if (e == cudaSuccess) e = sweep<2>(dim3(tiles(nx, TB), tiles(nz, TA), ny), P, U, qin, qbase, qout, dt, kind, B, st);
+    return e;
+  }
+  static cudaError_t launch(const DevParams& P, const UniformCoef& U, const double* qin, const double* qbase,
+                            double* qout, double dt, int kind, cudaStream_t st) {
+    const PrimPairs B{nullptr, nullptr, 0, 0, reinterpret_cast<f32x2*>(P.work) + int64_t(K<0>::NPR) * P.sv};
+    return launch_prims(P, U, qin, qbase, qout, dt, kind, B, st);
+  }
+  static StageEntry entry() {
+    StageEntry e{3, NF, 5, 1, TA, TB, NT, K<0>::kCoefOffset + K<0>::kCoefBytes, 3, &prepare, &launch, false, TMA};
+    e.launch_prims = &launch_prims;
+    return e;
   }
 };
 

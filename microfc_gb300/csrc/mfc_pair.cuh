@@ -112,10 +112,13 @@ __device__ __forceinline__ unsigned char* pair_staging(unsigned char* smem_raw) 
 // conservative values: half the bytes of a tile, no conversion of its halo
 // (448 cells for 256), and interior tiles arrive in their final layout by one
 // bulk copy.  The conversion is the same, so the bits are too.
+// 3-D (mfc_pair_sweep.cuh): pair k of cell o at k * sv + o; cur: in, or where
+// the x sweep puts the pairs of a state that comes without.
 struct PrimPairs {
   const f32x2* in;
   f32x2* out;
   int64_t pitch, plane;
+  f32x2* cur;
 };
 __host__ __device__ inline int64_t prim_pitch(int nx) { return (nx + 2 + 15) / 16 * 16; }
 

@@ -50,25 +50,6 @@ __device__ __forceinline__ T narrow(double x) {
 __device__ __forceinline__ double widen(double x) { return x; }
 __device__ __forceinline__ double widen(float x) { return f2d_bits(x); }
 
-// Work distribution of a split WENO5 phase: NPOS positions (cells of the
-// tile's rows or columns) times S items (the variable pairs).  Each full
-// pass gives a thread one position with all S items, so that the position's
-// index arithmetic, gate flag and coefficient record serve S
-// reconstructions; the NPOS % NT positions left over are dealt out per
-// (position, item), so that no thread does more than ceil(S * NPOS / NT).
-// f(p, v, all): position p, all items when all, else item v.
-template <int NPOS, int S, int NT, class F>
-__device__ __forceinline__ void deal_positions(const int tid, F&& f) {
-  constexpr int FULL = (NPOS / NT) * NT, REM = NPOS - FULL;
-  for (int p = tid; p < FULL; p += NT) f(p, 0, true);
-  if constexpr (REM > 0) {
-    for (int it = tid; it < REM * S; it += NT) {
-      const int v = it / REM;
-      f(FULL + (it - v * REM), v, false);
-    }
-  }
-}
-
 template <int ND, int NF, int WO, class RT, int TX, int TY, bool VISC = false>
 struct StageShape {
   using Q = Eqs<ND, NF>;

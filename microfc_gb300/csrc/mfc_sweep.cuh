@@ -19,13 +19,15 @@
 // work buffer's second segment, [S][z][y][x] in the reconstruction type),
 // and the y and z sweeps read them instead of converting the state again:
 // the conversion's FP64 operations (E - Pi, and the divisions of the plain
-// path) run once per cell and stage instead of three times, and the split
-// path's y and z sweeps load 4-byte instead of 8-byte values.  The stored
+// path) run once per cell and stage instead of three times.  The stored
 // values are the bits the conversion gives, and a reflected ghost cell's
 // normal velocity is the stored one negated, which is what converting the
 // reflected momentum gives (the conversion is odd in the momentum), so the
 // result is unchanged bit for bit.  Ghost cells of processor boundaries come
 // from the halo buffers as conservative values and are converted as before.
+//
+// Compiled for plain FP64 (TMA tiles, characteristic fields) and split WENO1/3;
+// split WENO5 runs on pairs (mfc_pair_sweep.cuh).
 #pragma once
 
 #include "mfc_device.cuh"
@@ -43,11 +45,9 @@ struct SweepShape {
   static constexpr int NQ = S * NP * LA;      // primitive tile [S][pencil][LA]
   static constexpr int NW = S * NP * (TA + 2);
   static constexpr int NFL = (S + 1) * NP * (TA + 1);
-  // split precision: FP32 coefficient records of kCoefRec floats per cell (float4 loads)
-  static constexpr int NCOEF = (sizeof(RT) == 4 && WO == 5) ? kCoefRec * (TA + 2) : 0;
   static constexpr int align16(int n) { return (n * int(sizeof(RT)) + 15) / 16 * 16 / int(sizeof(RT)); }
   static constexpr int OC = align16(NQ + 2 * NW + NFL);
-  static constexpr size_t kSmemBytes = sizeof(RT) * (size_t(OC) + size_t(NCOEF));
+  static constexpr size_t kSmemBytes = sizeof(RT) * size_t(OC);
   // TMA staging box of the tile (x, y, z extents; all S variables), in the
   // WENO and flux arrays: DIR 0 starts x on an even cell
   static constexpr int BX = DIR == 0 ? TmaBox<TA, H>::kWidth : TB;
@@ -78,7 +78,7 @@ __device__ __forceinline__ void sweep_coords(int a, int b, int c, int& x, int& y
 // CHAR: WENO of the characteristic fields (char_weno_position, FP64).
 template <int NF, int WO, class RT, int DIR, int TA, int TB, int TC, int NT, bool TMA = false, int MINB = 0,
           bool CHAR = false>
-__global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, const __grid_constant__ UniformCoef U,
+__global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P,
                                                    const __grid_constant__ TileMap T, const double* __restrict__ qin,
                                                    const double* __restrict__ qbase, double* __restrict__ qout,
                                                    const double dt, const int kind) {
@@ -102,18 +102,8 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
   RT* wl = sq + Sh::NQ;
   RT* wr = wl + Sh::NW;
   RT* fl = wr + Sh::NW;
-  RT* sc = sq + Sh::OC;  // 16-byte aligned coefficient records
-  // split WENO5 keeps the variables in interleaved pairs (2p, 2p+1) of the
-  // primitive tile and the WENO values, reconstructed two at a time with
-  // packed FP32 instructions (sys_size is even in 3-D)
-  constexpr bool kPair = Sh::NCOEF > 0;
-  static_assert(!kPair || (S % 2 == 0 && DIR == 0), "pairs: an even number of variables, the x sweep (y and z: mfc_pair_sweep.cuh)");
-  auto qi = [](int v, int p, int la) {
-    return kPair ? (((v >> 1) * NP + p) * LA + la) * 2 + (v & 1) : (v * NP + p) * LA + la;
-  };
-  auto wi = [](int v, int p, int ca) {
-    return kPair ? (((v >> 1) * NP + p) * (TA + 2) + ca) * 2 + (v & 1) : (v * NP + p) * (TA + 2) + ca;
-  };
+  auto qi = [](int v, int p, int la) { return (v * NP + p) * LA + la; };
+  auto wi = [](int v, int p, int ca) { return (v * NP + p) * (TA + 2) + ca; };
 
   const int tid = threadIdx.x;
   // block origin: blockIdx.x tiles the fastest non-sweep axis for DIR != 0
@@ -136,23 +126,9 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
   N eps;
   if constexpr (kSplit) eps = P.weno_eps_f;
   else eps = num(P.weno_eps);
-  // split WENO5 on a uniform grid: one coefficient record for the whole sweep
-  const bool ua = Sh::NCOEF > 0 && U.on[DIR];
-  (void)ua;
   const int64_t st[3] = {1, P.sy, P.sz};
 
   // ---- load + BCs + cons -> prim ------------------------------------------------
-  // the tile's coefficient records come from constant tables: staged before
-  // the wait for the previous kernel
-  if constexpr (Sh::NCOEF > 0) {
-    for (int it = ua ? kCoefRec * (TA + 2) : tid; it < kCoefRec * (TA + 2); it += NT) {
-      const int ca = it % (TA + 2), k = it / (TA + 2);
-      sc[ca * kCoefRec + k] =
-          k < kNumCoef
-              ? d2f_bits(__ldg(P.coef[DIR] + k * P.cstride[DIR] + clamp_coef_index(a0 - 1 + ca, na) + P.coff))
-              : 0.f;
-    }
-  }
   // the primitives of the stage input: written by the x sweep for the cells
   // it owns, read by the y and z sweeps
   RT* const gprim = reinterpret_cast<RT*>(P.work) + int64_t(S) * P.sv;
@@ -171,14 +147,8 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
 #pragma unroll
     for (int v = 0; v < S; ++v) sq[qi(v, p, la)] = pr[v];
     if (DIR == 0 && own >= 0) {
-      if constexpr (kPair) {  // as pairs, like the partial RHS
-        f32x2* const g = reinterpret_cast<f32x2*>(gprim) + own;
 #pragma unroll
-        for (int k = 0; k < S / 2; ++k) g[k * P.sv] = f2_pack(pr[2 * k], pr[2 * k + 1]);
-      } else {
-#pragma unroll
-        for (int v = 0; v < S; ++v) gprim[own + v * P.sv] = pr[v];
-      }
+      for (int v = 0; v < S; ++v) gprim[own + v * P.sv] = pr[v];
     }
   };
   // x sweep: the offset of tile cell (la, pb, pc) when the block owns it
@@ -330,47 +300,7 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
     wl[wi(v, p, ca)] = low(vl);
     wr[wi(v, p, ca)] = low(vr);
   };
-  if constexpr (kPair) {
-    constexpr int NPR = S / 2;
-    const f32x2 eps2 = f2_pack(eps, eps);
-    // variable pair pr of cell ca of pencil p; C(k): coefficient k as a (c, c) pair
-    auto pair = [&](const auto& C, const int ca, const int p, const int pr) {
-      const f32x2* line = reinterpret_cast<const f32x2*>(sq) + (pr * NP + p) * LA + ca + H - 1;
-      f32x2 stc[5];
-#pragma unroll
-      for (int k = 0; k < 5; ++k) stc[k] = line[k - 2];
-      f32x2 vl, vr;
-      weno5_pair_fast(C, stc, eps2, vl, vr);
-      reinterpret_cast<f32x2*>(wl)[(pr * NP + p) * NCA + ca] = vl;
-      reinterpret_cast<f32x2*>(wr)[(pr * NP + p) * NCA + ca] = vr;
-    };
-    // UNI: the shared record of a uniform grid, else the cell's staged
-    // record; chosen once per block
-    auto positions = [&](auto uni) {
-      constexpr bool UNI = decltype(uni)::value;
-      deal_positions<NP * NCA, NPR, NT>(tid, [&](const int q, const int v, const bool all) {
-        const int ca = q % NCA, p = q / NCA;
-        auto one = [&](const int w) {
-          if constexpr (UNI) {
-            const f32x2* rec = U.rec[DIR];
-            pair([&](int k) { return rec[k]; }, ca, p, w);
-          } else {
-            RT c[kCoefRec];
-            load_coef_record(sc + ca * kCoefRec, c);
-            pair([&](int k) { return f2_pack(c[k], c[k]); }, ca, p, w);
-          }
-        };
-        if (all) {
-#pragma unroll 1
-          for (int w = 0; w < NPR; ++w) one(w);
-        } else {
-          one(v);
-        }
-      });
-    };
-    if (ua) positions(FlagC<true>{});
-    else positions(FlagC<false>{});
-  } else if constexpr (CHAR) {
+  if constexpr (CHAR) {
     static_assert(sizeof(RT) == 8 && WO > 1, "characteristic-field WENO is compiled for FP64 WENO3/5");
     // one thread per position, all variables
     for (int it = tid; it < NP * NCA; it += NT) {
@@ -456,11 +386,7 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P, cons
         const N a = num(sq[qi(Q::ADV + f, p, ta + H)]);
         r[Q::ADV + f] = mul_add(inv * a, du, r[Q::ADV + f]);
       }
-      if constexpr (kPair) {
-        f32x2* const g = reinterpret_cast<f32x2*>(rhs_buf) + o;
-#pragma unroll
-        for (int k = 0; k < S / 2; ++k) g[k * P.sv] = f2_pack(r[2 * k], r[2 * k + 1]);
-      } else if constexpr (DIR < 2) {
+      if constexpr (DIR < 2) {
 #pragma unroll
         for (int v = 0; v < S; ++v) rhs_buf[o + v * P.sv] = low(r[v]);
       } else {
