@@ -337,7 +337,7 @@ int mfc_gate_infer(const float* X, int n, const float* w, void* wh_scratch, floa
 /* ---- Ensemble mode (no reference counterpart; the reference runs one case
  * per process).  Up to 96 independent 2-D cases that share num_fluids,
  * weno_order, precision, time_stepper (2 or 3) and device, each with its own
- * grid, boundary conditions, fluids and dt, advanced by one persistent
+ * grid, boundary conditions, fluids and dt, advanced by one
  * launch per RK stage over a work list of (case, tile) pairs. */
 typedef struct mfc_gpu_ensemble mfc_gpu_ensemble;
 

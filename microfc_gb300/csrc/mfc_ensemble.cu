@@ -1,6 +1,6 @@
 // C ABI of the ensemble mode (include/mfc_gpu.h, mfc_gpu_ensemble_*): many
-// independent 2-D cases of uneven grid size advanced by one persistent
-// launch per RK stage, optionally replayed from a CUDA graph, with the tile
+// independent 2-D cases of uneven grid size advanced by one launch per RK
+// stage, optionally replayed from a CUDA graph, with the tile
 // shape chosen by a project-written autotuner.
 #include <cuda_runtime.h>
 

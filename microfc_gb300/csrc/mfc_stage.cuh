@@ -238,8 +238,7 @@ __device__ __forceinline__ void char_weno_position(const double (&c)[kCoefRec], 
 }
 
 // One tile of one RK stage; the tile's first cell is (x0, y0).  Used by the
-// single-case kernel (one tile per block) and by the ensemble kernel (many
-// tiles of many cases per persistent block).  smem_raw must hold
+// single-case kernel and by the FP64 ensemble kernel.  smem_raw must hold
 // stage_smem_total().
 template <int ND, int NF, int WO, class RT, int TX, int TY, int NT, bool VISC = false, bool TMA = false,
           bool CHAR = false>

@@ -1,7 +1,7 @@
 """Ensemble mode: many independent 2-D cases advanced together.
 
 ``Ensemble(cases)`` uploads every case and advances all of them with one
-persistent launch per RK stage (C ABI ``mfc_gpu_ensemble_*``); ``run``
+launch per RK stage (C ABI ``mfc_gpu_ensemble_*``); ``run``
 replays the stage launches of a step from a CUDA graph; ``tune`` runs the
 project's autotuner over the compiled tile shapes.  Each case keeps its own
 grid, boundary conditions, fluids and dt, and gets the same bits it would
