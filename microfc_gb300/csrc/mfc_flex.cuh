@@ -25,7 +25,8 @@
 // 16x16 and in 1-D 128 cells): 100x100 632 -> 118, 301x101 634 -> 272,
 // 400x200 1225 -> 647, 1024x512 4293 -> 4008, 2048x1024 16552 -> 15761,
 // viscous 320x160 871 -> 526, 1-D 1000 cells 140 -> 42 (with hllc_face's
-// later form 263, 620, 3848, 522 and 38).  640 threads (96
+// later form 263, 620, 3848, 522 and 38, and in 1-D, with
+// flex_sides and flex_lane_pairs, 29.5).  640 threads (96
 // registers) against 512 (114): 4008 and 4093 at 1024x512; the viscous
 // kernel, whose faces need the registers, is faster with 512.
 #pragma once
@@ -54,6 +55,26 @@ struct FlexShape {
                              (size_t)ncoef(tx, ty));
   }
 };
+
+// The phases of small 1-D tiles, whose few warps are bound by their chains (64
+// cycles an operation) and not by the FP64 unit (16.5 a warp operation): a
+// reconstruction's two face values go to two items (53 operations each in
+// place of 72 for both) and a face's two states to two lanes (59 operations
+// deep in place of 85) where that is the shorter of the two bounds.  gi, ge:
+// groups of interior and of end positions, gs: groups of one side's values.
+// us a step without and with both: 300 cells 36.1 -> 28.8, 1000 38.1 -> 29.5,
+// 4000 44.0 -> 41.0; 20000, which take neither, 103.4 and 104.1.
+template <int WO>
+__host__ __device__ inline bool flex_sides(int gi, int ge, int gs, int warps) {
+  constexpr float both = WO == 5 ? 72.f : 26.f, one = WO == 5 ? 53.f : 18.f;
+  const float u0 = (gi * both + 2 * ge * one) * 16.5f, u1 = both * 64.f * ((gi + 2 * ge + warps - 1) / warps);
+  const float s0 = 2 * gs * one * 16.5f, s1 = one * 64.f * ((2 * gs + warps - 1) / warps);
+  return WO > 1 && (s0 > s1 ? s0 : s1) < (u0 > u1 ? u0 : u1);
+}
+__host__ __device__ inline bool flex_lane_pairs(int faces, int warps) {
+  const int g = (2 * faces + 31) / 32;
+  return g <= 4 && g <= warps;
+}
 
 template <int ND, int NF, int WO, int NT, bool VISC>
 __global__ void __launch_bounds__(NT) flex_kernel(const DevParams P, const double* __restrict__ qin,
@@ -149,7 +170,31 @@ __global__ void __launch_bounds__(NT) flex_kernel(const DevParams P, const doubl
     const int nex = S * th, gex = (nex + 31) >> 5;
     const int ney = ND > 1 ? S * tw : 0, gey = (ney + 31) >> 5;
     const int gint = ND * gi, groups = gint + 2 * gex + 2 * gey;
-    for (int g = warp; g < groups; g += NW) {
+    const int ns = S * (tw + 1), gs1 = (ns + 31) >> 5;
+    const bool sides = ND == 1 && flex_sides<WO>(gi, gex, gs1, NW);
+    // small 1-D tiles: every face value an item of its own, the right values
+    // of cells -1 .. tw-1, then the left ones of cells 0 .. tw
+    for (int g = sides ? warp : 2 * gs1; g < 2 * gs1; g += NW) {
+      const bool left = g >= gs1;
+      const int it = (left ? g - gs1 : g) * 32 + lane;
+      if (it >= ns) continue;
+      const int v = it / (tw + 1), c0 = it - v * (tw + 1), col = left ? c0 : c0 - 1;
+      const double* at = sq + v * LXY + col + H;
+      N s[5];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) s[k] = num(k - 2 >= -(WO / 2) && k - 2 <= WO / 2 ? at[k - 2] : 0.0);
+      // one code for both sides: the side's coefficients in the left's places
+      double c[kCoefRec];
+      if constexpr (WO > 1) {
+#pragma unroll
+        for (int k = 0; k < kNumCoef; ++k) {
+          const int from = left ? k : k >= kPL && k < kPL + 6 ? k + (kPR - kPL) : k >= kDL && k < kDL + 3 ? k + (kDR - kDL) : k;
+          c[k] = cx[from * NCX + col + 1];
+        }
+      }
+      (left ? wxl : wxr)[wxi(v, 0, col + 1)] = low(weno_cell_side<WO, 0, N>(NumCoef<N>{c, u0}, s, eps));
+    }
+    for (int g = sides ? groups : warp; g < groups; g += NW) {
       if (g < gint) {
         const bool ydir = ND > 1 && g >= gi;
         const int it = (ydir ? g - gi : g) * 32 + lane;
@@ -223,7 +268,37 @@ __global__ void __launch_bounds__(NT) flex_kernel(const DevParams P, const doubl
     const int nfx = (tw + 1) * th, gx = (nfx + 31) >> 5;
     const int nfy = ND > 1 ? tw * (th + 1) : 0, gy = (nfy + 31) >> 5;
     auto U = [&](int c, int x, int y) { return num(sq[(Q::MOM + c) * LXY + y * LX + x]); };
-    for (int g = warp; g < gx + gy; g += NW) {
+    // few faces in 1-D: two lanes to a face, each with one of its states until
+    // they meet
+    const bool pairs = ND == 1 && !VISC && flex_lane_pairs(nfx, NW);
+    if constexpr (ND == 1 && !VISC) {
+      for (int g = warp; pairs && g < (2 * nfx + 31) >> 5; g += NW) {
+        const int f0 = g * 16 + (lane >> 1), f = min(f0, tw);  // every lane of the warp takes part
+        const bool mine = (lane & 1) != 0;                     // the right state
+        const int gface = x0 - 1 + f;
+        const bool lfr = gface == -1 && P.bc_beg[0] == -4, rfl = gface == nx - 1 && P.bc_end[0] == -4;
+        N qL[S], qR[S], q[S], F[S], us;
+#pragma unroll
+        for (int v = 0; v < S; ++v) {
+          const N a = num(wxr[wxi(v, 0, f)]), b = num(wxl[wxi(v, 0, f + 1)]);
+          qL[v] = lfr ? b : a;
+          qR[v] = rfl ? a : b;
+          q[v] = mine ? qR[v] : qL[v];
+        }
+        const HllcSide<N> own = hllc_side<ND, NF, N>(q, gam_i, pi_i);
+        const HllcSide<N> other{num(__shfl_xor_sync(0xffffffffu, low(own.rho), 1)),
+                                num(__shfl_xor_sync(0xffffffffu, low(own.E), 1)),
+                                num(__shfl_xor_sync(0xffffffffu, low(own.c), 1))};
+        hllc_solve<ND, NF, 0, N>(qL, qR, mine ? other : own, mine ? own : other, F, us);
+        __syncwarp();  // the face's states are read by both lanes
+        if (f0 <= tw && !mine) {
+#pragma unroll
+          for (int v = 0; v < S; ++v) fxv(v, 0, f) = low(F[v]);
+          fxv(S, 0, f) = low(us);
+        }
+      }
+    }
+    for (int g = pairs ? gx + gy : warp; g < gx + gy; g += NW) {
       N qL[S], qR[S], F[S], us;
       if (g < gx) {
         const int it = g * 32 + lane;

@@ -271,8 +271,13 @@ Plan plan(int nx, int ny) {
       const int gi = groups(S * x * y), ge = groups(S * y) + (ND > 1 ? groups(S * x) : 0);
       const int gf = groups((x + 1) * y) + (ND > 1 ? groups(x * (y + 1)) : 0);
       const int gl = groups(x * y + 2 * H * (y + (ND > 1 ? x : 0)));
-      return phase(gl * prim, gl, prim, NW) + phase(ND * gi * both + 2 * ge * one, ND * gi + 2 * ge, both, NW) +
-             phase(gf * face, gf, face, NW) + phase(gi * cell, gi, cell, NW) + kTile;
+      double weno = phase(ND * gi * both + 2 * ge * one, ND * gi + 2 * ge, both, NW), hllc = phase(gf * face, gf, face, NW);
+      if (ND == 1) {
+        const int gs = groups(S * (x + 1)), gp = groups(2 * (x + 1));
+        if (flex_sides<WO>(gi, ge, gs, NW)) weno = phase(2 * gs * one, 2 * gs, one, NW);
+        if (!VISC && flex_lane_pairs(x + 1, NW)) hllc = phase(gp * 59.0, gp, 59.0, NW);
+      }
+      return phase(gl * prim, gl, prim, NW) + weno + hllc + phase(gi * cell, gi, cell, NW) + kTile;
     };
     return search(nx, ny, 1, ND > 1 ? 4 : 2, ND > 1 ? 96 : 512, ND > 1 ? 4 : 1, 96, cost,
                   [](int x, int y) { return Sh::bytes(x, y) <= kFlexSmemMax; });
