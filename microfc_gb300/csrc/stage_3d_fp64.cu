@@ -3,11 +3,41 @@
 
 namespace mfc {
 
+namespace {
+// Fixed tiles, TMA-staged: ahead of the sized ones where whole tiles cover the
+// grid and there are many waves of them (us a step, sized and fixed: 160x96x96
+// 19025 and 17969, 128^3 26598 and 25466, 256^3 205498 and 201893; where they
+// do not, 97x80x71 7477 and 8677, 60^3 2760 and 3216).  Both give the same bits.
+using Fixed = Sweep3D<2, 5, double, 32, 4, 2, 16, 16, 320, true, 2, false, 2>;
+
+bool whole_tiles(const int* n) {
+  const int64_t tiles = (int64_t)(n[0] / 16) * (n[1] / 16) * n[2];  // of the y sweep, two on an SM
+  return n[0] % 32 == 0 && n[1] % 16 == 0 && n[2] % 16 == 0 && tiles >= 16 * 2 * flex::kSMs;
+}
+
+StageEntry sized_or_fixed() {
+  StageEntry e = flex_sweep_entry<2, 5, 640>();
+  e.prepare = [] {
+    const cudaError_t r = flex_sweep_entry<2, 5, 640>().prepare();
+    return r == cudaSuccess ? Fixed::prepare() : r;
+  };
+  e.launch = [](const DevParams& P, const UniformCoef& U, const double* qin, const double* qbase, double* qout,
+                double dt, int kind, cudaStream_t st) {
+    return (whole_tiles(P.n) ? &Fixed::launch : flex_sweep_entry<2, 5, 640>().launch)(P, U, qin, qbase, qout, dt, kind,
+                                                                                   st);
+  };
+  e.tile = [](const int* n, int* tx, int* ty, int* nt) {
+    const StageEntry f = Fixed::entry();
+    if (whole_tiles(n)) *tx = f.tx, *ty = f.ty, *nt = f.nt;
+    else flex_sweep_entry<2, 5, 640>().tile(n, tx, ty, nt);
+  };
+  return e;
+}
+}  // namespace
+
 void register_stage_3d_fp64(std::vector<StageEntry>& r) {
-  r.push_back(flex_sweep_entry<2, 5, 640>());
-  // fixed tiles, TMA-staged: even with the sized ones where the grid is a
-  // multiple of both tiles (26.05 and 26.01 ms a step at 128^3), slower elsewhere
-  r.push_back(Sweep3D<2, 5, double, 32, 4, 2, 16, 16, 320, true, 2, false, 2>::entry());
+  r.push_back(sized_or_fixed());
+  r.push_back(Fixed::entry());
   r.push_back(flex_sweep_entry<1, 5, 640>());
   r.push_back(flex_sweep_entry<2, 3, 512>());
   r.push_back(flex_sweep_entry<2, 1, 512>());
