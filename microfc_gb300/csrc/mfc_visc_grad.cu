@@ -248,8 +248,8 @@ __global__ void __launch_bounds__(256) visc_face_gradients_y(const DevParams P, 
 // with a halo of 5, both cell gradients with a halo of 3 and the face values
 // live in shared memory, both components are reconstructed by packed FP32
 // operations that round as weno_cell's do, and a uniform grid's coefficients
-// come from the parameters.  Measured at 1024x512: 130 -> 48 us a stage with
-// the velocities; a split weno_Re_flux step 604 -> 338 us.  Bound by FP32 issue.
+// come from the parameters.  Measured at 1024x512: 130 -> 49 us a stage with
+// the velocities; a split weno_Re_flux step 604 -> 343 us.  Bound by FP32 issue.
 constexpr int kGX = 32, kGY = 16, kGT = 256;
 struct GradShape {
   static constexpr int UX = kGX + 9, UY = kGY + 9;    // velocities: x0-5 .. x0+kGX+3
@@ -267,8 +267,16 @@ struct GradShape {
 // instructions, and the reciprocal of b_k^2 serves both faces, that of the
 // sum all three weights.  A product that a sum takes is fma(a, b, nz) with
 // nz = -0 in a register: ptxas contracts packed multiplies and adds whatever
-// their rounding modifiers say.  b_k is scaled by 2^-4 first, which leaves the
-// weights as they are and their divisors inside the reciprocal's range.
+// their rounding modifiers say.
+//
+// The weights do not change when all b_k are scaled alike, so each lane's are
+// scaled by the power of two that brings its least b_k to [1, 2): b_k^2 of a
+// uniform velocity (weno_eps^2) stays a normal number for every weno_eps that
+// FP32 holds, and that of the smoothest stencil never overflows.  A stencil
+// 2^63 times rougher has no weight either way; its b_k is cut there, which
+// keeps the divisors inside the reciprocal's range (the Newton step of an
+// infinity or a zero is not a number).  The scale and the cut cost 1 % of a
+// step (340 -> 343 us at 1024x512) and change no bit of ordinary values.
 __device__ __forceinline__ f32x2 f2_neg(f32x2 a) { return a ^ 0x8000000080000000ull; }
 __device__ __forceinline__ f32x2 f2_reciprocal(f32x2 a) {
   const f32x2 r = f2_rcp(a);
@@ -278,18 +286,39 @@ __device__ __forceinline__ f32x2 f2_quotient(f32x2 n, f32x2 d, f32x2 r) {
   const f32x2 q = f2_mul(n, r);
   return f2_fma(f2_fma(f2_neg(d), q, n), r, q);
 }
+// 2^-e of each lane, e the exponent of the lane's least value.
+__device__ __forceinline__ f32x2 f2_scale_to_one(f32x2 a, f32x2 b, f32x2 c) {
+  float a0, a1, b0, b1, c0, c1;
+  f2_unpack(a, a0, a1);
+  f2_unpack(b, b0, b1);
+  f2_unpack(c, c0, c1);
+  auto inverse = [](float x) { return __uint_as_float(0x7f000000u - (__float_as_uint(x) & 0x7f800000u)); };
+  return f2_pack(inverse(fminf(fminf(a0, b0), c0)), inverse(fminf(fminf(a1, b1), c1)));
+}
+// The smaller of each lane and 2^63; NaN stays NaN.
+__device__ __forceinline__ f32x2 f2_cut(f32x2 a) {
+  float x, y;
+  f2_unpack(a, x, y);
+  asm("min.NaN.f32 %0, %0, 0f5F000000;" : "+f"(x));
+  asm("min.NaN.f32 %0, %0, 0f5F000000;" : "+f"(y));
+  return f2_pack(x, y);
+}
 template <class Coef>
 __device__ __forceinline__ void grad_weno(const Coef& C, const f32x2 (&v)[5], const f32x2 eps, const f32x2 nz,
                                           f32x2& vL, f32x2& vR) {
   const f32x2 d1 = f2_sub(v[4], v[3]), d0 = f2_sub(v[3], v[2]), dm1 = f2_sub(v[2], v[1]), dm2 = f2_sub(v[1], v[0]);
-  const f32x2 scale = f2_pack(0.0625f, 0.0625f);
-  auto indicator = [&](const int k, const f32x2 a, const f32x2 b) {  // (b_k 2^-4)^2
+  auto indicator = [&](const int k, const f32x2 a, const f32x2 b) {  // b_k
     const f32x2 t0 = f2_fma(f2_mul(C(kBeta + 3 * k), a), a, nz), t1 = f2_fma(f2_mul(C(kBeta + 3 * k + 1), a), b, nz),
                 t2 = f2_fma(f2_mul(C(kBeta + 3 * k + 2), b), b, nz);
-    const f32x2 s = f2_mul(f2_add(f2_add(f2_add(t0, t1), t2), eps), scale);
-    return f2_mul(s, s);
+    return f2_add(f2_add(f2_add(t0, t1), t2), eps);
   };
-  const f32x2 D0 = indicator(0, d1, d0), D1 = indicator(1, d0, dm1), D2 = indicator(2, dm1, dm2);
+  const f32x2 b0 = indicator(0, d1, d0), b1 = indicator(1, d0, dm1), b2 = indicator(2, dm1, dm2);
+  const f32x2 scale = f2_scale_to_one(b0, b1, b2);
+  auto square = [&](const f32x2 b) {
+    const f32x2 t = f2_cut(f2_mul(b, scale));
+    return f2_mul(t, t);
+  };
+  const f32x2 D0 = square(b0), D1 = square(b1), D2 = square(b2);
   const f32x2 r0 = f2_reciprocal(D0), r1 = f2_reciprocal(D1), r2 = f2_reciprocal(D2);
 #pragma unroll
   for (int side = 0; side < 2; ++side) {
