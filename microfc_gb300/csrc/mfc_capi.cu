@@ -173,6 +173,7 @@ struct mfc_gpu_ctx {
   mfc::f32x2* prim[2] = {nullptr, nullptr};
   int prim_at = 0;
   const double* prim_of = nullptr;
+  bool captured = false;  // a graph holds launches of this context: its replays change registers and pairs unseen
   unsigned long long* monitor = nullptr;  // max ICFL of the monitored steps (double bits)
   bool monitor_on = false;
   double* tables = nullptr;     // inv_d and coefficient tables
@@ -253,8 +254,9 @@ int validate(const mfc_params* p) {
   return why.empty() ? MFC_OK : fail(MFC_ERR_INVALID, why);
 }
 
+// follows: qin is what this call's previous launch made
 int launch_stage(mfc_gpu_ctx* c, const double* qin, const double* qbase, double* qout, double dt, int kind,
-                 bool last_stage = false) {
+                 bool last_stage = false, bool follows = false) {
   mfc::DevParams P = c->dev;
   if (last_stage && c->monitor_on) P.monitor = c->monitor;  // ICFL of the step's new state
   if (c->wrf && c->visc) {  // weno_Re_flux = T: the stage input's face gradients first
@@ -267,9 +269,13 @@ int launch_stage(mfc_gpu_ctx* c, const double* qin, const double* qbase, double*
   if (c->prim[0] != nullptr && c->stage->launch_prims != nullptr) {
     const bool keep = kind != mfc::kRhsOnly;  // an RHS evaluation makes no state
     const int64_t pitch = mfc::prim_pitch(c->n[0]);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    e = cudaStreamIsCapturing(c->stream, &capture);
+    if (e != cudaSuccess) return fail(MFC_ERR_CUDA, std::string("stage launch: ") + cudaGetErrorString(e));
+    c->captured |= capture != cudaStreamCaptureStatusNone;
     // 3-D stages always have the pairs of their input somewhere: an RHS
     // evaluation's go where they spare the last stage's
-    const bool have = c->prim_of == qin;
+    const bool have = c->prim_of == qin && (follows || !c->captured);
     const mfc::PrimPairs B{have ? c->prim[c->prim_at] : nullptr, keep ? c->prim[c->prim_at ^ 1] : nullptr, pitch,
                            pitch * c->n[1], c->prim[have || keep ? c->prim_at : c->prim_at ^ 1]};
     e = c->stage->launch_prims(P, c->ucoef, qin, qbase, qout, dt, kind, B, c->stream);
@@ -665,11 +671,11 @@ int mfc_gpu_tvd_rk(mfc_gpu_ctx* c, double dt, int last_step) {
       return MFC_OK;
     case 2:
       if ((rc = launch_stage(c, R[0], R[0], R[1], dt, mfc::kRkEuler))) return rc;
-      return launch_stage(c, R[1], R[0], R[0], dt, mfc::kRk2Final, true);
+      return launch_stage(c, R[1], R[0], R[0], dt, mfc::kRk2Final, true, true);
     default:
       if ((rc = launch_stage(c, R[0], R[0], R[1], dt, mfc::kRkEuler))) return rc;
-      if ((rc = launch_stage(c, R[1], R[0], R[2], dt, mfc::kRk3Mid))) return rc;
-      return launch_stage(c, R[2], R[0], R[0], dt, mfc::kRk3Final, true);
+      if ((rc = launch_stage(c, R[1], R[0], R[2], dt, mfc::kRk3Mid, false, true))) return rc;
+      return launch_stage(c, R[2], R[0], R[0], dt, mfc::kRk3Final, true, true);
   }
 }
 
