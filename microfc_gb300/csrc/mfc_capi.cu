@@ -167,9 +167,9 @@ struct mfc_gpu_ctx {
   void* gate_w = nullptr;       // MFC_PREC_GATED: FP16 gate parameters
   uint8_t* gate_flags = nullptr;  // MFC_PREC_GATED: a step's first-stage gate decisions
   bool gate_ready = false;
-  // split and gated 2-D and split 3-D WENO5: the primitive pairs of the last stage's output
-  // (prim[prim_at]; of register prim_of, or of none), and the buffer that the
-  // next stage writes them to
+  // split and gated 2-D (null where there was no room) and split 3-D WENO5:
+  // the primitive pairs of the last stage's output (prim[prim_at]; of register
+  // prim_of, or of none), and the buffer that the next stage writes them to
   mfc::f32x2* prim[2] = {nullptr, nullptr};
   int prim_at = 0;
   const double* prim_of = nullptr;
@@ -252,6 +252,23 @@ namespace {
 int validate(const mfc_params* p) {
   const std::string why = mfc::validate_params(p, /*allow_processor=*/true);
   return why.empty() ? MFC_OK : fail(MFC_ERR_INVALID, why);
+}
+
+// cudaMalloc for the buffers that come after mfc_gpu_init: where it finds no
+// room, a 2-D context gives its primitive pairs back first (not those that a
+// captured graph points to).
+template <class T>
+cudaError_t ctx_malloc(mfc_gpu_ctx* c, T** ptr, size_t bytes) {
+  cudaError_t e = cudaMalloc(ptr, bytes);
+  if (e == cudaErrorMemoryAllocation && c->nd == 2 && c->prim[0] != nullptr && !c->captured) {
+    (void)cudaGetLastError();
+    if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return e;
+    cudaFree(c->prim[0]);
+    c->prim[0] = c->prim[1] = nullptr;
+    c->prim_of = nullptr;
+    e = cudaMalloc(ptr, bytes);
+  }
+  return e;
 }
 
 // follows: qin is what this call's previous launch made
@@ -442,16 +459,6 @@ int mfc_gpu_init(const mfc_params* p, mfc_gpu_ctx** out) {
   if (p->precision == MFC_PREC_GATED &&
       (e = cudaMalloc(&c->gate_flags, mfc::gate_flag_bytes(c->n[0], c->n[1]))) != cudaSuccess)
     return cleanup(fail(MFC_ERR_NOMEM, cudaGetErrorString(e)));
-  // 2-D split and gated: two buffers of primitive pairs, the next stage's
-  // input and output (not with processor boundaries, whose ghost cells come
-  // as conservative values)
-  if (c->nd == 2 && p->weno_order == 5 && (p->precision == MFC_PREC_SPLIT || p->precision == MFC_PREC_GATED) &&
-      p->bc_x_beg < 0 && p->bc_x_end < 0 && p->bc_y_beg < 0 && p->bc_y_end < 0) {
-    const size_t bytes = sizeof(mfc::f32x2) * (size_t)((c->S + 1) / 2) * c->n[1] * mfc::prim_pitch(c->n[0]);
-    for (int k = 0; k < 2; ++k)
-      if ((e = cudaMalloc(&c->prim[k], bytes)) != cudaSuccess)
-        return cleanup(fail(MFC_ERR_NOMEM, cudaGetErrorString(e)));
-  }
   // 3-D: the partial RHS, then the primitives the x sweep stores (S x sv
   // values each, in the reconstruction type: FP64 at most); split WENO5: three
   // quarters of it, for the partial RHS and two buffers of primitive pairs
@@ -531,6 +538,18 @@ int mfc_gpu_init(const mfc_params* p, mfc_gpu_ctx** out) {
   D.work = c->work;  // shares its slot with gate_flags: set the one in use
   if (c->gate_flags) D.gate_flags = c->gate_flags;
   D.gate_w = c->gate_w;
+
+  // 2-D split and gated: two buffers of primitive pairs, the next stage's
+  // input and output (not with processor boundaries, whose ghost cells come
+  // as conservative values).  The last allocation, and not a needed one: a
+  // state that leaves no room for them runs without (ctx_malloc gives them
+  // back to a later allocation that needs the room).
+  if (c->nd == 2 && p->weno_order == 5 && (p->precision == MFC_PREC_SPLIT || p->precision == MFC_PREC_GATED) &&
+      !c->has_proc) {
+    const size_t pairs = (size_t)((c->S + 1) / 2) * c->n[1] * mfc::prim_pitch(c->n[0]);
+    if (cudaMalloc(&c->prim[0], 2 * sizeof(mfc::f32x2) * pairs) == cudaSuccess) c->prim[1] = c->prim[0] + pairs;
+    else (void)cudaGetLastError();
+  }
 
   if ((e = c->stage->prepare()) != cudaSuccess) return cleanup(fail(MFC_ERR_CUDA, cudaGetErrorString(e)));
   if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return cleanup(fail(MFC_ERR_CUDA, cudaGetErrorString(e)));
@@ -775,7 +794,7 @@ int mfc_gpu_set_viscosity(mfc_gpu_ctx* c, const double* re_shear, const double* 
     V.fg[0] = c->vg.fg[0];
     V.fg[1] = c->vg.fg[1];
   }
-  if (!c->visc && cudaMalloc(&c->visc, sizeof(mfc::ViscParams)) != cudaSuccess)
+  if (!c->visc && ctx_malloc(c, &c->visc, sizeof(mfc::ViscParams)) != cudaSuccess)
     return fail(MFC_ERR_NOMEM, "viscous parameters");
   MFC_CUDA(cudaMemcpy(c->visc, &V, sizeof(V), cudaMemcpyHostToDevice));
   if (e->prepare() != cudaSuccess) return fail(MFC_ERR_CUDA, "viscous kernel does not fit on this device");
@@ -844,7 +863,7 @@ int mfc_gpu_set_viscous_gradients(mfc_gpu_ctx* c, int weno_re_flux) {
   }
   cudaError_t e = cudaSuccess;
   auto alloc = [&](double** ptr, size_t count) {
-    if (e == cudaSuccess) e = cudaMalloc(ptr, sizeof(double) * count);
+    if (e == cudaSuccess) e = ctx_malloc(c, ptr, sizeof(double) * count);
   };
   alloc(&c->vg.vel, (size_t)nd * (nd > 1 ? ny + 10 : 1) * (nx + 10));
   alloc(&c->vg.g, (size_t)k * (nd > 1 ? ny + 6 : 1) * (nx + 6));
@@ -864,7 +883,7 @@ int mfc_gpu_set_viscous_gradients(mfc_gpu_ctx* c, int weno_re_flux) {
       for (size_t j = 0; j < stride; ++j)
         cf[d][kk * stride + j] = (float)gt.host[gt.off_coef[d] + (size_t)kk * gt.cstride[d] + j];
     for (size_t j = 0; j < stride; ++j) cf[d][mfc::kNumCoef * stride + j] = (float)(1.0 / w[d][j]);
-    if (e == cudaSuccess) e = cudaMalloc(&c->vg.cf[d], sizeof(float) * cf[d].size());
+    if (e == cudaSuccess) e = ctx_malloc(c, &c->vg.cf[d], sizeof(float) * cf[d].size());
   }
   if (e != cudaSuccess) {
     free_visc_gradients(c);
@@ -1127,7 +1146,7 @@ int mfc_gpu_snapshot(mfc_gpu_ctx* c, int slot) {
     MFC_CUDA(cudaEventCreateWithFlags(&c->snap_staged, cudaEventDisableTiming));
   }
   if (!c->snap_host[slot]) {
-    if (cudaMalloc(&c->snap_dev[slot], bytes) != cudaSuccess) return fail(MFC_ERR_NOMEM, "snapshot staging buffer");
+    if (ctx_malloc(c, &c->snap_dev[slot], bytes) != cudaSuccess) return fail(MFC_ERR_NOMEM, "snapshot staging buffer");
     if (cudaMallocHost(&c->snap_host[slot], bytes) != cudaSuccess) return fail(MFC_ERR_NOMEM, "pinned snapshot slot");
     MFC_CUDA(cudaEventCreateWithFlags(&c->snap_done[slot], cudaEventDisableTiming));
   }
@@ -1189,10 +1208,7 @@ int mfc_gpu_finalize(mfc_gpu_ctx* c) {
   cudaFree(c->tables);
   cudaFree(c->status);
   cudaFree(c->work);
-  if (c->nd < 3) {  // 3-D: parts of work
-    cudaFree(c->prim[0]);
-    cudaFree(c->prim[1]);
-  }
+  if (c->nd < 3) cudaFree(c->prim[0]);  // 3-D: part of work
   cudaFree(c->scratch);
   cudaFree(c->vg.vel);
   cudaFree(c->vg.g);

@@ -53,7 +53,7 @@ struct mfc_gpu_ensemble {
   std::vector<double> dt;
   double* state = nullptr;
   double* tables = nullptr;
-  mfc::f32x2* prim = nullptr;  // split and gated: every case's primitive pairs, two buffers each
+  mfc::f32x2* prim = nullptr;  // split and gated: every case's primitive pairs, two buffers each (null: no room)
   uint32_t* status = nullptr;
   void* gate_w = nullptr;  // MFC_PREC_GATED: FP16 gate parameters
   uint8_t* gate_flags = nullptr;  // MFC_PREC_GATED: every case's first-stage gate decisions
@@ -98,9 +98,11 @@ int configure(mfc_gpu_ensemble* e, const mfc::EnsembleEntry* en) {
     std::vector<mfc::TileMap> maps(3 * (size_t)e->num);
     for (int i = 0; i < e->num; ++i) {
       const mfc::EnsCase& C = e->cases[i];
-      mfc::encode_tile_map(maps[i], C.reg[0], e->nx[i], e->ny[i], 2 * e->nf + 3, C.P.sy, C.P.sv, en->box_w, en->box_h);
       const int64_t pitch = mfc::prim_pitch(e->nx[i]);
-      for (int k = 0; k < 2; ++k)
+      for (int r = 0; r < (e->prim ? 1 : 3); ++r)
+        mfc::encode_tile_map(maps[(size_t)r * e->num + i], C.reg[r], e->nx[i], e->ny[i], 2 * e->nf + 3, C.P.sy, C.P.sv,
+                             en->box_w, en->box_h);
+      for (int k = 0; k < 2 && e->prim; ++k)
         mfc::encode_tile_map(maps[(size_t)(k + 1) * e->num + i], reinterpret_cast<const double*>(C.prim[k]), (int)pitch,
                              e->ny[i], e->nf + 2, pitch, pitch * e->ny[i], en->tx + 6, en->ty + 6);
     }
@@ -240,8 +242,6 @@ int mfc_gpu_ensemble_init(const mfc_params* cases, const double* dts, int num_ca
       (err = cudaMalloc(&e->state, sizeof(double) * state_elems)) != cudaSuccess ||
       (err = cudaMalloc(&e->tables, sizeof(double) * table_elems)) != cudaSuccess ||
       (err = cudaMalloc(&e->status, sizeof(uint32_t))) != cudaSuccess ||
-      (c0.precision != MFC_PREC_FP64 &&
-       (err = cudaMalloc(&e->prim, sizeof(mfc::f32x2) * prim_elems)) != cudaSuccess) ||
       (err = cudaMalloc(&e->maps, sizeof(mfc::TileMap) * 3 * (size_t)num_cases)) != cudaSuccess ||
       (c0.precision == MFC_PREC_GATED && (err = cudaMalloc(&e->gate_w, mfc::kGateBufferBytes)) != cudaSuccess))
     return cleanup(mfc::report_error(MFC_ERR_NOMEM, cudaGetErrorString(err)));
@@ -249,6 +249,10 @@ int mfc_gpu_ensemble_init(const mfc_params* cases, const double* dts, int num_ca
   for (int i = 0; i < num_cases; ++i) flag_bytes += mfc::gate_flag_bytes(e->nx[i], e->ny[i]);
   if (c0.precision == MFC_PREC_GATED && (err = cudaMalloc(&e->gate_flags, flag_bytes)) != cudaSuccess)
     return cleanup(mfc::report_error(MFC_ERR_NOMEM, cudaGetErrorString(err)));
+  // the pairs come last and are not needed: where there is no room every stage
+  // converts the conservative state
+  if (c0.precision != MFC_PREC_FP64 && cudaMalloc(&e->prim, sizeof(mfc::f32x2) * prim_elems) != cudaSuccess)
+    (void)cudaGetLastError();
   size_t flag_off = 0;
   cudaMemsetAsync(e->state, 0, sizeof(double) * state_elems, e->stream);
   cudaMemsetAsync(e->status, 0, sizeof(uint32_t), e->stream);

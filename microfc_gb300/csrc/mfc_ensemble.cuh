@@ -22,7 +22,8 @@ struct EnsCase {
   DevParams P;
   double* reg[3];         // RK registers; reg[0] holds q_cons_ts(1)
   // split and gated: the primitive pairs (PrimPairs, mfc_pair.cuh) that the
-  // first and the second stage of a step write and the next one reads
+  // first and the second stage of a step write and the next one reads; null:
+  // there was no room for them
   f32x2* prim[2];
   double dt, dt_last;     // the case's dt and its (possibly trimmed) last-step dt
   int tiles_x, tile_base; // tiles per row, first tile in the work list
@@ -31,8 +32,8 @@ struct EnsCase {
 struct EnsParams {
   int num_cases, total_tiles, stage, time_stepper, last_step;
   // TMA maps of every case's stage inputs, [stage][case] (device memory; the
-  // first stage's conservative register, then the pairs), for the tile
-  // variant launched; null: plain loads
+  // first stage's conservative register, then the pairs or, without them, the
+  // other registers), for the tile variant launched; null: plain loads
   const TileMap* maps;
   // split WENO5: the coefficient record every cell of every case shares when
   // all cases have uniform grids (the FP32 records of a uniform grid do not
