@@ -865,16 +865,18 @@ int mfc_gpu_set_viscous_gradients(mfc_gpu_ctx* c, int weno_re_flux) {
   auto alloc = [&](double** ptr, size_t count) {
     if (e == cudaSuccess) e = ctx_malloc(c, ptr, sizeof(double) * count);
   };
-  alloc(&c->vg.vel, (size_t)nd * (nd > 1 ? ny + 10 : 1) * (nx + 10));
-  alloc(&c->vg.g, (size_t)k * (nd > 1 ? ny + 6 : 1) * (nx + 6));
-  alloc(&c->vg.fg[0], (size_t)k * ny * (nx + 1));
+  const bool fp32 = c->prm.precision == MFC_PREC_SPLIT || c->prm.precision == MFC_PREC_GATED;
+  // 2-D split and gated: pairs of the two components, no cell gradients
+  const int in8 = fp32 && nd == 2 ? 2 : 1;  // values in 8 bytes
+  alloc(&c->vg.vel, (size_t)nd / in8 * (nd > 1 ? ny + 10 : 1) * (nx + 10));
+  if (in8 == 1) alloc(&c->vg.g, (size_t)k * (nd > 1 ? ny + 6 : 1) * (nx + 6));
+  alloc(&c->vg.fg[0], (size_t)k / in8 * ny * (nx + 1));
   alloc(&c->vg.w[0], w[0].size());
   if (nd > 1) {
-    alloc(&c->vg.fg[1], (size_t)k * (ny + 1) * nx);
+    alloc(&c->vg.fg[1], (size_t)k / in8 * (ny + 1) * nx);
     alloc(&c->vg.w[1], w[1].size());
   }
   // split and gated: the reconstructions' FP32 table of each direction
-  const bool fp32 = c->prm.precision == MFC_PREC_SPLIT || c->prm.precision == MFC_PREC_GATED;
   std::vector<float> cf[2];
   for (int d = 0; fp32 && d < nd; ++d) {
     const size_t stride = w[d].size();  // cells -kCoefPad .. n-1+kCoefPad

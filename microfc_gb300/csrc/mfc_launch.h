@@ -527,7 +527,7 @@ cudaError_t ctx_scratch(mfc_gpu_ctx* c, size_t bytes, void** out);
 // precisions, an FP32 table per direction: the WENO coefficients of those
 // cells ([kNumCoef][n + 2 kCoefPad]) followed by their inverse widths.
 // In 2-D those precisions hold the velocities and the face gradients as FP32
-// pairs of the two components in the same buffers (fg[0]: [d][ny][nx + 1]).
+// pairs of the two components (fg[0]: [d][ny][nx + 1]), and no cell gradients.
 // uniform: their coefficients, then the inverse width, as (c, c) pairs, when
 // every cell of each direction has the same.
 struct GradCoef {

@@ -197,40 +197,36 @@ __global__ void __launch_bounds__(256) visc_face_gradients_x(const DevParams P, 
   }
 }
 
-// y faces: a thread walks one column through a run of R faces (cells
+// y faces (2-D, FP64): a thread walks one column through a run of R faces (cells
 // f0-1 .. f0+R-1), carrying each cell's right values to the next face.
-template <int ND, class RT, int R>
-__global__ void __launch_bounds__(256) visc_face_gradients_y(const DevParams P, const float* __restrict__ cft,
-                                                            const double* __restrict__ G, const int gib,
-                                                            const int gjb, const int gncol, const int gnrow,
-                                                            double* __restrict__ out) {
+template <int R>
+__global__ void __launch_bounds__(256) visc_face_gradients_y(const DevParams P, const double* __restrict__ G,
+                                                            const int gib, const int gjb, const int gncol,
+                                                            const int gnrow, double* __restrict__ out) {
   const int nx = P.n[0], ny = P.n[1], nf = ny + 1;
   const int runs = (nf + R - 1) / R;
   const int64_t items = (int64_t)nx * runs;
   const int64_t plane_out = (int64_t)nf * nx;
-  using N = std::conditional_t<sizeof(RT) == 8, Num64, RT>;
-  N u0;
-  if constexpr (sizeof(RT) == 8) u0 = num64_unit(P.inv_d[0]);
-  else u0 = RT(0);
-  const N eps = lift(narrow<RT>(P.weno_eps), u0);
+  using N = Num64;
+  const N u0 = num64_unit(P.inv_d[0]), eps = lift(P.weno_eps, u0);
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < items; t += (int64_t)gridDim.x * blockDim.x) {
     const int l = (int)(t % nx), f0 = (int)(t / nx) * R;
-    N prev[ND * ND];
+    N prev[4];
 #pragma unroll 1
     for (int j = -1; j < R; ++j) {
       const int cell = f0 + j;  // -1 .. ny
       if (cell > ny) break;
-      RT cf[kCoefRec];
-      coef_of(P, cft, 1, cell, cf);
+      double cf[kCoefRec];
+      coef_of(P, nullptr, 1, cell, cf);
       const double* col = G + (int64_t)(cell - gjb) * gncol + (l - gib);
 #pragma unroll
-      for (int k = 0; k < ND * ND; ++k) {
+      for (int k = 0; k < 4; ++k) {
         N st[5];
 #pragma unroll
-        for (int o = 0; o < 5; ++o) st[o] = lift(narrow<RT>(__ldg(col + ((int64_t)k * gnrow + (o - 2)) * gncol)), u0);
+        for (int o = 0; o < 5; ++o) st[o] = lift(__ldg(col + ((int64_t)k * gnrow + (o - 2)) * gncol), u0);
         N vl, vr;
         grad_cell(cf, st, eps, u0, vl, vr);
-        if (j >= 0) out[k * plane_out + (int64_t)cell * nx + l] = widen(low(lift(RT(0.5), u0) * (prev[k] + vl)));
+        if (j >= 0) out[k * plane_out + (int64_t)cell * nx + l] = low(lift(0.5, u0) * (prev[k] + vl));
         prev[k] = vr;
       }
     }
@@ -512,9 +508,10 @@ cudaError_t launch_all(const DevParams& P, const ViscGradBuffers& B, const doubl
   visc_face_gradients_x<ND, RT><<<grid(32 * xwarps), 256, 0, st>>>(P, B.cf[0], B.g, -3, gjb, gcol, grow, B.fg[0]);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if constexpr (ND > 1) {
+    static_assert(sizeof(RT) == 8, "2-D split and gated contexts take launch_tiled");
     constexpr int R = 8;  // faces per thread
-    visc_face_gradients_y<ND, RT, R><<<grid((int64_t)nx * ((ny + 1 + R - 1) / R)), 256, 0, st>>>(
-        P, B.cf[1], B.g, -3, gjb, gcol, grow, B.fg[1]);
+    visc_face_gradients_y<R><<<grid((int64_t)nx * ((ny + 1 + R - 1) / R)), 256, 0, st>>>(P, B.g, -3, gjb, gcol, grow,
+                                                                                        B.fg[1]);
     e = cudaGetLastError();
   }
   return e;

@@ -92,6 +92,16 @@ def test_pairs_give_way_to_the_gradient_buffers():
     assert np.array_equal(outs[0].view(np.uint64), outs[1].view(np.uint64))
 
 
+def test_gradient_buffers_hold_what_the_precision_stores():
+    """Split: velocity and two face-gradient pairs of each direction, 40 bytes a cell."""
+    from microfc_gb300 import Simulation
+    c, x, y, z, q = _case("split")
+    with Simulation(c.replace(re_shear=(10.0, 500.0)), x, y, z, q_cons=q) as sim:
+        before = _free()
+        sim.set_viscous_gradients(True)
+        assert before - _free() <= 40 * (NX + 10) * (NY + 10) + 16 * MB
+
+
 @pytest.mark.parametrize("stepper", [2, 3])
 def test_ensemble_runs_without_pairs(stepper):
     from microfc_gb300.ensemble import Ensemble
