@@ -101,8 +101,9 @@ int mfc_gpu_abi_version(void);
 const char* mfc_gpu_last_error(void);
 
 /* Allocates the device state (3 RK registers + rhs + grid tables; 3-D cases
- * also a work area of 2 registers for the directional sweeps) and uploads
- * the grid.  Replaces s_initialize_*_module. */
+ * also a work area of 2 registers for the directional sweeps; 2-D split and
+ * gated cases, where there is room, 64 bytes a cell of FP32 primitives) and
+ * uploads the grid.  Replaces s_initialize_*_module. */
 int mfc_gpu_init(const mfc_params* params, mfc_gpu_ctx** ctx_out);
 
 /* Number of equations (sys_size = 2*num_fluids + num_dims + 1). */
@@ -116,7 +117,9 @@ int mfc_gpu_sys_size(const mfc_gpu_ctx* ctx);
 int mfc_gpu_upload(mfc_gpu_ctx* ctx, int var, const double* host_sf, int64_t ld_y, int64_t ld_z);
 int mfc_gpu_download(mfc_gpu_ctx* ctx, int var, double* host_sf, int64_t ld_y, int64_t ld_z);
 
-/* Whole-state copies of register 0, [S][p+1][n+1][m+1] contiguous. */
+/* Whole-state copies of register 0, [S][p+1][n+1][m+1] contiguous.  (What a
+ * host array holds after a call that was to fill it and failed is not
+ * specified: here, of mfc_gpu_compute_rhs, _weno and _ensemble_download.) */
 int mfc_gpu_upload_state(mfc_gpu_ctx* ctx, const double* host_q);
 int mfc_gpu_download_state(mfc_gpu_ctx* ctx, double* host_q);
 

@@ -7,6 +7,7 @@
 // fused stage kernels for the TVD RK schemes of m_time_steppers.fpp and the
 // time loop of p_main.fpp.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
@@ -67,12 +68,30 @@ const StageEntry* find_stage(int nd, int nf, int wo, int prec, bool visc, bool c
 
 int report_error(int code, const std::string& msg) { return fail(code, msg); }
 
-void touch_pages(void* p, size_t bytes) {
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+void populate_pages(void* p, size_t bytes) {
   if (!p || bytes == 0) return;
   static const size_t page = [] {
     const long s = sysconf(_SC_PAGESIZE);
     return s > 0 ? (size_t)s : (size_t)4096;
   }();
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {  // no device, or an earlier error that the copy will report
+    (void)cudaGetLastError();
+    return;
+  }
+  if (at.type != cudaMemoryTypeUnregistered) return;
+  const uintptr_t first = reinterpret_cast<uintptr_t>(p) / page * page;
+  const size_t pages = (reinterpret_cast<uintptr_t>(p) + bytes - first + page - 1) / page;
+  if (pages > 256) {
+    unsigned char in[16];
+    bool resident = mincore(reinterpret_cast<void*>(first + pages / 2 * page), sizeof(in) * page, in) == 0;
+    for (unsigned char k : in) resident = resident && (k & 1);
+    if (!resident) (void)madvise(reinterpret_cast<void*>(first), pages * page, MADV_POPULATE_WRITE);
+    return;
+  }
   volatile char* c = static_cast<volatile char*>(p);
   for (size_t i = 0; i < bytes; i += page) c[i] = 0;
   c[bytes - 1] = 0;
@@ -618,7 +637,7 @@ int mfc_gpu_generate_ic(mfc_gpu_ctx* c, const mfc_patch* patches, int num_patche
 int mfc_gpu_download_state(mfc_gpu_ctx* c, double* host_q) {
   if (!c || !host_q) return fail(MFC_ERR_INVALID, "NULL argument");
   const size_t rows = (size_t)c->S * c->n[1] * c->n[2];
-  mfc::touch_pages(host_q, rows * c->n[0] * 8);
+  mfc::populate_pages(host_q, rows * c->n[0] * 8);
   if (c->sy == c->n[0])
     MFC_CUDA(cudaMemcpyAsync(host_q, c->reg[0], rows * c->n[0] * 8, cudaMemcpyDeviceToHost, c->stream));
   else
@@ -650,8 +669,8 @@ int mfc_gpu_compute_rhs(mfc_gpu_ctx* c, double* rhs_out, double* prim_out) {
   int rc = launch_stage(c, c->reg[0], c->reg[0], c->rhs, 0.0, mfc::kRhsOnly);
   if (rc) return rc;
   const int64_t cells = (int64_t)c->n[0] * c->n[1] * c->n[2];
-  mfc::touch_pages(rhs_out, (size_t)c->S * cells * 8);
-  mfc::touch_pages(prim_out, (size_t)c->S * cells * 8);
+  mfc::populate_pages(rhs_out, (size_t)c->S * cells * 8);
+  mfc::populate_pages(prim_out, (size_t)c->S * cells * 8);
   if (rhs_out) {
     for (int v = 0; v < c->S; ++v)
       if ((rc = copy_var(c, c->rhs, v, nullptr, rhs_out + v * cells, c->n[0], (int64_t)c->n[0] * c->n[1]))) return rc;

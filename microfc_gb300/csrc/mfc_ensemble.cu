@@ -316,7 +316,7 @@ int mfc_gpu_ensemble_download(mfc_gpu_ensemble* e, int i, double* host_q) {
   if (!e || !host_q || i < 0 || i >= e->num) return mfc::report_error(MFC_ERR_INVALID, "bad ensemble download");
   const mfc::EnsCase& C = e->cases[i];
   const int S = 2 * e->nf + 3;
-  mfc::touch_pages(host_q, (size_t)S * e->nx[i] * e->ny[i] * 8);
+  mfc::populate_pages(host_q, (size_t)S * e->nx[i] * e->ny[i] * 8);
   for (int v = 0; v < S; ++v) {
     cudaError_t err = cudaMemcpy2DAsync(host_q + (int64_t)v * e->nx[i] * e->ny[i], (size_t)e->nx[i] * 8,
                                         C.reg[0] + v * C.P.sv, (size_t)C.P.sy * 8, (size_t)e->nx[i] * 8,

@@ -211,8 +211,10 @@ extern "C" int mfc_gpu_weno(mfc_gpu_ctx* ctx, int dir, double* vL, double* vR) {
     return mfc::launch_weno<decltype(ND)::value, decltype(NF)::value>(*v.dev, v.q0, v.wo, dir, w, B.p[0], B.p[1],
                                                                        v.stream);
   });
-  mfc::touch_pages(vL, bytes);
-  mfc::touch_pages(vR, bytes);
+  if (e == cudaSuccess) {
+    mfc::populate_pages(vL, bytes);
+    mfc::populate_pages(vR, bytes);
+  }
   if (e == cudaSuccess) e = cudaMemcpyAsync(vL, B.p[0], bytes, cudaMemcpyDeviceToHost, v.stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(vR, B.p[1], bytes, cudaMemcpyDeviceToHost, v.stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(v.stream);

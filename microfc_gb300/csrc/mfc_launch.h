@@ -556,11 +556,16 @@ const StageEntry* find_stage(int nd, int nf, int wo, int prec, bool visc = false
 int report_error(int code, const std::string& msg);
 
 // Makes the pages of a host array that a device copy is about to fill
-// resident: one store per page (the copy overwrites the whole array).  On
-// Grace a copy into untouched pages faults them in one by one from the GPU's
-// side, about 40 us per 64 KB page: 24 fresh ensemble states (82 MB) took
-// 52 ms to download, 4.4 ms with the stores.
-void touch_pages(void* p, size_t bytes);
+// resident.  On Grace a copy into fresh pages faults them in one by one from
+// the GPU's side, about 40 us per 64 KB page: 24 fresh ensemble states (82 MB)
+// took 52 ms to download, 4.4 ms with this.  Pinned arrays and addresses that
+// are not host memory are left alone.  Up to 256 pages: one store per page,
+// which the copy overwrites.  More: where pages of the middle are missing the
+// kernel is asked to populate the range.  (us a download, without, with: 112 KB
+// fresh 104 and 27, again into the same array 12.3 and 12.6; 28 MB fresh 1230
+// and 1090, again 164.8 and 167.2, by stores 1160 and 169.5.  The kernel's
+// residency map costs 1.7 us, more than the stores of 256 pages.)
+void populate_pages(void* p, size_t bytes);
 
 // Gate training samples of a 2-D state (mfc_gate.cu).
 int gate_samples(const DevParams& P, int nf, const double* q, int dir, float* xout, float* dev_out, cudaStream_t st);
