@@ -516,17 +516,19 @@ __device__ __forceinline__ void monitor_max(unsigned long long* w, double v) {
 // The FP64 operations are DFMAs of three registers where they can be (Fma64:
 // 16 instead of 19 SM cycles each; one: the register holding 1.0), and a fluid without pi_inf (an ideal gas) adds none: its
 // products are zeros, whose sum changes nothing while the state is finite.
-template <int ND, int NF>
+// FLUSH: for units whose own arithmetic keeps subnormals (mfc_gate.cu).
+template <int ND, int NF, bool FLUSH = false>
 __device__ __forceinline__ void cons_to_prim_split(const double (&q)[Eqs<ND, NF>::S], const DevParams& P,
                                                    double one, float (&out)[Eqs<ND, NF>::S]) {
   using Q = Eqs<ND, NF>;
+  auto cut = [](double x) { return FLUSH ? d2f_bits(x) : d2f_ftz(x); };
   float rho = 0.f, gam = 0.f;
   double e = q[Q::E];
   bool any = false;
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
-    out[f] = d2f_ftz(q[f]);
-    out[Q::ADV + f] = d2f_ftz(q[Q::ADV + f]);
+    out[f] = cut(q[f]);
+    out[Q::ADV + f] = cut(q[Q::ADV + f]);
     rho = rho + out[f];
     gam = fmaf(out[Q::ADV + f], d2f_bits(P.gammas[f]), gam);
     any |= __double_as_longlong(P.pi_infs[f]) != 0;  // integer: a comparison would occupy the FP64 unit
@@ -543,12 +545,12 @@ __device__ __forceinline__ void cons_to_prim_split(const double (&q)[Eqs<ND, NF>
   float m2 = 0.f;
 #pragma unroll
   for (int d = 0; d < ND; ++d) {
-    const float m = d2f_ftz(q[Q::MOM + d]);
+    const float m = cut(q[Q::MOM + d]);
     out[Q::MOM + d] = m * irho;
     m2 = fmaf(m, m, m2);
   }
   const double dE = __fma_rn(-f2d_bits(0.5f * m2 * irho), one, e);
-  out[Q::E] = __fdividef(d2f_ftz(dE), gam);
+  out[Q::E] = __fdividef(cut(dE), gam);
 }
 
 // ---------------------------------------------------------------------------

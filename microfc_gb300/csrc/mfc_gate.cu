@@ -45,7 +45,7 @@ __global__ void gate_sample_kernel(const mfc::DevParams P, const double* __restr
       for (int v = 0; v < Q::S; ++v) qq[v] = q[gy * P.sy + gx + v * P.sv];
       if (flip) qq[Q::MOM + dir] = -qq[Q::MOM + dir];
       float pr[Q::S];
-      mfc::cons_to_prim_split<2, NF>(qq, P, 1.0, pr);
+      mfc::cons_to_prim_split<2, NF, true>(qq, P, 1.0, pr);
       a[k] = pr[Q::ADV];
       p[k] = pr[Q::E];
     }
