@@ -279,8 +279,10 @@ Plan plan(int nx, int ny) {
       }
       return phase(gl * prim, gl, prim, NW) + weno + hllc + phase(gi * cell, gi, cell, NW) + kTile;
     };
-    return search(nx, ny, 1, ND > 1 ? 4 : 2, ND > 1 ? 96 : 512, ND > 1 ? 4 : 1, 96, cost,
-                  [](int x, int y) { return Sh::bytes(x, y) <= kFlexSmemMax; });
+    // (a launch takes 65535 rows of tiles)
+    return search(nx, ny, 1, ND > 1 ? 4 : 2, ND > 1 ? 96 : 512, ND > 1 ? 4 : 1, 96, cost, [ny](int x, int y) {
+      return Sh::bytes(x, y) <= kFlexSmemMax && (ny + y - 1) / y <= 65535;
+    });
   });
 }
 
