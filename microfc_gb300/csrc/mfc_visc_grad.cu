@@ -350,7 +350,8 @@ __global__ void __launch_bounds__(kGT) visc_gradients_tiled(const DevParams P, c
   f32x2* const sl = sg + 2 * Sh::NG;    // [d][..] left values
   f32x2* const sr = sl + 2 * (Sh::NX > Sh::NY ? Sh::NX : Sh::NY);
   const int tid = threadIdx.x, nx = P.n[0], ny = P.n[1];
-  const int x0 = blockIdx.x * kGX, y0 = blockIdx.y * kGY;
+  const unsigned tiles_x = nx / kGX + 1;
+  const int x0 = blockIdx.x % tiles_x * kGX, y0 = blockIdx.x / tiles_x * kGY;
   const float eps = d2f_bits(P.weno_eps);  // cut like every value, where weno_eps_f is rounded
   const f32x2 eps2 = f2_pack(eps, eps);
   const f32x2 half = f2_pack(0.5f, 0.5f);
@@ -485,7 +486,8 @@ cudaError_t launch_tiled(const DevParams& P, const ViscGradBuffers& B, const dou
   const auto kernel = B.uniform.on ? visc_gradients_tiled<true> : visc_gradients_tiled<false>;
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GradShape::kBytes);
   if (e != cudaSuccess) return e;
-  const dim3 grid((unsigned)(nx / kGX + 1), (unsigned)(ny / kGY + 1));  // nx + 1 and ny + 1 faces
+  // nx + 1 and ny + 1 faces; along x alone, which takes more than 65535 rows of tiles
+  const dim3 grid((unsigned)(nx / kGX + 1) * (unsigned)(ny / kGY + 1));
   return launch_dependent(kernel, grid, dim3(kGT), GradShape::kBytes, st, P, B.uniform, B.cf[0], B.cf[1],
                           reinterpret_cast<const f32x2*>(B.vel), reinterpret_cast<f32x2*>(B.fg[0]),
                           reinterpret_cast<f32x2*>(B.fg[1]));

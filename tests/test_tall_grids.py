@@ -3,7 +3,10 @@ import os
 import shutil
 import subprocess
 
+import numpy as np
 import pytest
+
+from microfc_gb300 import cases
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "microfc_gb300", "csrc")
 
@@ -37,3 +40,19 @@ def test_plans_of_tall_grids_can_be_launched(tmp_path):
                     "-I", CSRC, "-o", str(exe), str(src)], check=True, capture_output=True)
     r = subprocess.run([str(exe)], check=True, capture_output=True, text=True)
     assert r.stdout == "done\n", r.stdout
+
+
+@pytest.mark.gpu
+def test_gradients_of_the_tallest_grid():
+    """Split weno_Re_flux on 25 x 1048560 cells: 65535 rows of 16 cells and one
+    row of faces more."""
+    from microfc_gb300 import Simulation
+    ny = 65535 * 16
+    c = cases.shock_droplet_2d(nx=64, ny=32, steps=1, dt=1e-15, precision="split")
+    c = c.replace(m=24, n=ny - 1, patches=c.patches[:2], re_shear=(1e6, 1e6), weno_re_flux=True)  # the shock alone
+    with Simulation(c, ic="device") as sim:
+        sim.tvd_rk(0, c.dt)
+        assert sim.status() == 0
+        u = np.zeros((ny, 25))
+        sim.download_var(2, u, 25)
+    assert np.isfinite(u).all() and np.abs(u).max() > 0
