@@ -97,11 +97,13 @@ __global__ void riemann_window_kernel(const DevParams P, const double* __restric
   using Q = Eqs<ND, NF>;
   constexpr int S = Q::S;
   const int64_t faces = fw.count(), cells = cw.count();
-  double gam[NF], pin[NF];
+  using N = Num64;  // the number type of the plain FP64 steps
+  const N u0 = num64_unit(P.inv_d[0]);
+  N gam[NF], pin[NF];
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
-    gam[f] = P.gammas[f];
-    pin[f] = P.pi_infs[f];
+    gam[f] = lift(P.gammas[f], u0);
+    pin[f] = lift(P.pi_infs[f], u0);
   }
   int64_t step = 1;  // window stride along DIR
   if (DIR >= 1) step *= cw.e[0];
@@ -114,18 +116,18 @@ __global__ void riemann_window_kernel(const DevParams P, const double* __restric
     const int64_t rc = lc + step;
     const bool lfr = j == -1 && P.bc_beg[DIR] == -4;
     const bool rfl = j == P.n[DIR] - 1 && P.bc_end[DIR] == -4;
-    double qL[S], qR[S], F[S], us;
+    N qL[S], qR[S], F[S], us;
 #pragma unroll
     for (int s = 0; s < S; ++s) {
-      const double a = __ldg(ql + lc + s * cells);  // qL_rs(j)
-      const double b = __ldg(qr + rc + s * cells);  // qR_rs(j + 1)
-      qL[s] = lfr ? __ldg(qr + rc + s * cells) : a;
-      qR[s] = rfl ? __ldg(ql + lc + s * cells) : b;
+      const N a = lift(__ldg(ql + lc + s * cells), u0);  // qL_rs(j)
+      const N b = lift(__ldg(qr + rc + s * cells), u0);  // qR_rs(j + 1)
+      qL[s] = lfr ? b : a;
+      qR[s] = rfl ? a : b;
     }
-    hllc_face<ND, NF, DIR, double>(qL, qR, gam, pin, F, us);
+    hllc_face<ND, NF, DIR, N>(qL, qR, gam, pin, F, us);
 #pragma unroll
-    for (int s = 0; s < S; ++s) flux[c + s * faces] = F[s];
-    src[c] = us;
+    for (int s = 0; s < S; ++s) flux[c + s * faces] = low(F[s]);
+    src[c] = low(us);
   }
 }
 
