@@ -161,11 +161,15 @@ StageEntry pair_entry() {
 }
 
 // Two pair entries as one: tiles of 8x8 cells where 16x16 ones are too few
-// to fill the chip (kSmallTiles of them or less), else 16x16.  Where the line
-// lies (us a step, 8x8 and 16x16): 100x50 (28 tiles) 14.6 and 19.0, 333x167
-// (231) 22.5 and 27.9, 400x200 (325) 31.9 and 31.9, 512x256 (512) 45.4 and
-// 37.5.
-constexpr int64_t kSmallTiles = 320;
+// to fill the chip (kSmallTiles of them or less: up to there the 8x8 ones, six
+// blocks on an SM, are one wave), else 16x16.  Where the line lies (us a step,
+// 8x8 and 16x16, two fluids): 100x50 (28 tiles) split 13.7 and 19.1, gated 17.0
+// and 26.2, viscous 20.7 and 25.2; 333x167 (231) split 22.3 and 27.9, one fluid
+// 20.3 and 23.1, gated 25.9 and 31.9, viscous 33.1 and 36.1, weno_Re_flux 67.7
+// and 69.5; 360x180 (276) split 29.2 and 30.0, stretched 32.9 and 29.9, one
+// fluid 25.3 and 24.3, gated 35.5 and 34.2, viscous 44.3 and 37.9,
+// weno_Re_flux 80.5 and 71.3; 512x256 (512) split 45.4 and 37.0.
+constexpr int64_t kSmallTiles = 240;
 template <class Small, class Large>
 StageEntry sized_entry(const Small&, const Large&) {
   StageEntry e = Large::entry();
