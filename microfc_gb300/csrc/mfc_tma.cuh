@@ -47,12 +47,6 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// Orders this thread's earlier generic-proxy accesses of shared memory
-// before later copy-engine (async-proxy) writes to it.
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
 // Acquire of a tensor map held in global memory (written by a copy from the
 // host), before the copy engine reads it.
 __device__ __forceinline__ void tensormap_acquire(const void* map) {
