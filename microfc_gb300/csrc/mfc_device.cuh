@@ -514,8 +514,9 @@ __device__ __forceinline__ void monitor_max(unsigned long long* w, double v) {
 // GB300's FP64 pipe bounds the split stage, and this conversion runs on every
 // halo cell as well (1.75x the interior for 16x16 tiles).
 // The FP64 operations are DFMAs of three registers where they can be (Fma64:
-// 16 instead of 19 SM cycles each; one: the register holding 1.0), and a fluid without pi_inf (an ideal gas) adds none: its
-// products are zeros, whose sum changes nothing while the state is finite.
+// 16 instead of 19 SM cycles each; one: the register holding 1.0), and a fluid
+// without pi_inf (an ideal gas) adds none: its products are zeros unless its
+// volume fraction is not finite, which then makes the pressure a NaN by itself.
 // FLUSH: for units whose own arithmetic keeps subnormals (mfc_gate.cu).
 template <int ND, int NF, bool FLUSH = false>
 __device__ __forceinline__ void cons_to_prim_split(const double (&q)[Eqs<ND, NF>::S], const DevParams& P,
@@ -524,9 +525,10 @@ __device__ __forceinline__ void cons_to_prim_split(const double (&q)[Eqs<ND, NF>
   auto cut = [](double x) { return FLUSH ? d2f_bits(x) : d2f_ftz(x); };
   float rho = 0.f, gam = 0.f;
   double e = q[Q::E];
-  bool any = false;
+  bool any = false, bad = false;
 #pragma unroll
   for (int f = 0; f < NF; ++f) {
+    bad |= not_finite(q[Q::ADV + f]);
     out[f] = cut(q[f]);
     out[Q::ADV + f] = cut(q[Q::ADV + f]);
     rho = rho + out[f];
@@ -550,7 +552,8 @@ __device__ __forceinline__ void cons_to_prim_split(const double (&q)[Eqs<ND, NF>
     m2 = fmaf(m, m, m2);
   }
   const double dE = __fma_rn(-f2d_bits(0.5f * m2 * irho), one, e);
-  out[Q::E] = __fdividef(cut(dE), gam);
+  const float p = __fdividef(cut(dE), gam);
+  out[Q::E] = bad ? __int_as_float(0x7fffffff) : p;
 }
 
 // ---------------------------------------------------------------------------
