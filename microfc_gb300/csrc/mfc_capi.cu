@@ -82,19 +82,28 @@ void populate_pages(void* p, size_t bytes) {
     (void)cudaGetLastError();
     return;
   }
-  if (at.type != cudaMemoryTypeUnregistered) return;
+  if (at.type != cudaMemoryTypeUnregistered && at.type != cudaMemoryTypeHost) return;
+  volatile char* c = static_cast<volatile char*>(p);
+  auto touch = [&](auto&& f) {
+    for (size_t i = 0; i < bytes; i += page) f(c + i);
+    f(c + bytes - 1);
+  };
   const uintptr_t first = reinterpret_cast<uintptr_t>(p) / page * page;
   const size_t pages = (reinterpret_cast<uintptr_t>(p) + bytes - first + page - 1) / page;
-  if (pages > 256) {
+  if (at.type == cudaMemoryTypeUnregistered && pages <= 256) {
+    touch([](volatile char* x) { *x = 0; });
+    return;
+  }
+  if (at.type == cudaMemoryTypeUnregistered) {
     unsigned char in[16];
     bool resident = mincore(reinterpret_cast<void*>(first + pages / 2 * page), sizeof(in) * page, in) == 0;
     for (unsigned char k : in) resident = resident && (k & 1);
-    if (!resident) (void)madvise(reinterpret_cast<void*>(first), pages * page, MADV_POPULATE_WRITE);
-    return;
+    if (!resident) {
+      (void)madvise(reinterpret_cast<void*>(first), pages * page, MADV_POPULATE_WRITE);
+      return;
+    }
   }
-  volatile char* c = static_cast<volatile char*>(p);
-  for (size_t i = 0; i < bytes; i += page) c[i] = 0;
-  c[bytes - 1] = 0;
+  touch([](volatile char* x) { (void)*x; });
 }
 
 namespace {

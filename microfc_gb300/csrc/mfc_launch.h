@@ -561,16 +561,20 @@ const StageEntry* find_stage(int nd, int nf, int wo, int prec, bool visc = false
 // Records msg as the calling thread's mfc_gpu_last_error() and returns code.
 int report_error(int code, const std::string& msg);
 
-// Makes the pages of a host array that a device copy is about to fill
-// resident.  On Grace a copy into fresh pages faults them in one by one from
-// the GPU's side, about 40 us per 64 KB page: 24 fresh ensemble states (82 MB)
-// took 52 ms to download, 4.4 ms with this.  Pinned arrays and addresses that
-// are not host memory are left alone.  Up to 256 pages: one store per page,
-// which the copy overwrites.  More: where pages of the middle are missing the
-// kernel is asked to populate the range.  (us a download, without, with: 112 KB
-// fresh 104 and 27, again into the same array 12.3 and 12.6; 28 MB fresh 1230
-// and 1090, again 164.8 and 167.2, by stores 1160 and 169.5.  The kernel's
-// residency map costs 1.7 us, more than the stores of 256 pages.)
+// Makes the pages of a host array that a device copy is about to fill resident
+// and recently used.  On Grace a copy into fresh pages faults them in one by
+// one from the GPU's side, about 40 us per 64 KB page: 24 fresh ensemble states
+// (82 MB) took 52 ms to download, 4.4 ms with this.  And pages that the CPU has
+// not used for a while cost a copy 2 to 3 us each now and then, pinned ones too:
+// of 180 downloads of a pinned 1.07 GB state 26 took 40 to 100 ms instead of
+// 5.6, of as many with a read of each page (5.9 ms) one to three.
+//
+// Pinned arrays: one read per page.  Pageable ones of up to 256 pages: one
+// store, which the copy overwrites.  Larger ones: the kernel is asked to
+// populate the range where pages of the middle are missing, else one read per
+// page.  Other addresses are left alone.  (us a download, without, with: 112 KB
+// fresh 104 and 27, again into the same array 12.3 and 12.6, pinned 11.7 and
+// 11.7; 28 MB fresh 1230 and 1075, again 164.8 and 172.7, pinned 163.5 and 168.6.)
 void populate_pages(void* p, size_t bytes);
 
 // Gate training samples of a 2-D state (mfc_gate.cu).
