@@ -24,12 +24,13 @@
 // not depend on the tile shape.
 //
 // Measured (us a step; before: the x-then-y stage kernel with 16x16 tiles and
-// TMA): split 100x50 22.8 -> 14.6, 333x167 32.3 -> 22.5, 1024x512 126 -> 111,
-// 2048x1024 453 -> 403; gated 1024x512 145 -> 132, 2048x1024 504 -> 468;
-// viscous split 1024x512 233 -> 214; 1-D 1000 cells 12.9 -> 9.6.  Of the
-// 1024x512 stage's 42 us (ncu: issue 55 %, FP64 unit 48 %, FMA 40 %, shared
-// memory 38 %, L2 5.9 TB/s before the stored pairs): load and conversion 31 %
-// before, reconstruction 26 %, HLLC 14 %, the last phase 21 %, launch 7 %.
+// TMA): split 100x50 22.8 -> 13.7, 333x167 32.3 -> 22.3, 1024x512 126 -> 110,
+// 2048x1024 453 -> 403; gated 1024x512 145 -> 133, 2048x1024 504 -> 471;
+// viscous split 1024x512 233 -> 194; 1-D 1000 cells 12.9 -> 9.6.  Counters at
+// 2048x1024, first and later stages (121 and 140 us): issue 69 and 64 %, FP64
+// unit 37 and 50 %, FMA 57 and 50 %, L1 45 and 42 %, DRAM 2.7 and 3.2 TB/s;
+// per issue 2.2 to 2.3 warps wait at barriers, 1.7 for a fixed latency, 1.1 to
+// 1.6 for shared memory, 1.2 for global loads.
 #pragma once
 
 #include "mfc_device.cuh"
