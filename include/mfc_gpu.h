@@ -300,14 +300,14 @@ int mfc_gpu_finalize(mfc_gpu_ctx* ctx);
  * its index and per-launch time in milliseconds.  A variant that stages its
  * tiles by TMA (MFC_VARIANT_TMA) wins a tie within 1 %. */
 int mfc_gpu_tune(mfc_gpu_ctx* ctx, int reps, int* variant_out, double* ms_out);
-/* Pins tile variant `variant` (the numbering mfc_gpu_tune reports) and
- * returns its tile shape and threads per block; MFC_ERR_INVALID past the
+/* Pins tile variant `variant` (the numbering mfc_gpu_tune reports, which is
+ * that of one build of this library) and returns its tile shape and threads per block; MFC_ERR_INVALID past the
  * last variant of the context's configuration. */
 int mfc_gpu_select_variant(mfc_gpu_ctx* ctx, int variant, int* tx, int* ty, int* threads);
 /* Features of tile variant `variant` of the context's configuration, as
  * MFC_VARIANT_* bits in *features; MFC_ERR_INVALID past the last variant. */
 #define MFC_VARIANT_TMA 0x1u /* interior tiles arrive by one TMA bulk tensor copy (2-D and
-                                3-D inviscid kernels)                                       */
+                                3-D kernels)                                                */
 int mfc_gpu_variant_features(mfc_gpu_ctx* ctx, int variant, uint32_t* features);
 
 /* ---- Learned WENO gate (no reference counterpart).  A 10-32-32-1 MLP on a
