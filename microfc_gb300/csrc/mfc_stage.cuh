@@ -263,7 +263,9 @@ __device__ __forceinline__ void stage_tile(const DevParams& P, const double* __r
   if constexpr (kSplit) u0 = 0.f;
   else u0 = num64_unit(P.inv_d[0]);
   auto num = [&](RT x) { return lift(x, u0); };
-  const double one = kSplit ? fma64_unit(P.inv_d[0]).one : 1.0;  // split: the FP64 sums' register operand
+  // split: the FP64 sums' register operand (1-D: a constant; loading it cost
+  // 30.4 against 28.9 us a step at 1000 cells, WENO3)
+  const double one = kSplit && ND > 1 ? fma64_unit(P.inv_d[0]).one : 1.0;
   (void)one;
 
   RT* sq = reinterpret_cast<RT*>(smem_raw);  // [S][LY][LX] primitive

@@ -93,7 +93,9 @@ __global__ void __launch_bounds__(NT, MINB) sweep_kernel(const DevParams P,
   if constexpr (kSplit) u0 = 0.f;
   else u0 = num64_unit(P.inv_d[0]);
   auto num = [&](RT x) { return lift(x, u0); };
-  const double one = kSplit ? fma64_unit(P.inv_d[0]).one : 1.0;  // split: the FP64 sums' register operand
+  // split: the FP64 sums' register operand (WENO3: a constant; us a step, loaded
+  // and constant, 40^3 556 and 516, 128^3 6063 and 6041; WENO1 792 and 812)
+  const double one = kSplit && WO == 1 ? fma64_unit(P.inv_d[0]).one : 1.0;
   (void)one;
   constexpr int OA = DIR, OB = DIR == 0 ? 1 : 0, OC = DIR == 2 ? 1 : 2;  // axis index of a, b, c
 
